@@ -49,10 +49,10 @@ HEIGHT, WIDTH = 5782, 3946
 SEED = 2
 # Algorithmic bytes: the stencil stage reads 8 B of
 # RGBI and writes a 24 B float64 candidate plus 1 B of status per pixel; the
-# serial walk reads a 32 B interval/jump entry and writes a 4 B running count
-# per RNG-dependent channel.
+# serial walk reads a 16 B entry and writes one bit and its share of an 8 B
+# word per 32 RNG-dependent channels.
 STENCIL_BYTES_PER_PIXEL = 33
-WALK_BYTES_PER_CHANNEL = 36
+WALK_BYTES_PER_CHANNEL = 16.25
 BATCH_FRAMES = 16          # uneven sizes, seeds 100..115
 HEAVY_FRAMES = 8           # full 5782x3946 frames at ~5% coverage, seeds 200..207
 SERVE_RATES = (2.0, 8.0, 32.0, 400.0)  # the last one above the GPU's capacity
@@ -60,21 +60,21 @@ SERVE_RATES = (2.0, 8.0, 32.0, 400.0)  # the last one above the GPU's capacity
 NCU_COUNTERS = os.path.join(ROOT, "profiles", "ncu_counters.json")
 
 
-WALK_BLOCKS_PER_SM = 3   # window-walk blocks per SM in one wave (kWinBlocksPerSM)
+WALK_BLOCKS_PER_SM = 4   # window-walk blocks per SM in one wave (kWinBlocksPerSM)
+WALK_AVG_CHUNKS = 18     # most 256-channel chunks per segment on average (kWalkAvgMax)
 
 
 def launches_per_frame(h: int, w: int, sms: int) -> int:
     """Kernel launches of one plain pass (the library's launch sequence):
     producer 3, planes 1, stencil 1, startup 1, chain 4, walk 1 per wave + 1
     rewalk, apply 3.  Waves are sized from the RNG-dependent list capacity,
-    with three window blocks per SM less one slot for the wave's resolve
-    block."""
+    with four window blocks per SM."""
 
     sites = 6 * w + h * w
     capacity = max(65536, sites // 2)
-    segments = (capacity + 4095) // 4096 + 1
-    per_wave = WALK_BLOCKS_PER_SM * sms - 1
-    waves = (segments + per_wave - 1) // per_wave
+    chunks = (capacity + 255) // 256
+    reach = WALK_BLOCKS_PER_SM * sms * WALK_AVG_CHUNKS
+    waves = (chunks + reach - 1) // reach
     return 14 + waves
 
 

@@ -47,8 +47,11 @@ struct Arena {
     uint32_t *seg_base = nullptr, *seg_amb = nullptr;
     uint32_t *seg_raw = nullptr;  // seg_raw_words(segments): per-segment and per-block sums
     AmbEntry *entries = nullptr;
-    uint32_t *pos = nullptr, *extra = nullptr;
+    SecondInterval *second = nullptr;
+    uint32_t *pos = nullptr, *site_of = nullptr;
+    ExtraWord *extra = nullptr;
     uint8_t *chunk_two = nullptr;
+    ChunkStat *chunk_stat = nullptr;
     void *producer = nullptr;
     float *rows = nullptr;
     uint16_t *out = nullptr;
@@ -59,7 +62,7 @@ struct Arena {
     int64_t amb_capacity = 0;
 };
 
-static int g_per_wave = 444;  // window blocks per wave: walk_per_wave(SM count)
+static int g_per_wave = 591;  // window blocks per wave: walk_per_wave(SM count)
 
 static size_t arena_layout(const Geometry &g, int64_t amb_cap, Arena *a) {
     size_t off = 0;
@@ -81,10 +84,13 @@ static size_t arena_layout(const Geometry &g, int64_t amb_cap, Arena *a) {
     const size_t o_sb = take((g.segments + 1) * 4);
     const size_t o_sa = take((g.segments + 1) * 4);
     const size_t o_sr = take(seg_raw_words(g.segments) * 4);
-    const size_t o_ent = take(amb_cap * sizeof(AmbEntry) + 64);
+    const size_t o_ent = take(amb_cap * sizeof(AmbEntry));
+    const size_t o_sec = take(amb_cap * sizeof(SecondInterval));
     const size_t o_pos = take(amb_cap * 4);
-    const size_t o_ext = take(amb_cap * 4);
+    const size_t o_site = take(amb_cap * 4);
+    const size_t o_ext = take(extra_words(amb_cap) * sizeof(ExtraWord));
     const size_t o_two = take(walk_chunks(amb_cap));
+    const size_t o_stat = take(walk_chunks(amb_cap) * sizeof(ChunkStat));
     const size_t o_prod = take(producer_bytes(g.h, g.w));
     const size_t o_rows = take(4 * (size_t)g.h * 4);
     const size_t o_out = take(px * 6);
@@ -106,9 +112,12 @@ static size_t arena_layout(const Geometry &g, int64_t amb_cap, Arena *a) {
         a->seg_amb = (uint32_t *)(b + o_sa);
         a->seg_raw = (uint32_t *)(b + o_sr);
         a->entries = (AmbEntry *)(b + o_ent);
+        a->second = (SecondInterval *)(b + o_sec);
         a->pos = (uint32_t *)(b + o_pos);
-        a->extra = (uint32_t *)(b + o_ext);
+        a->site_of = (uint32_t *)(b + o_site);
+        a->extra = (ExtraWord *)(b + o_ext);
         a->chunk_two = (uint8_t *)(b + o_two);
+        a->chunk_stat = (ChunkStat *)(b + o_stat);
         a->producer = (void *)(b + o_prod);
         a->rows = (float *)(b + o_rows);
         a->out = (uint16_t *)(b + o_out);
@@ -162,7 +171,7 @@ struct fx_context {
     int device = 0;
     bool profile = false;
     bool parallel_walk = true;
-    int walk_wave = 0;  // window segments per wave; 0: g_per_wave (three per SM)
+    int walk_wave = 0;  // window segments per wave; 0: g_per_wave (four per SM)
     double walk_sigmas = fx::kDefaultWindowSigmas;  // walk window half-width
     int stencil_rows = 8;  // stencil tile height: 8 (four blocks per SM) or 16 (two)
     double list_per_site = 0.0;  // longest RNG-dependent list per site a pass has needed
@@ -328,9 +337,10 @@ static int enqueue_pass(fx_context *ctx, Slot &s, const Geometry &g, const fx_pa
     // the walk scratch is sized for g_per_wave; a narrower wave uses part of it
     const int wave = (ctx->walk_wave > 0 && ctx->walk_wave < g_per_wave) ? ctx->walk_wave
                                                                          : g_per_wave;
-    WriterBuffers wb{a.seg_base, a.seg_amb, a.seg_raw, a.entries, a.pos, a.extra, a.counters,
+    WriterBuffers wb{a.seg_base, a.seg_amb, a.seg_raw, a.entries, a.second, a.pos,
+                     a.site_of, a.extra, a.counters,
                      a.amb_capacity, a.walk, wave, ctx->parallel_walk, ctx->walk_sigmas, cancel,
-                     a.chunk_two, ctx->use_priority ? ctx->top_priority : 0};
+                     a.chunk_two, a.chunk_stat, ctx->use_priority ? ctx->top_priority : 0};
     FX_CUDA(ctx, launch_writer(g, a.meta, a.cand, d_in, ctx->lut, ctx->high, ctx->low, ctx->ident, a.stages,
                                p, rng, wb, d_out, d_changed, a.err, st, marks));
     return FX_OK;

@@ -75,10 +75,25 @@ __host__ __device__ __forceinline__ int meta_amb(uint8_t m) {
 // One RNG-dependent channel for the serial walk.  In "T space" the 24-bit
 // state s is held as T = s << 8, so the LCG s -> 125 s + 1 (mod 2^24)
 // becomes T -> 125 T + 256 (mod 2^32) and interval tests need no masking.
+//
+// The walk's state S is the job's first state advanced by the extra draws
+// alone, S = G^E(T0): the fixed draws before a channel are a constant of the
+// channel, so its first-draw state is the affine map G^(pos + 1) of S.  With
+// the copy interval's start l1 subtracted in that map,
+//   t = a S + b = G^(pos + 1)(S) - l1,  copy iff t <= w  (a cyclic interval),
+// and S itself moves (S -> 125 S + 256) only when the channel does not copy.
+// A step is a multiply-add, a compare and a predicated multiply-add, and an
+// entry 16 bytes (the first form, stepping T from channel to channel with
+// one jump per outcome, took five instructions and 32 bytes).
 struct __align__(16) AmbEntry {
-    uint32_t l1, w1, l2, w2; // copy iff (T - l1) <= w1 || (T - l2) <= w2
-    uint32_t a0, c0;         // T_first_draw = a0 * T_prev + c0 (previous channel drew once)
-    uint32_t a1, c1;         // T_first_draw = a1 * T_prev + c1 (previous channel drew twice)
+    uint32_t a, b, w;
+    uint32_t two;            // 1: the copy set has a second interval (SecondInterval)
+};
+// The second copy interval of a channel, at the channel's index in its own
+// array and written only for channels that have one:
+// copy iff also t + d <= w, d = l1 - l2.
+struct SecondInterval {
+    uint32_t d, w;
 };
 
 // ---------------------------------------------------------------------------
@@ -190,12 +205,67 @@ __host__ __device__ inline int64_t seg_raw_words(int64_t segments) {
     return ((segments + 63) / 64) * 64 + 2 * (((groups + 63) / 64) * 64);
 }
 
+constexpr double kDefaultWindowSigmas = 4.5;
+// Channels per staged chunk of the window walk; chunks start at multiples
+// of it in list order (segments are whole chunks).
+constexpr int kWalkChunk = 256;
+// How a chain of n listed channels is cut into walk segments.  The fewest
+// waves whose segments average at most kWalkAvgMax chunks share the chain
+// evenly, so a short chain gets short segments on every SM instead of a few
+// long ones.  Inside a wave the candidate windows grow with the root of the
+// distance from the wave's start, so with long segments the later ones are
+// made shorter: segment x of B is (1 + r (1 - 1.5 sqrt(x / B))) times the
+// average (which integrates to 1), r = kWalkRamp.
+constexpr uint32_t kWalkAvgMax = 18;   // 4608 channels: a wave's widest window is 7.5 k
+constexpr double kWalkRamp = 0.5;
+constexpr uint32_t kWalkSegMax = 28 * kWalkChunk;  // most channels of a segment
+struct WalkPlan {
+    uint32_t chunks, waves, wave_chunks;  // of the chain; chunks of every wave but the last
+    uint32_t segs;                        // segments of a full wave
+    uint32_t even;                        // chunks per segment, or 0: ramped lengths
+    // first chunk of segment x (0..segs) of a wave, relative to the wave
+    __host__ __device__ uint32_t start(uint32_t x) const {
+        if (even) return x * even < wave_chunks ? x * even : wave_chunks;
+        if (x >= segs) return wave_chunks;
+        const double u = (double)x / (double)segs;
+        return (uint32_t)((double)wave_chunks * (u + kWalkRamp * (u - u * sqrt(u))));
+    }
+};
+__host__ __device__ inline WalkPlan walk_plan(uint32_t n, uint32_t per_wave) {
+    WalkPlan p;
+    p.chunks = (n + kWalkChunk - 1) / kWalkChunk;
+    const uint32_t reach = per_wave * kWalkAvgMax;
+    p.waves = p.chunks > reach ? (p.chunks + reach - 1) / reach : 1u;
+    p.wave_chunks = (p.chunks + p.waves - 1) / p.waves;
+    p.even = 0;
+    p.segs = per_wave;
+    if (p.wave_chunks < 4u * per_wave) {  // a ramp would leave segments empty
+        p.even = p.wave_chunks > 0 ? (p.wave_chunks + per_wave - 1) / per_wave : 1u;
+        p.segs = (p.wave_chunks + p.even - 1) / p.even;
+    }
+    return p;
+}
+// Copying states of one chunk's channels and their spread, for the windows'
+// prediction (k_coef): sums of m / 2 and of m (2^24 - m) / 2^23.
+struct ChunkStat {
+    uint32_t copy, spread;
+};
+// Extra draws of 32 consecutive listed channels: the count before the first,
+// and one bit per channel.  (One running count per channel took 16 times the
+// bytes, written once and read twice.)
+struct ExtraWord {
+    uint32_t before, bits;
+};
+__host__ __device__ inline int64_t extra_words(int64_t capacity) { return capacity / 32 + 2; }
+
 struct WriterBuffers {
     uint32_t *seg_base, *seg_amb;  // segments + 1 each
     uint32_t *seg_raw;             // seg_raw_words(segments): the prefix's partial sums
-    AmbEntry *entries;             // capacity (+64 bytes slack)
+    AmbEntry *entries;             // capacity
+    SecondInterval *second;        // capacity, sparse
     uint32_t *pos;                 // capacity
-    uint32_t *extra_after;         // capacity
+    uint32_t *site_of;             // capacity: the site of each listed channel
+    ExtraWord *extra;              // extra_words(capacity)
     void *counters;                // DevCounters
     int64_t capacity;
     void *walk_scratch;            // walk_scratch_bytes(capacity, per_wave)
@@ -205,6 +275,7 @@ struct WriterBuffers {
     const uint32_t *cancel;        // host-mapped cancel word read by the stage gates, or null
     uint8_t *chunk_two;            // walk_chunks(capacity): 1 when a chunk holds a
                                    // two-interval entry
+    ChunkStat *chunk_stat;         // walk_chunks(capacity)
     int priority;                  // launch priority of the chain and the walk (0: default)
 };
 
@@ -258,20 +329,14 @@ size_t dev_counters_bytes();
 cudaError_t walk_init();
 size_t walk_scratch_bytes(int64_t capacity, int per_wave);
 int walk_per_wave(int sms);
-constexpr double kDefaultWindowSigmas = 4.5;
-// Channels per staged chunk of the window walk; chunks start at multiples
-// of it in list order (segments are whole chunks).
-constexpr int kWalkChunk = 256;
-constexpr uint32_t kWalkSegLen = 4096;  // channels per walk segment (whole chunks)
 __host__ __device__ inline size_t walk_chunks(int64_t capacity) {
     return (size_t)((capacity + kWalkChunk - 1) / kWalkChunk) + 1;
 }
-void walk_segment_stats(void *scratch, int64_t capacity, unsigned long long **copy,
-                        unsigned long long **spread, size_t *bytes_each);
-cudaError_t launch_walk(const AmbEntry *entries, const uint32_t *pos, const uint32_t *n_ptr,
-                        int64_t capacity, uint32_t s0, void *scratch, int per_wave,
+cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
+                        const uint32_t *n_ptr, int64_t capacity, uint32_t s0, void *scratch, int per_wave,
                         bool parallel, double window_sigmas, const uint8_t *chunk_two,
-                        uint32_t *extra_after, uint32_t *fallbacks_out,
+                        const ChunkStat *chunk_stat,
+                        ExtraWord *extra, uint32_t *fallbacks_out,
                         unsigned long long *stats_out, const uint32_t *err,
                         cudaStream_t stream, int priority);
 // Stage gate: when *cancel (host-mapped) is set, stop the pass: err[1] = 1

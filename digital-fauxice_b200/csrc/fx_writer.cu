@@ -15,10 +15,12 @@
 //      that copy the original, as at most two state intervals (found by
 //      binary search on the exact binary64 expressions, which are monotone
 //      in the state).
-//   4. k_coef: the affine LCG jump g^gap between consecutive such channels.
-//   5. the walk (fx_walk.cu) visits only the RNG-dependent channels: a jump,
-//      an interval test, a select per channel, parallelised over segments by
-//      speculation.  Output: the running count of extra draws.
+//   4. k_coef: the interval test of each such channel as a function of the
+//      extra draws before it (the channel's fixed draws folded into an affine
+//      LCG jump).
+//   5. the walk (fx_walk.cu) visits only the RNG-dependent channels: a
+//      multiply-add, a test and a conditional LCG step per channel,
+//      parallelised over segments by speculation.  Output: the running count of extra draws.
 //   6. k_apply: every public site recomputes its exact draws and values from
 //      its own start state g^(fixed + extra before it)(s0), in parallel, and
 //      emits public RGB16 with the counters.
@@ -97,13 +99,14 @@ __device__ __forceinline__ T block_sum(T v, T *scratch) {
 
 constexpr int kPer = kSegment / kSegThreads;  // sites per thread
 
-// Running extra-draw count after `count` RNG-dependent channels (clamped to
-// the list capacity; an overflowing frame is rerun by the host).
-__device__ __forceinline__ uint32_t extra_before(const uint32_t *extra_after, uint32_t count,
+// Extra draws of the first `count` RNG-dependent channels (clamped to the
+// list capacity; an overflowing frame is rerun by the host).
+__device__ __forceinline__ uint32_t extra_before(const ExtraWord *extra, uint32_t count,
                                                  int64_t capacity) {
     if (count == 0) return 0u;
-    const int64_t i = (int64_t)count - 1;
-    return extra_after[i < capacity ? i : capacity - 1];
+    const uint32_t i = (uint32_t)((int64_t)count < capacity ? (int64_t)count : capacity);
+    const uint2 w = __ldg(reinterpret_cast<const uint2 *>(extra) + (i >> 5));
+    return w.x + (uint32_t)__popc(w.y & ((1u << (i & 31u)) - 1u));
 }
 
 // Packed local (base << 16 | amb) of one thread's sites.
@@ -292,6 +295,11 @@ __device__ __forceinline__ SiteInfo site_info(int64_t site, int w, const uint16_
     return si;
 }
 
+// Affine jump tables: g_jump[j][d] = g^(d * 64^j) in T space, so any jump
+// below 2^36 draws is six table lookups and compositions.
+constexpr int kJumpDigits = 6;
+__device__ Affine g_jump[kJumpDigits][64];
+
 // ---------------------------------------------------------------------------
 // Copy intervals of one RNG-dependent channel
 // ---------------------------------------------------------------------------
@@ -371,7 +379,13 @@ __device__ __forceinline__ double crossing(const ChannelView &cv, double base, d
     return ((target - base) / scale + 0.5) / kNormalization - 1.0;
 }
 
-__device__ void copy_intervals(const ChannelView &cv, AmbEntry &e, uint32_t *err) {
+// Copy set of one channel in T space: copy iff (T - l1) <= w1 or
+// (T - l2) <= w2 (modulo 2^32); l = 0x80 marks an empty interval.
+struct CopySet {
+    uint32_t l1, w1, l2, w2;
+};
+
+__device__ void copy_intervals(const ChannelView &cv, CopySet &e, uint32_t *err) {
     uint32_t b[3] = {
         switch_point([&](uint32_t s) { return cv.low_ok(s); }, crossing(cv, cv.cd, cv.dc.low)),
         switch_point([&](uint32_t s) { return cv.high_ok(s); }, crossing(cv, cv.cd, cv.dc.high)),
@@ -501,8 +515,8 @@ __global__ void __launch_bounds__(kSegWarps * 32)
 // k_coef's inputs of one entry, gathered in two dependent steps: the list
 // (coalesced) gives the site, the site gives its meta, pixel and candidates.
 struct CoefList {
-    uint32_t site, gap_lo, gap_hi;  // gap_lo/hi: pos[i-1] (0 for the first) and pos[i]
-    int k;                          // this entry is the k-th of its site
+    uint32_t site, pos;  // pos: fixed draws before the channel
+    int k;               // this entry is the k-th of its site
 };
 struct CoefSite {
     uint8_t meta;
@@ -513,14 +527,13 @@ struct CoefSite {
 __device__ __forceinline__ CoefList coef_list(const uint32_t *__restrict__ site_of,
                                               const uint32_t *__restrict__ pos, uint32_t i,
                                               uint32_t n) {
-    CoefList l{0u, 0u, 0u, 0};
+    CoefList l{0u, 0u, 0};
     if (i >= n) return l;
     l.site = site_of[i];
     // a site's RNG-dependent channels are listed in channel order
     l.k = (i >= 1 && site_of[i - 1] == l.site) ? ((i >= 2 && site_of[i - 2] == l.site) ? 2 : 1)
                                                 : 0;
-    l.gap_hi = pos[i];
-    l.gap_lo = i ? pos[i - 1] : 0u;
+    l.pos = pos[i];
     return l;
 }
 
@@ -540,19 +553,24 @@ __device__ __forceinline__ CoefSite coef_site(const CoefList &l, bool live, int6
     return c;
 }
 
-// Copy intervals and jumps of every RNG-dependent channel.  A thread's
+// Copy intervals and state map of every RNG-dependent channel.  A thread's
 // entries i, i + stride, ... run through a three-stage software pipeline:
 // while entry i's interval search computes, the site of entry i + 2 stride
 // and the meta, pixel and candidates of entry i + stride are in flight, so
 // the dependent gathers overlap the arithmetic instead of stalling it.
-__global__ void __launch_bounds__(256, 4) k_coef(AmbEntry *__restrict__ entries, const uint32_t *__restrict__ pos,
+__global__ void __launch_bounds__(256, 4) k_coef(AmbEntry *__restrict__ entries, SecondInterval *__restrict__ second,
+                       const uint32_t *__restrict__ pos,
                        const uint32_t *__restrict__ n_amb_ptr, int64_t capacity,
                        const uint32_t *__restrict__ site_of, const uint8_t *__restrict__ meta,
                        const double *__restrict__ cand, int w, const uint16_t *__restrict__ rgbi,
                        const float *__restrict__ lut, fx_params p, uint32_t *err,
-                       uint8_t *__restrict__ chunk_two, unsigned long long *__restrict__ seg_copy,
-                       unsigned long long *__restrict__ seg_spread) {
+                       uint8_t *__restrict__ chunk_two, ChunkStat *__restrict__ chunk_stat) {
+    // powers of the LCG step: states repeat after 2^24 draws, so the four
+    // low base-64 digits of a draw count give its map on states
+    __shared__ Affine s_jump[4][64];
     if (pass_stopped(err)) return;
+    for (int j = threadIdx.x; j < 4 * 64; j += blockDim.x) s_jump[j / 64][j % 64] = g_jump[j / 64][j % 64];
+    __syncthreads();
     const uint32_t n = (uint32_t)min((int64_t)*n_amb_ptr, capacity);
     const DitherConst dc = dither_const(p);
     const int64_t su = 6 * (int64_t)w;
@@ -578,38 +596,36 @@ __global__ void __launch_bounds__(256, 4) k_coef(AmbEntry *__restrict__ entries,
         cv.env = ((dc.high - cv.cd) * (cv.cd - dc.low)) * dc.coefficient;
         cv.span = (float)((double)p.dither_scales[c] * cv.cd);
         cv.od = (double)__ldg(lut + lane);
-        AmbEntry e;
+        CopySet e;
         copy_intervals(cv, e, err);
         // a chunk of walk channels with a two-interval entry steps with both
         // interval tests (every other chunk with one)
         if (e.l2 != 0x80u) chunk_two[i / kWalkChunk] = 1;
-        // the walk's prediction for this segment: m copying states of 2^24
-        // (an extra draw with probability p = 1 - m / 2^24), summed exactly
-        // per segment, with the spread m (2^24 - m) >> 22 (p (1 - p) in
-        // units of 2^-26).  A warp holds 32 consecutive entries of one
-        // segment; the lanes past the chain's end have left the loop.
+        // the walk's prediction: m copying states of 2^24 (an extra draw with
+        // probability p = 1 - m / 2^24), summed per chunk with the spread
+        // p (1 - p).  A warp holds 32 consecutive entries of one chunk; the
+        // lanes past the chain's end have left the loop.
         {
             uint32_t m = 0;
             if (e.l1 != 0x80u) m += (e.w1 >> 8) + 1u;
             if (e.l2 != 0x80u) m += (e.w2 >> 8) + 1u;
-            const uint32_t q = (uint32_t)(((unsigned long long)m * ((1u << 24) - m)) >> 22);
+            const uint32_t q = (uint32_t)(((unsigned long long)m * ((1u << 24) - m)) >> 23);
             const uint32_t lane = threadIdx.x & 31, live = n - (i - lane);
             const uint32_t mask = live >= 32u ? 0xFFFFFFFFu : ((1u << live) - 1u);
-            const uint32_t ms = __reduce_add_sync(mask, m), qs = __reduce_add_sync(mask, q);
+            const uint32_t ms = __reduce_add_sync(mask, m >> 1), qs = __reduce_add_sync(mask, q);
             if (lane == 0) {
-                atomicAdd(&seg_copy[i / kWalkSegLen], (unsigned long long)ms);
-                atomicAdd(&seg_spread[i / kWalkSegLen], (unsigned long long)qs);
+                atomicAdd(&chunk_stat[i / kWalkChunk].copy, ms);
+                atomicAdd(&chunk_stat[i / kWalkChunk].spread, qs);
             }
         }
-        const uint64_t gap = (i == 0) ? (uint64_t)l0.gap_hi + 1u
-                                      : (uint64_t)(uint32_t)(l0.gap_hi - l0.gap_lo);
-        const Affine f = lcg_power_t(gap);
-        const Affine f1 = affine_compose(Affine{125u, 256u}, f);  // one more draw
-        e.a0 = f.a;
-        e.c0 = f.c;
-        e.a1 = (i == 0) ? f.a : f1.a;  // no previous channel before the first
-        e.c1 = (i == 0) ? f.c : f1.c;
-        entries[i] = e;
+        // G^(pos + 1) less the first interval's start
+        const uint32_t draws = l0.pos + 1u;
+        Affine f = s_jump[0][draws & 63u];
+#pragma unroll
+        for (int j = 1; j < 4; ++j)
+            f = affine_compose(s_jump[j][(draws >> (6 * j)) & 63u], f);
+        entries[i] = AmbEntry{f.a, f.c - e.l1, e.w1, e.l2 != 0x80u ? 1u : 0u};
+        if (e.l2 != 0x80u) second[i] = SecondInterval{e.l1 - e.l2, e.w2};
         l0 = l1;
         s0 = s1;
         l1 = l2;
@@ -629,7 +645,7 @@ __global__ void __launch_bounds__(256, 4) k_coef(AmbEntry *__restrict__ entries,
 // the six rows (the extra draws of a row come from the walk's running count
 // at the row's ends).
 __global__ void k_startup_counts(const uint8_t *__restrict__ meta, int w,
-                                 const uint32_t *__restrict__ extra_after, uint32_t s0,
+                                 const ExtraWord *__restrict__ extra, uint32_t s0,
                                  DevCounters *ctr, int64_t capacity,
                                  const uint32_t *__restrict__ err) {
     __shared__ unsigned long long scratch[8];
@@ -660,14 +676,14 @@ __global__ void k_startup_counts(const uint8_t *__restrict__ meta, int w,
     uint32_t a_run = 0, p_run = 0;
     for (int r = 0; r < 6; ++r) {
         const uint32_t rb = vc->su_base[r], ra = vc->su_amb[r];
-        const uint32_t e_start = extra_before(extra_after, a_run, capacity);
+        const uint32_t e_start = extra_before(extra, a_run, capacity);
         const uint32_t a_end = a_run + ra;
-        const uint32_t e_end = extra_before(extra_after, a_end, capacity);
+        const uint32_t e_end = extra_before(extra, a_end, capacity);
         ctr->su_advances[r] = (unsigned long long)rb + (e_end - e_start);
         a_run = a_end;
         p_run += rb;
     }
-    const uint32_t e = extra_before(extra_after, a_run, capacity);
+    const uint32_t e = extra_before(extra, a_run, capacity);
     ctr->startup_base = p_run;
     ctr->startup_amb = a_run;
     ctr->startup_extra = e;
@@ -709,10 +725,6 @@ cudaError_t writer_identity_table(const float *lut, const uint32_t *hi, const ui
     return cudaGetLastError();
 }
 
-// Affine jump tables: g_jump[j][d] = g^(d * 64^j) in T space, so any jump
-// below 2^36 draws is six table lookups and compositions.
-constexpr int kJumpDigits = 6;
-__device__ Affine g_jump[kJumpDigits][64];
 constexpr int kApplyBlocksPerSM = 5;  // k_apply's resident blocks per SM
 static int g_apply_blocks = kApplyBlocksPerSM * 148;
 
@@ -757,7 +769,7 @@ __global__ void __launch_bounds__(kSegThreads, kApplyBlocksPerSM)
             const uint32_t *__restrict__ g_high, const uint32_t *__restrict__ g_low,
             const uint16_t *__restrict__ ident, const fx_stage *__restrict__ stages, fx_params p,
             const uint32_t *__restrict__ seg_base, const uint32_t *__restrict__ seg_amb,
-            const uint32_t *__restrict__ extra_after, uint32_t s0, uint16_t *__restrict__ rgb_out,
+            const ExtraWord *__restrict__ extra, uint32_t s0, uint16_t *__restrict__ rgb_out,
             uint8_t *__restrict__ changed_out, DevCounters *ctr, uint32_t *err,
             int64_t capacity) {
     __shared__ uint32_t hi[256], lo[256];
@@ -849,8 +861,8 @@ __global__ void __launch_bounds__(kSegThreads, kApplyBlocksPerSM)
             float values[3] = {orig[0], orig[1], orig[2]};
             const uint32_t Ak = s_a[k];
             const int amb = meta_amb(mi);
-            const uint32_t e_before = extra_before(extra_after, Ak, capacity);
-            const uint32_t extra = extra_before(extra_after, Ak + amb, capacity) - e_before;
+            const uint32_t e_before = extra_before(extra, Ak, capacity);
+            const uint32_t redraws = extra_before(extra, Ak + amb, capacity) - e_before;
             uint32_t state = jump_by_table(s_jump, s0, (uint64_t)s_p[k] + e_before);
             const double *cd = cand + 3 * site;
             const double c3[3] = {cd[0], cd[1], cd[2]};
@@ -877,7 +889,7 @@ __global__ void __launch_bounds__(kSegThreads, kApplyBlocksPerSM)
                     }
                 }
             }
-            if ((int64_t)(Ak + amb) <= capacity && draws != (uint32_t)meta_base(mi) + extra)
+            if ((int64_t)(Ak + amb) <= capacity && draws != (uint32_t)meta_base(mi) + redraws)
                 raise_error(err, FX_ERR_INTERNAL);
             att += 1;
             draws_total += draws;
@@ -923,12 +935,12 @@ __global__ void __launch_bounds__(kSegThreads, kApplyBlocksPerSM)
 }
 
 __global__ void k_final(const uint32_t *__restrict__ seg_base, const uint32_t *__restrict__ seg_amb,
-                        int64_t segments, const uint32_t *__restrict__ extra_after, uint32_t s0,
+                        int64_t segments, const ExtraWord *__restrict__ extra, uint32_t s0,
                         DevCounters *ctr, uint32_t *err, int64_t capacity) {
     if (pass_stopped(err)) return;
     const uint32_t p_total = seg_base[segments];
     const uint32_t a_total = seg_amb[segments];
-    const uint32_t e_total = extra_before(extra_after, a_total, capacity);
+    const uint32_t e_total = extra_before(extra, a_total, capacity);
     ctr->n_amb = a_total;
     ctr->final_state = lcg_jump(s0, (uint64_t)p_total + e_total);
     const unsigned long long expect =
@@ -965,38 +977,33 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
     e = launch_prio(k_seg_scan, dim3(1), dim3(1024), 0, stream, pr, b.seg_raw, segs, b.seg_base,
                     b.seg_amb, err);
     if (e != cudaSuccess) return e;
-    // the site list lives in extra_after until the walk writes the counts
     e = launch_prio(k_amb, dim3(seg_blocks), dim3(kSegWarps * 32), 0, stream, pr, meta, g.sites,
-                    segs, b.seg_raw, b.seg_base, b.seg_amb, b.extra_after, b.pos, b.capacity,
+                    segs, b.seg_raw, b.seg_base, b.seg_amb, b.site_of, b.pos, b.capacity,
                     err);
     if (e != cudaSuccess) return e;
     const uint32_t *n_amb = b.seg_amb + segs;
     cudaMemsetAsync(b.chunk_two, 0, walk_chunks(b.capacity), stream);
-    unsigned long long *seg_copy, *seg_spread;
-    size_t stat_bytes;
-    walk_segment_stats(b.walk_scratch, b.capacity, &seg_copy, &seg_spread, &stat_bytes);
-    cudaMemsetAsync(seg_copy, 0, stat_bytes, stream);
-    cudaMemsetAsync(seg_spread, 0, stat_bytes, stream);
-    e = launch_prio(k_coef, dim3(1184), dim3(256), 0, stream, pr, b.entries, b.pos, n_amb,
-                    b.capacity, b.extra_after, meta, cand, g.w, rgbi, lut, p, err, b.chunk_two,
-                    seg_copy, seg_spread);
+    cudaMemsetAsync(b.chunk_stat, 0, walk_chunks(b.capacity) * sizeof(ChunkStat), stream);
+    e = launch_prio(k_coef, dim3(1184), dim3(256), 0, stream, pr, b.entries, b.second, b.pos, n_amb,
+                    b.capacity, b.site_of, meta, cand, g.w, rgbi, lut, p, err, b.chunk_two,
+                    b.chunk_stat);
     if (e != cudaSuccess) return e;
     marks.mark(5, stream);
     e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
-    e = launch_walk(b.entries, b.pos, n_amb, b.capacity, s0, b.walk_scratch, b.per_wave,
-                    b.parallel_walk, b.window_sigmas, b.chunk_two, b.extra_after,
+    e = launch_walk(b.entries, b.second, n_amb, b.capacity, s0, b.walk_scratch, b.per_wave,
+                    b.parallel_walk, b.window_sigmas, b.chunk_two, b.chunk_stat, b.extra,
                     &ctr->walk_fallbacks, ctr->walk_stats, err, stream, pr);
     if (e != cudaSuccess) return e;
     marks.mark(6, stream);
     e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
-    k_startup_counts<<<6, 256, 0, stream>>>(meta, g.w, b.extra_after, s0 & kLcgMask, ctr,
+    k_startup_counts<<<6, 256, 0, stream>>>(meta, g.w, b.extra, s0 & kLcgMask, ctr,
                                             b.capacity, err);
     k_apply<<<(unsigned)std::min<int64_t>(segs, g_apply_blocks), kSegThreads, 0, stream>>>(
         meta, cand, g.sites, g.w, rgbi, lut, high, low, ident, stages, p, b.seg_base, b.seg_amb,
-        b.extra_after, s0 & kLcgMask, rgb_out, changed_out, ctr, err, b.capacity);
-    k_final<<<1, 1, 0, stream>>>(b.seg_base, b.seg_amb, segs, b.extra_after, s0 & kLcgMask,
+        b.extra, s0 & kLcgMask, rgb_out, changed_out, ctr, err, b.capacity);
+    k_final<<<1, 1, 0, stream>>>(b.seg_base, b.seg_amb, segs, b.extra, s0 & kLcgMask,
                                  ctr, err, b.capacity);
     marks.mark(7, stream);
     return cudaGetLastError();
