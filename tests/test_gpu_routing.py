@@ -165,3 +165,50 @@ def test_primitives_reject_bad_arguments():
     assert lib.fx_label8(None, 4, 4, None, None, None, None, ctypes.byref(count), None) == 1
     assert lib.fx_tile_extract(ctypes.c_void_p(16), 4, 4, 2, 2, 3, 3, 1, ctypes.c_void_p(16),
                                None) == 1  # tile outside the plane: rejected before launch
+
+
+@pytest.mark.parametrize("shape", [(65, 31), (64, 32), (130, 33), (200, 257), (3, 640), (640, 3)])
+@pytest.mark.parametrize("fill", ["stripes", "full", "corner"])
+def test_deep_and_word_edge_shapes_match_oracle(shape, fill):
+    """Words that end a row, tiles that end the frame, components that cross
+    word boundaries, and distances on both sides of the bit plane's reach."""
+
+    import torch
+
+    h, w = shape
+    mask = np.ones(shape, bool)
+    if fill == "stripes":
+        mask[:, 31::33] = False
+        mask[::7, ::5] = False
+    elif fill == "full":
+        mask[h // 2, w // 2] = False
+    else:
+        mask[0, 0] = False
+    dev = _dev()
+    m = torch.from_numpy(mask.view(np.uint8)).cuda()
+    labels, count = dev.label8(m, h, w)
+    expected, expected_count = ro.label8(mask)
+    assert count == expected_count
+    assert np.array_equal(labels.cpu().numpy(), expected)
+    dist = dev.distance(m, h, w)
+    assert np.array_equal(dist.cpu().numpy(), ro.chessboard_distance(mask))
+    areas, boxes, maxima = dev.stats(labels, dist, h, w, count)
+    d = dist.cpu().numpy()
+    for k in range(count):
+        ys, xs = np.nonzero(expected == k + 1)
+        assert areas[k] == ys.size and maxima[k] == d[ys, xs].max()
+        assert list(boxes[k]) == [ys.min(), xs.min(), ys.max() + 1, xs.max() + 1]
+    counts = dev.count_where(labels, (dist > 1).int(), count)
+    assert [counts[k + 1] for k in range(count)] == [
+        int(((expected == k + 1) & (d > 1)).sum()) for k in range(count)]
+
+
+@pytest.mark.parametrize("radius", [1, 15, 16, 30, 31, 32, 40])
+@pytest.mark.parametrize("shape", [(1, 700), (700, 1), (64, 256), (65, 257), (130, 31)])
+def test_dilation_tiles_match_oracle(shape, radius):
+    import torch
+
+    mask = np.random.default_rng(radius).random(shape) < 0.004
+    mask[shape[0] // 2, shape[1] // 2] = True
+    out = _dev().dilate(torch.from_numpy(mask.view(np.uint8)).cuda(), *shape, radius)
+    assert np.array_equal(out.cpu().numpy().view(np.bool_), ro.dilate_square(mask, radius))
