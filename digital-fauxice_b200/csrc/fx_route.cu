@@ -358,14 +358,15 @@ constexpr int32_t kDistInf = 0x3FFFFFFF;
 // Distances up to kDistNear from the bit plane.  A pixel's distance is the
 // least over the rows y +- k of max(k, distance along that row), and only rows
 // with k below the best so far can lower it; the row distances come from the
-// 64 bits to either side of the pixel.  A block covers 64 rows x 256 columns
-// with 64 pixels of halo in shared memory (9 KB); a tile without a set
+// 64 bits to either side of the pixel.  A block covers 16 rows x 256 columns
+// with 64 pixels of halo in shared memory (7 KB); a tile without a set
 // pixel only writes zeros.  Pixels outside the frame are no background.  A
 // deeper pixel gets kDistInf, from which the relaxation finishes it.
 // (Relaxing every tile from scratch took four launches of 500 us on a native
-// frame; this takes one of 60 us, with the packing 100.)
+// frame; this takes one of 140 us after 35 us of packing, 39 instead of 80 us on
+// 701x933; tiles of 64 rows left a small frame 44 blocks: 77 us.)
 constexpr int kDistNear = 63;
-constexpr int kNearRows = 64, kNearWords = 8;
+constexpr int kNearRows = 16, kNearWords = 8;
 
 __global__ void __launch_bounds__(kRouteThreads)
     k_dist_near(const uint32_t *__restrict__ bits, int h, int w, int32_t *__restrict__ dist,
@@ -546,11 +547,11 @@ __global__ void __launch_bounds__(kRouteThreads)
 // Square dilation, separable: a pixel is set when a set pixel lies within
 // `r` along the row, then within `r` along the column.
 //
-// Radii up to kDilateBits: a block packs its 64 x 256 tile and the halo into
+// Radii up to kDilateBits: a block packs its 32 x 256 tile and the halo into
 // bits, dilates the rows with shifts (doubling: the union over shifts 0..n
 // becomes 0..2n + 1 in one step) and ORs 2 r + 1 rows.
 constexpr int kDilateBits = 31;
-constexpr int kDilateRows = 64, kDilateWords = 8;
+constexpr int kDilateRows = 32, kDilateWords = 8;
 
 __global__ void __launch_bounds__(kRouteThreads)
     k_dilate_tile(const uint8_t *__restrict__ in, int h, int w, int rv, int rh,
