@@ -66,7 +66,7 @@ WALK_AVG_CHUNKS = 18     # most 256-channel chunks per segment on average (kWalk
 
 def launches_per_frame(h: int, w: int, sms: int) -> int:
     """Kernel launches of one plain pass (the library's launch sequence):
-    producer 3, planes 1, stencil 1, startup 1, chain 4, walk 1 per wave + 1
+    producer 2, planes 1, stencil 1, startup 1, chain 4, walk 1 per wave + 1
     rewalk, apply 3.  Waves are sized from the RNG-dependent list capacity,
     with four window blocks per SM."""
 
@@ -75,7 +75,7 @@ def launches_per_frame(h: int, w: int, sms: int) -> int:
     chunks = (capacity + 255) // 256
     reach = WALK_BLOCKS_PER_SM * sms * WALK_AVG_CHUNKS
     waves = (chunks + reach - 1) // reach
-    return 14 + waves
+    return 13 + waves
 
 
 def ncu_counter(kernel: str, name: str):

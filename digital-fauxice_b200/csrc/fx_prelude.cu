@@ -5,8 +5,8 @@
 // producer_parameters.py:498-541 / stage_parameters.py:93-197, plus the host
 // prepass reducer of prepass.py:96-236.  Every reduction keeps the
 // reference's strictly sequential binary64 order: the per-row sums run one
-// row per thread along the columns, the cumulative sums and the epoch chain
-// run in one warp.
+// row per lane along the columns, the cumulative sums and the epoch chain in
+// one block.
 #include <cmath>
 #include <cstring>
 
@@ -15,6 +15,8 @@
 namespace fx {
 
 constexpr float kIrThreshold = 8847.2255859375f;  // producer_parameters.py:36
+// an IR sample passes when it is above the threshold, and samples are integers
+constexpr uint32_t kIrLastFailing = (uint32_t)kIrThreshold;
 constexpr float kInitialVisibleMean = 46618.78515625f;
 constexpr float kInitialInfraredMean = 56239.65625f;
 constexpr float kInitialScale = 0.15f;
@@ -56,32 +58,34 @@ __host__ __device__ inline int setter_stage(float p1, float p2, float p3, float 
 // ---------------------------------------------------------------------------
 
 struct ProducerBuffers {
-    // [ne][cells] and [ne][cells][4]: kept in the scratch layout but no
-    // longer written (k_producer_rows accumulates the epoch sums itself), so
-    // the layout and the fixed-size scratch limits of the no-alloc entry stay
-    // as they are
+    // [ne][cells], [ne][cells][4], [3][h] and [2][ne]: kept in the scratch
+    // layout but no longer written (the epoch sums stay in k_producer_rows,
+    // the cumulative sums and epoch pairs in k_producer_scan), so the layout
+    // and the fixed-size scratch limits of the no-alloc entry stay as they are
     uint8_t *cell_ok;
     double2 *terms;
     double *row_sums;      // [3][h]  visible, infrared, weight
-    double *cum;           // [3][h]
+    double *cum;
     float *add;            // [2][ne]
-    float *p_epoch;        // [2][ne] p1, p2 after epoch e
+    float *p_epoch;
 };
 
-__device__ __forceinline__ float quadrant_tree(const float v[8][8], int ry, int cx) {
-    double first = (double)v[ry][cx];
-    first += (double)v[ry][cx + 1];
-    first += (double)v[ry][cx + 2];
-    first += (double)v[ry][cx + 3];
-    first += (double)v[ry + 1][cx];
-    first += (double)v[ry + 1][cx + 1];
-    const double second_tail = (double)v[ry + 1][cx + 2] + (double)v[ry + 1][cx + 3];
+// at(i, j): response of the quadrant's row i, column j.
+template <class At>
+__device__ __forceinline__ float quadrant_tree(At at) {
+    double first = (double)at(0, 0);
+    first += (double)at(0, 1);
+    first += (double)at(0, 2);
+    first += (double)at(0, 3);
+    first += (double)at(1, 0);
+    first += (double)at(1, 1);
+    const double second_tail = (double)at(1, 2) + (double)at(1, 3);
     first += second_tail;
-    double third = (double)v[ry + 2][cx] + (double)v[ry + 2][cx + 1];
-    const double third_tail = (double)v[ry + 2][cx + 2] + (double)v[ry + 2][cx + 3];
+    double third = (double)at(2, 0) + (double)at(2, 1);
+    const double third_tail = (double)at(2, 2) + (double)at(2, 3);
     third += third_tail;
-    double fourth = (double)v[ry + 3][cx] + (double)v[ry + 3][cx + 1];
-    const double fourth_tail = (double)v[ry + 3][cx + 2] + (double)v[ry + 3][cx + 3];
+    double fourth = (double)at(3, 0) + (double)at(3, 1);
+    const double fourth_tail = (double)at(3, 2) + (double)at(3, 3);
     fourth += fourth_tail;
     third += fourth;
     const double total = first + third;
@@ -99,513 +103,479 @@ __device__ __forceinline__ void center_quadrants(const float q[4], float out[4])
 }
 
 // Scale-epoch terms of one complete cell whose eight rows all pass the IR
-// test (_scale_epoch_additions, producer_parameters.py:183-263), in two
-// parts so a tile's cells spread over many threads: the eight quadrant trees
-// (visible and infrared response of each 4x4 quadrant), then the centring,
-// ratios and weights of the cell.
-
-// Quadrant tree `which` (0..3 visible quadrants, 4..7 infrared) of a cell;
-// raw(i, j) gives the cell's RGBI sample at row i, column j (uint2).
-template <class Raw>
-__device__ float quadrant_value(Raw raw, const float *__restrict__ lut, int which) {
-    const int q = which & 3, ir_lane = which >> 2;
-    const int qy = (q >> 1) * 4, qx = (q & 1) * 4;
-    float v[8][8];  // only the quadrant's 4x4 entries are touched
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint2 px = raw(qy + i, qx + j);
-            v[qy + i][qx + j] = __ldg(lut + (ir_lane ? (px.y >> 16) : (px.x & 0xFFFFu)));
-        }
-    return quadrant_tree(v, qy, qx);
-}
-
-// The four (term, ratio * term) pairs from the quadrant values and the raw
-// IR total.  The reference accumulates the raw IR samples in float32; every
-// partial sum is an integer below 64 * 65535 < 2^24, so each rounding is
+// test (_scale_epoch_additions, producer_parameters.py:183-263): the
+// (term, ratio * term) pair of quadrant q from the cell's quadrant means and
+// its raw IR total.  The reference accumulates the raw IR samples in float32;
+// every partial sum is an integer below 64 * 65535 < 2^24, so each rounding is
 // exact and the integer total is the same value.
-__device__ void finish_terms(const float vq[4], const float iq[4], uint32_t raw_total,
-                             double2 out[4]) {
+__device__ double2 finish_term(const float vq[4], const float iq[4], uint32_t raw_total, int q) {
     float vd[4], id[4];
     center_quadrants(vq, vd);
     center_quadrants(iq, id);
     const double rs = (double)(float)raw_total;
     const double low = (double)-0.125f, full_high = (double)0.3f, high = (double)0.425f;
     const double outer = (double)0.70710677f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const double vw = (double)vd[q];
-        double ratio, weight;
-        if (vw == 0.0) {
-            ratio = 0.0;
-            weight = 0.0;
-        } else {
-            ratio = (double)id[q] / vw;
-            if (ratio < low || ratio > high) weight = 0.0;
-            else if (ratio < 0.0 || ratio > full_high) weight = vw * outer;
-            else weight = vw;
-        }
-        double term = weight * weight;
-        term *= rs;
-        term *= rs;
-        out[q] = make_double2(term, ratio * term);
+    const double vw = (double)(q == 0 ? vd[0] : q == 1 ? vd[1] : q == 2 ? vd[2] : vd[3]);
+    const double iw = (double)(q == 0 ? id[0] : q == 1 ? id[1] : q == 2 ? id[2] : id[3]);
+    double ratio, weight;
+    if (vw == 0.0) {
+        ratio = 0.0;
+        weight = 0.0;
+    } else {
+        ratio = iw / vw;
+        if (ratio < low || ratio > high) weight = 0.0;
+        else if (ratio < 0.0 || ratio > full_high) weight = vw * outer;
+        else weight = vw;
     }
+    double term = weight * weight;
+    term *= rs;
+    term *= rs;
+    return make_double2(term, ratio * term);
 }
 
 // ---------------------------------------------------------------------------
-// Cells and per-row sums in one pass over the frame.  A block owns 32 rows
-// (four 8-row blocks) and walks 32 x 64 tiles, the next tile's samples
-// arriving by cp.async while the current one is worked on:
-//   * every warp but the first finds, by ballot, the first IR position in
-//     each 8x8 cell that fails the threshold (cells of the tile);
-//   * warps 1..7 compute the quadrant trees of complete passing cells of
-//     complete 8-row blocks (the scale epochs), one tree per thread, and
-//     warp 7 the cells' raw IR totals; warp 0 finishes the cells' terms one
-//     tile later;
-//   * warps 1..6 compute the per-pixel products of the row sums (zero where
-//     the cell failed earlier: adding +0.0 leaves a non-negative sum
-//     unchanged) into shared memory;
-//   * warp 0 adds the previous tile's products, one row per lane, in strict
-//     column order -- the only sequential part.
+// Cells and per-row sums in one pass over the frame.  A block owns RB 8-row
+// blocks and walks tiles of 64 columns.  Its warps have roles and every role
+// works on a tile of its own, so one barrier per tile is enough and all warps
+// have independent work between barriers:
+//   * kComputeWarps warps load their samples of tile t + 3 into registers (no
+//     staging: the shared memory it would take is L1 the LUT gathers hit in),
+//     note the failing IR samples of tile t + 2 (one ballot per row of a
+//     cell block); gather the two responses of tile t's samples, keep them in
+//     shared memory and form the row sums' products (zero where the cell
+//     failed earlier: adding +0.0 leaves the sums as they are); and compute
+//     the quadrant trees and IR totals of the complete passing cells of tile
+//     t - 1 and the terms of those of tile t - 2, one tree or one (cell,
+//     quadrant) per thread;
+//   * one warp finds the first failing position of each cell of tile t + 1
+//     and adds tile t - 3 to the epochs in cell order;
+//   * two warps add the products of tile t - 1, one row per lane, in strict
+//     column order.
+// Measured on a native frame: 275 us with all roles on 16 shared warps and two
+// barriers per tile (one warp's chain of finished cells, epoch sums and row
+// sums made a tile 8.4k cycles), 171 us so.  Staging the samples in shared
+// memory beside these buffers (221 KB) left the gathers no L1: 259 us.  Two
+// smaller blocks per SM need 40 registers a thread and spill: 412 us.
 // ---------------------------------------------------------------------------
 
 constexpr int kRowTile = 64;          // columns per tile (8 cells)
-constexpr int kRowWarps = 16;
+constexpr int kComputeWarps = 16;    // 512 threads: eight rows of a tile at a time
+constexpr int kRowWarps = kComputeWarps + 3;  // five per scheduler at most: 96 registers each
 constexpr int kRowPitch = kRowTile + 1;
-// Staged sample rows are 68 samples (544 bytes) apart: consecutive rows then
-// start 8 banks apart, so the four rows of a cell's failing-position ballot
-// (8 lanes per row, 64 bytes each) take the two wavefronts 256 bytes need,
-// where a 512-byte pitch put all four rows on the same 16 banks.
-constexpr int kRawPitch = kRowTile + 4;
-constexpr int kProductWarps = 14;     // warps 1..14
-constexpr int kStageRows = kRowWarps * 32 / kRowTile;  // rows one staging pass covers
-// Rows per block: five 8-row epochs, so a native frame (5782 rows) is 145
-// blocks, one wave on 148 SMs.  Warp 0 sums rows 0..31 on its lanes; rows
-// 32..39 are summed on lanes 0..7 of the last warp, beside it.
-constexpr int kRows = 40;
-constexpr int kRowBlocks = kRows / 8;
-constexpr int kTileCells = kRowBlocks * 8;  // epoch cells of one tile
-static_assert((kRawPitch * 8) % 16 == 0, "staged rows keep 16-byte copies aligned");
-static_assert(kRows % 8 == 0 && kRows % kStageRows == 0 && kRows > 32 && kRows <= 64,
-              "rows 0..31 and 32..kRows-1 are summed by two warps");
+constexpr int kMaxRowBlocks = 5;      // 40 rows: a native frame (5782 rows) is 145 blocks
 
+template <int RB>
 struct RowSmem {
-    uint2 raw[2][kRows][kRawPitch];    // staged RGBI samples
-    double p[2][3][kRows][kRowPitch];  // [buffer][visible, infrared, weight][row][column]
-    int fp[kRowBlocks][8];             // first failing position per (8-row block, cell)
-    float qv[2][kTileCells][8];        // quadrant trees per tile cell (rb * 8 + cc)
-    uint32_t rsum[2][kTileCells];      // raw IR total per tile cell
-    int flag[2][kTileCells];           // 0: no complete epoch cell, 1: failing, 2: passing
-    double2 tq[kTileCells][4];         // finished terms of the previous tile's cells
-    int tok[kTileCells];               // 1: the cell's terms count (passing)
+    static constexpr int kRows = RB * 8, kCells = RB * 8;  // epoch cells of one tile
+    uint32_t failing[2][RB][2][8];     // [8-row block][32-column half][row]: a bit per column
+    double p[2][2][kRows][kRowPitch];  // [buffer][visible, infrared] products
+    float2 resp[2][kRows][kRowPitch];  // [buffer] responses: visible, infrared
+    uint32_t ir[2][kRows][kRowPitch];  // IR samples, 0 where not used
+    int fp[2][RB][8];                  // first failing position per (8-row block, cell)
+    float qv[2][kCells][8];            // quadrant trees per tile cell (rb * 8 + cc)
+    uint32_t qsum[2][kCells][4];       // raw IR total per quadrant
+    // per tile cell: 0 no complete epoch cell, 1 failing, 2 passing
+    uint32_t cell[4][kCells];
+    double2 tq[2][kCells][4];          // finished terms
+    int tok[2][kCells];                // 1: the cell's terms count (passing)
 };
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
-    const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
-}
-
+template <int RB>
 __global__ void __launch_bounds__(kRowWarps * 32, 1)
     k_producer_rows(const uint16_t *__restrict__ rgbi, int h, int w, int active_width, int cells,
                     const float *__restrict__ lut, ProducerBuffers b) {
+    using Smem = RowSmem<RB>;
+    constexpr int kRows = Smem::kRows, kCells = Smem::kCells;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    RowSmem &S = *reinterpret_cast<RowSmem *>(smem_raw);
+    Smem &S = *reinterpret_cast<Smem *>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r0 = blockIdx.x * kRows;
     const int tiles = (active_width + kRowTile - 1) / kRowTile;
     const int ne = h / 8;  // complete 8-row blocks
-    const double thr = (double)kIrThreshold;
-    // staging.  With an even width and a 16-byte aligned frame, every pair
-    // of samples starting at an even column is one 16-byte cp.async: thread
-    // tid copies pair tid % 32 of rows tid / 32 + 16 m (half the copy
-    // instructions of the 8-byte form, which thread tid issues for column
-    // tid % 64 of rows tid / 64 + 8 m).
-    const bool wide = (w & 1) == 0 && (reinterpret_cast<uintptr_t>(rgbi) & 15u) == 0;
-    const int sj = wide ? 2 * (tid % 32) : tid % kRowTile;
-    const int sk0 = wide ? tid / 32 : tid / kRowTile;
-    const int srows = wide ? 2 * kStageRows : kStageRows;  // rows one staging pass covers
-    const uint16_t *srow = rgbi + ((int64_t)(r0 + sk0) * w + sj) * 4;
-    const int64_t srow_step = (int64_t)srows * w * 4;
-    auto stage = [&](int t) {
-        if (t < tiles) {
-            const int col = t * kRowTile + sj;
-            const uint16_t *src = srow + (int64_t)t * kRowTile * 4;
-            if (wide) {
+    // special warps: 0, 1 row adders (half the rows each), 2 failing positions
+    // and epochs
+    const int role = warp - kComputeWarps;
+    const int arow = role * (kRows / 2) + lane;
+    const bool adds = (role == 0 || role == 1) && lane < kRows / 2;
+    // a compute thread's column and row inside the 8-row blocks
+    const int j = tid % kRowTile, i = tid / kRowTile;
+    double rv = 0.0, ri = 0.0, rw = 0.0;
+    double den = 0.0, num = 0.0;  // role 2, lane rb < RB: epoch (r0 / 8 + rb) sums
+    // a compute thread's samples of tiles t .. t + 2 (visible | IR << 16) and
+    // the ones of tile t + 3 on their way
+    uint32_t s0[RB], s1[RB], s2[RB];
+    uint2 in[RB];
+    auto request = [&](int t) {
+        const int col = t * kRowTile + j;
 #pragma unroll
-                for (int m = 0; m < (kRows + 2 * kStageRows - 1) / (2 * kStageRows); ++m) {
-                    const int k = sk0 + 2 * kStageRows * m;
-                    if (k < kRows && r0 + k < h && col < active_width)
-                        cp_async16(&S.raw[t & 1][k][sj], src);
-                    src += srow_step;
-                }
-            } else {
-#pragma unroll
-                for (int m = 0; m < kRows / kStageRows; ++m) {
-                    const int k = sk0 + kStageRows * m;
-                    if (r0 + k < h && col < active_width) cp_async8(&S.raw[t & 1][k][sj], src);
-                    src += srow_step;
-                }
-            }
+        for (int m = 0; m < RB; ++m) {
+            const int row = r0 + m * 8 + i;
+            in[m] = make_uint2(0u, 0xFFFF0000u);  // outside: not failing
+            if (row < h && col < active_width)
+                in[m] = reinterpret_cast<const uint2 *>(rgbi)[(int64_t)row * w + col];
         }
-        asm volatile("cp.async.commit_group;\n" ::);
     };
-    stage(0);
-    double rv = 0.0, ri = 0.0, rw = 0.0;     // row r0 + lane
-    double rv2 = 0.0, ri2 = 0.0, rw2 = 0.0;  // row r0 + 32 + lane (lanes < kRows - 32)
-    const int lane2 = lane < kRows - 32 ? lane + 32 : lane;
-    double den = 0.0, num = 0.0;  // lane rb < kRowBlocks: epoch (r0 / 8 + rb) sums
-    for (int t = 0; t <= tiles; ++t) {
-        asm volatile("cp.async.wait_group 0;\n" ::);
-        __syncthreads();  // tile t staged; tile t-1's products complete
-        stage(t + 1);
-        const int col0 = t * kRowTile;
-        const int bt = t & 1;
-        if (t < tiles && warp >= 1) {
-            // first failing IR position of each cell (row-major inside the cell)
-            for (int ci = warp - 1; ci < kTileCells; ci += kRowWarps - 1) {
-                const int rb = ci >> 3, cc = ci & 7;
-                const int cell = t * 8 + cc;
-                if (cell >= cells) continue;  // warp-uniform
-                bool fail[2];
+    auto take = [&](uint32_t (&s)[RB]) {
 #pragma unroll
-                for (int hlf = 0; hlf < 2; ++hlf) {
-                    const int pidx = lane + 32 * hlf, i = pidx >> 3, j = pidx & 7;
-                    const int row = r0 + rb * 8 + i;
-                    fail[hlf] = row < h &&
-                                !(thr < (double)(S.raw[bt][rb * 8 + i][cc * 8 + j].y >> 16));
-                }
-                const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, fail[0]);
-                const uint32_t b1 = __ballot_sync(0xFFFFFFFFu, fail[1]);
-                if (lane == 0)
-                    S.fp[rb][cc] = b0 ? __ffs(b0) - 1 : (b1 ? 32 + __ffs(b1) - 1 : 64);
-            }
+        for (int m = 0; m < RB; ++m) s[m] = (in[m].x & 0xFFFFu) | (in[m].y & 0xFFFF0000u);
+    };
+    auto failing = [&](int t, const uint32_t (&s)[RB]) {
+        uint32_t mine = 0;
+#pragma unroll
+        for (int m = 0; m < RB; ++m) {
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, (s[m] >> 16) <= kIrLastFailing);
+            if (lane == m) mine = b;
         }
-        __syncthreads();  // fail positions of tile t visible
-        if (t < tiles && warp >= 1 && warp <= kProductWarps) {
-            // fixed trip count, fully unrolled: every LUT gather of the
-            // thread's pixels is in flight before the first product
-            constexpr int kStride = kProductWarps * 32;
-            constexpr int kPerThread = (kRows * kRowTile + kStride - 1) / kStride;
-            const int q0 = tid - 32;
-            float lv[kPerThread], li[kPerThread];
-            uint32_t wir[kPerThread];
-            bool use[kPerThread];
-#pragma unroll
-            for (int m = 0; m < kPerThread; ++m) {
-                const int q = q0 + m * kStride;
-                const int k = q / kRowTile, j = q % kRowTile;
-                const int row = r0 + k, col = col0 + j;
-                use[m] = q < kRows * kRowTile && row < h && col < active_width &&
-                         (row & 7) * 8 + (col & 7) < S.fp[k >> 3][j >> 3];
-                const uint2 px = use[m] ? S.raw[bt][k][j] : make_uint2(0u, 0u);
-                wir[m] = px.y >> 16;
-                lv[m] = __ldg(lut + (px.x & 0xFFFFu));
-                li[m] = __ldg(lut + wir[m]);
-            }
-#pragma unroll
-            for (int m = 0; m < kPerThread; ++m) {
-                const int q = q0 + m * kStride;
-                if (q < kRows * kRowTile) {
-                    const int k = q / kRowTile, j = q % kRowTile;
-                    double pv = 0.0, pi = 0.0, pw = 0.0;
-                    if (use[m]) {
-                        const double weight = (double)((uint64_t)wir[m] * wir[m]);
-                        pv = weight * (double)lv[m];
-                        pi = weight * (double)li[m];
-                        pw = weight;
-                    }
-                    S.p[bt][0][k][j] = pv;
-                    S.p[bt][1][k][j] = pi;
-                    S.p[bt][2][k][j] = pw;
-                }
-            }
-        }
-        if (t < tiles && warp >= 1) {
-            // quadrant trees: one per thread of warps 1..kTileCells/4 (cells x 8)
-            const int z = tid - 32;
-            if (z < kTileCells * 8) {
-                const int cl = z >> 3, rb = cl >> 3, cc = cl & 7;
-                const int blk = (r0 >> 3) + rb, cell = t * 8 + cc;
-                if (blk < ne && cell < cells && S.fp[rb][cc] == 64)
-                    S.qv[bt][cl][z & 7] = quadrant_value(
-                        [&](int i, int j) { return S.raw[bt][rb * 8 + i][cc * 8 + j]; }, lut,
-                        z & 7);
-            }
-            if (warp == kRowWarps - 1) {  // lane = tile cell: status and raw total
-                for (int cl = lane; cl < kTileCells; cl += 32) {
-                    const int rb = cl >> 3, cc = cl & 7;
-                    const int blk = (r0 >> 3) + rb, cell = t * 8 + cc;
-                    int flag = 0;
-                    if (blk < ne && cell < cells) flag = S.fp[rb][cc] == 64 ? 2 : 1;
+        if (lane < RB) S.failing[t & 1][lane][j >> 5][i] = mine;
+    };
+    if (warp < kComputeWarps) {
+        request(0);
+        take(s1);
+        request(1);
+        failing(0, s1);
+        take(s2);
+        request(2);
+    }
+    for (int t = -1; t <= tiles + 2; ++t) {
+        // tile t + 1's failing samples and tile t's failing positions known,
+        // tile t - 1's products and responses, tile t - 2's trees and tile
+        // t - 3's terms complete
+        __syncthreads();
+        if (warp < kComputeWarps) {
+            const int bt = t & 1;
+            auto trees = [&] {
+                const int u = t - 1;
+                if (u < 0 || u >= tiles || tid >= kCells * 8) return;
+                // one tree per thread (cells x 8)
+                const int cl = tid >> 3, rb = cl >> 3, cc = cl & 7, which = tid & 7;
+                if (u * 8 + cc >= cells || S.cell[u & 3][cl] != 2u) return;
+                const int q = which & 3, qy = rb * 8 + (q >> 1) * 4, qx = cc * 8 + (q & 1) * 4;
+                const float *r = reinterpret_cast<const float *>(&S.resp[u & 1][qy][qx]) +
+                                 (which >> 2);
+                S.qv[u & 1][cl][which] = quadrant_tree(
+                    [&](int y, int x) { return r[2 * (y * kRowPitch + x)]; });
+                if (which >> 2) {
                     uint32_t total = 0;
-                    if (flag == 2) {
-#pragma unroll 8
-                        for (int i = 0; i < 64; ++i)
-                            total += S.raw[bt][rb * 8 + (i >> 3)][cc * 8 + (i & 7)].y >> 16;
-                    }
-                    S.flag[bt][cl] = flag;
-                    S.rsum[bt][cl] = total;
+#pragma unroll
+                    for (int y = 0; y < 4; ++y)
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) total += S.ir[u & 1][qy + y][qx + x];
+                    S.qsum[u & 1][cl][q] = total;
                 }
-            }
-        }
-        if (warp == 0 && t > 0) {
-            // finish the previous tile's epoch cells (lane = tile cell)
-            const int u = t - 1, ub = u & 1;
-            for (int cl = lane; cl < kTileCells; cl += 32) {
-                const int flag = S.flag[ub][cl];
-                S.tok[cl] = flag == 2;
-                if (flag == 2) {
+            };
+            // tile t - 2's epoch cells, one quadrant per thread, on the warps
+            // that compute no tree
+            static_assert(kCells * 12 <= kComputeWarps * 32, "a thread for every tree and term");
+            auto finish = [&] {
+                const int u = t - 2, ub = u & 1, z = tid - kCells * 8;
+                if (u < 0 || u >= tiles || z < 0 || z >= kCells * 4) return;
+                const int cl = z >> 2, q = z & 3;
+                const bool pass = u * 8 + (cl & 7) < cells && S.cell[u & 3][cl] == 2u;
+                if (q == 0) S.tok[ub][cl] = pass;
+                if (pass) {
                     const float *qv = S.qv[ub][cl];
                     const float vq[4] = {qv[0], qv[1], qv[2], qv[3]};
                     const float iq[4] = {qv[4], qv[5], qv[6], qv[7]};
-                    double2 terms[4];
-                    finish_terms(vq, iq, S.rsum[ub][cl], terms);
+                    const uint32_t *qs = S.qsum[ub][cl];
+                    S.tq[ub][cl][q] = finish_term(vq, iq, qs[0] + qs[1] + qs[2] + qs[3], q);
+                }
+            };
+            // s0, s1 move on to tiles t, t + 1, and s2 takes tile t + 2
+            const bool here = t >= 0 && t < tiles;
+            float lv[RB], li[RB];
+            uint32_t wir[RB];
+            if (here) {
+                // every gather is in flight before the trees are computed
+                const int pos = i * 8 + (j & 7);
+                const bool inside = t * kRowTile + j < active_width;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) S.tq[cl][q] = terms[q];
+                for (int m = 0; m < RB; ++m) {
+                    const bool use = inside && r0 + m * 8 + i < h && pos < S.fp[bt][m][j >> 3];
+                    // a cell used for its trees passes whole
+                    const uint32_t px = use ? s0[m] : 0u;
+                    wir[m] = px >> 16;
+                    lv[m] = __ldg(lut + (px & 0xFFFFu));
+                    li[m] = __ldg(lut + wir[m]);
                 }
             }
-            __syncwarp();
-            // the epoch sums (producer_parameters.py epoch cell order): cells
-            // in column order, quadrants in order, passing cells only
-            if (lane < kRowBlocks) {
+            failing(t + 2, s2);
+            trees();
+            finish();
+            if (here) {
+#pragma unroll
+                for (int m = 0; m < RB; ++m) {
+                    const int k = m * 8 + i;
+                    // a sample that is not used has weight 0 and a finite
+                    // response: its products are zeros
+                    const double weight = (double)(wir[m] * wir[m]);  // below 2^32
+                    S.p[bt][0][k][j] = weight * (double)lv[m];
+                    S.p[bt][1][k][j] = weight * (double)li[m];
+                    S.resp[bt][k][j] = make_float2(lv[m], li[m]);
+                    S.ir[bt][k][j] = wir[m];
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < RB; ++m) {
+                s0[m] = s1[m];
+                s1[m] = s2[m];
+            }
+            take(s2);
+            request(t + 4);
+            continue;
+        }
+        if (adds) {
+            const int u = t - 1, ub = u & 1;
+            if (u >= 0 && u < tiles) {
+                // the ordered row sums (one row per lane)
+                const int n = min(kRowTile, active_width - u * kRowTile);
+                const double *pv = S.p[ub][0][arow];
+                const double *pi = S.p[ub][1][arow];
+                const uint32_t *pw = S.ir[ub][arow];
+                auto add = [&](int c) {
+                    rv += pv[c];
+                    ri += pi[c];
+                    rw += (double)(pw[c] * pw[c]);  // below 2^32
+                };
+                if (n == kRowTile) {
+#pragma unroll 16
+                    for (int c = 0; c < kRowTile; ++c) add(c);
+                } else {
+                    for (int c = 0; c < n; ++c) add(c);
+                }
+            }
+        } else if (role == 2) {
+            const int v = t + 1;
+            if (v < tiles) {
+                // first failing IR position of each cell (row-major inside it)
+                for (int cl = lane; cl < kCells; cl += 32) {
+                    const int rb = cl >> 3, cc = cl & 7;
+                    const uint32_t *f = S.failing[v & 1][rb][cc >> 2];
+                    int fp = 64;
+#pragma unroll
+                    for (int y = 7; y >= 0; --y) {
+                        const uint32_t m = (f[y] >> ((cc & 3) * 8)) & 0xFFu;
+                        if (m) fp = y * 8 + __ffs(m) - 1;
+                    }
+                    S.fp[v & 1][rb][cc] = fp;
+                    S.cell[v & 3][cl] = (r0 >> 3) + rb < ne ? (fp == 64 ? 2u : 1u) : 0u;
+                }
+            }
+            if (t >= 3 && lane < RB) {
+                // the epoch sums (producer_parameters.py epoch cell order):
+                // cells in column order, quadrants in order, passing cells only
+                const int vb = (t - 3) & 1;
+#pragma unroll
                 for (int cc = 0; cc < 8; ++cc) {
                     const int cl = lane * 8 + cc;
-                    if (S.tok[cl]) {
+                    if (S.tok[vb][cl]) {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
-                            den += S.tq[cl][q].x;
-                            num += S.tq[cl][q].y;
+                            den += S.tq[vb][cl][q].x;
+                            num += S.tq[vb][cl][q].y;
                         }
                     }
                 }
             }
-            __syncwarp();
-            // the ordered row sums of rows 0..31 (one row per lane)
-            const int n = min(kRowTile, active_width - u * kRowTile);
-            const double *pv = S.p[u & 1][0][lane];
-            const double *pi = S.p[u & 1][1][lane];
-            const double *pw = S.p[u & 1][2][lane];
-            if (n == kRowTile) {
-#pragma unroll 16
-                for (int j = 0; j < kRowTile; ++j) {
-                    rv += pv[j];
-                    ri += pi[j];
-                    rw += pw[j];
-                }
-            } else {
-                for (int j = 0; j < n; ++j) {
-                    rv += pv[j];
-                    ri += pi[j];
-                    rw += pw[j];
-                }
-            }
-        }
-        if (warp == kRowWarps - 1 && t > 0 && lane < kRows - 32) {
-            // the ordered row sums of rows 32..kRows-1, beside warp 0 (the
-            // previous tile's products stay in their buffer until tile t+1's)
-            const int u = t - 1;
-            const int n = min(kRowTile, active_width - u * kRowTile);
-            const double *pv2 = S.p[u & 1][0][lane2];
-            const double *pi2 = S.p[u & 1][1][lane2];
-            const double *pw2 = S.p[u & 1][2][lane2];
-            for (int j = 0; j < n; ++j) {
-                rv2 += pv2[j];
-                ri2 += pi2[j];
-                rw2 += pw2[j];
-            }
         }
     }
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    const int row = r0 + lane;
-    if (warp == 0 && row < h) {
-        b.row_sums[row] = rv;
-        b.row_sums[h + row] = ri;
-        b.row_sums[2 * h + row] = rw;
-    }
-    const int row2 = r0 + 32 + lane;
-    if (warp == kRowWarps - 1 && lane < kRows - 32 && row2 < h) {
-        b.row_sums[row2] = rv2;
-        b.row_sums[h + row2] = ri2;
-        b.row_sums[2 * h + row2] = rw2;
+    if (adds && r0 + arow < h) {
+        b.row_sums[r0 + arow] = rv;
+        b.row_sums[h + r0 + arow] = ri;
+        b.row_sums[2 * h + r0 + arow] = rw;
     }
     const int e = (r0 >> 3) + lane;
-    if (warp == 0 && lane < kRowBlocks && e < ne) {
+    if (role == 2 && lane < RB && e < ne) {
         b.add[e] = (float)den;
         b.add[ne + e] = (float)num;
     }
 }
 
-// Cumulative row sums (3 binary64 chains) and the epoch p1/p2 chain.  Warp
-// 1 walks the epoch chain on its own.  The other warps stream the row sums
-// through shared memory in chunks (synchronising on a named barrier that
-// warp 1 does not take part in), and threads 0..2 each walk one chain.
+// Cumulative row sums (3 binary64 chains), the epoch p1/p2 chain and the
+// stage table in one block, pipelined over chunks of 1024 rows (128 epochs):
+// in one iteration warp 0 runs the chains of chunk c in place in shared
+// memory, warp 1 the epochs of chunk c, and the other warps load chunk c + 1
+// and write the stage records of chunk c - 1.  The cumulative chain bounds
+// it: 13 cycles per row (load, 8-cycle add, store) against 26 when the
+// chain's thread also stored to global memory (80 us on a native frame).
 constexpr int kScanChunk = 1024;
 constexpr int kScanThreads = 256;
-constexpr int kScanLoaders = kScanThreads - 32;
-
-constexpr int kEpochChunk = 1024;
+constexpr int kScanHelpers = kScanThreads - 64;
+constexpr int kEpochChunk = kScanChunk / 8;
 
 struct ScanSmem {
-    double v[2][3][kScanChunk];
-    float add[2][kEpochChunk];     // the epoch chain's inputs, staged by warp 1
-    double sum[2][kEpochChunk];    // the chain's binary64 sums (den, num) per epoch
-    float q[2][kEpochChunk];       // (p1, p2) of epochs with a nonzero denominator
-    uint8_t defined[kEpochChunk];  // 1 when the epoch's denominator is nonzero
+    // [chunk % 3][chain]: row sums, then cumulative; the chains start four banks
+    // apart (three lanes walk them side by side)
+    double v[3][3][kScanChunk + 2];
+    float add[2][kEpochChunk];        // the epoch chain's inputs, staged by warp 1
+    double sum[2][kEpochChunk];       // the chain's binary64 sums (den, num) per epoch
+    float q[2][2][kEpochChunk + 1];   // [chunk % 2]: (p1, p2) per epoch, after the pair
+                                      // before the chunk
+    uint8_t defined[kEpochChunk];     // 1 when the epoch's denominator is nonzero
 };
 
-__device__ __forceinline__ void scan_barrier() {
-    asm volatile("bar.sync 1, %0;\n" ::"n"(kScanLoaders) : "memory");
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_producer_scan(int h, int ne, ProducerBuffers b) {
+__global__ void __launch_bounds__(kScanThreads)
+    k_producer_scan(int h, int ne, float factor_b, ProducerBuffers b, fx_stage *stages,
+                    float *rows_out, uint32_t *err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ScanSmem &S = *reinterpret_cast<ScanSmem *>(smem_raw);
-    const int tid = threadIdx.x;
-    if (tid >= 32 && tid < 64) {
-        // the epoch chain: warp 1 stages each chunk of its inputs into shared
-        // memory (coalesced); lane 0 runs the accumulations, the warp the
-        // quotients (off the chain), lane 0 carries the last defined pair
-        const int lane = tid - 32;
-        float den = 0.0f, num = 0.0f, p1 = kInitialScale, p2 = kInitialScale;
-        for (int e0 = 0; e0 < ne; e0 += kEpochChunk) {
-            const int n = min(kEpochChunk, ne - e0);
-            for (int k = lane; k < n; k += 32) {
-                S.add[0][k] = b.add[e0 + k];
-                S.add[1][k] = b.add[ne + e0 + k];
-            }
-            __syncwarp();
-            // the float accumulations are the only dependence between
-            // epochs: lane 0 runs them alone and keeps each epoch's sums
-            if (lane == 0) {
-                for (int k = 0; k < n; ++k) {
-                    const double dw = (double)den + (double)S.add[0][k];
-                    const double nw = (double)num + (double)S.add[1][k];
-                    den = (float)dw;
-                    num = (float)nw;
-                    S.sum[0][k] = dw;
-                    S.sum[1][k] = nw;
-                }
-            }
-            __syncwarp();
-            // each epoch's quotient on its own lane
-            for (int k = lane; k < n; k += 32) {
-                const double dw = S.sum[0][k];
-                S.defined[k] = dw != 0.0;
-                if (dw != 0.0) {
-                    const double ratio = S.sum[1][k] / dw;
-                    S.q[1][k] = (float)ratio;
-                    S.q[0][k] = (float)((double)kScaleMultiplier * ratio);
-                }
-            }
-            __syncwarp();
-            // an epoch without a denominator keeps the last defined pair
-            if (lane == 0) {
-                for (int k = 0; k < n; ++k) {
-                    if (S.defined[k]) {
-                        p1 = S.q[0][k];
-                        p2 = S.q[1][k];
-                    }
-                    S.q[0][k] = p1;
-                    S.q[1][k] = p2;
-                }
-            }
-            __syncwarp();
-            for (int k = lane; k < n; k += 32) {
-                b.p_epoch[e0 + k] = S.q[0][k];
-                b.p_epoch[ne + e0 + k] = S.q[1][k];
-            }
-            __syncwarp();
-        }
-        return;
-    }
-    const int lt = tid < 32 ? tid : tid - 32;  // loader index, 0..kScanLoaders-1
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int chunks = (h + kScanChunk - 1) / kScanChunk;
+    const int ht = tid - 64;  // helper index
     auto load = [&](int c) {
         const int base = c * kScanChunk, n = min(kScanChunk, h - base);
-        for (int i = lt; i < 3 * kScanChunk; i += kScanLoaders) {
-            const int chain = i / kScanChunk, k = i % kScanChunk;
-            if (k < n) S.v[c & 1][chain][k] = b.row_sums[(int64_t)chain * h + base + k];
+        for (int chain = 0; chain < 3; ++chain)
+            for (int k = ht; k < n; k += kScanHelpers)
+                S.v[c % 3][chain][k] = b.row_sums[(int64_t)chain * h + base + k];
+    };
+    // stage record of row `row` (stage row + 1), from the chunk's shared state
+    auto record = [&](int c, int row, int stage) {
+        const int k = row - c * kScanChunk;
+        const double tw = S.v[c % 3][2][k];
+        float mv = kInitialVisibleMean, mi = kInitialInfraredMean;
+        if (tw != 0.0) {
+            mv = (float)(S.v[c % 3][0][k] / tw);
+            mi = (float)(S.v[c % 3][1][k] / tw);
         }
+        // epochs finalised at rows 7, 15, ...: (row + 1) / 8 of them, counted
+        // from the pair before the chunk
+        const int done = (row + 1) / 8 - c * kEpochChunk;
+        const float p1 = S.q[c & 1][0][done], p2 = S.q[c & 1][1][done];
+        if (rows_out && stage == row) {
+            rows_out[row] = p1;
+            rows_out[h + row] = p2;
+            rows_out[2 * h + row] = mv;
+            rows_out[3 * h + row] = mi;
+        }
+        fx_stage st;
+        const int rc = setter_stage(p1, p2, mv, mi, factor_b, &st);
+        if (rc != FX_OK) {
+            raise_error(err, (uint32_t)rc);
+            st = fx_stage{0.0f, 0.0f, 0.0f, 0, 0.0f, 0.0f, 0, 0};
+        }
+        stages[stage] = st;
     };
     double acc = 0.0;
-    if (chunks > 0) load(0);
-    scan_barrier();
-    for (int c = 0; c < chunks; ++c) {
-        if (c + 1 < chunks) load(c + 1);
-        if (tid < 3) {
-            const int base = c * kScanChunk, n = min(kScanChunk, h - base);
-            const double *src = S.v[c & 1][tid];
-            double *dst = b.cum + (int64_t)tid * h + base;
-            if (n == kScanChunk) {
-#pragma unroll 8
-                for (int k = 0; k < kScanChunk; ++k) {
-                    acc += src[k];
-                    dst[k] = acc;
+    float den = 0.0f, num = 0.0f, p1 = kInitialScale, p2 = kInitialScale;
+    if (warp >= 2) load(0);
+    __syncthreads();
+    for (int c = 0; c <= chunks; ++c) {
+        if (warp == 0) {
+            if (c < chunks && lane < 3) {
+                const int n = min(kScanChunk, h - c * kScanChunk);
+                double *v = S.v[c % 3][lane];
+                constexpr int kG = 16;  // loads and stores of a group around its adds
+                int k = 0;
+                for (; k + kG <= n; k += kG) {
+                    double x[kG];
+#pragma unroll
+                    for (int m = 0; m < kG; ++m) x[m] = v[k + m];
+#pragma unroll
+                    for (int m = 0; m < kG; ++m) {
+                        acc += x[m];
+                        x[m] = acc;
+                    }
+#pragma unroll
+                    for (int m = 0; m < kG; ++m) v[k + m] = x[m];
                 }
-            } else {
-                for (int k = 0; k < n; ++k) {
-                    acc += src[k];
-                    dst[k] = acc;
+                for (; k < n; ++k) {
+                    acc += v[k];
+                    v[k] = acc;
                 }
             }
+        } else if (warp == 1) {
+            if (c < chunks) {
+                const int e0 = c * kEpochChunk, n = max(0, min(kEpochChunk, ne - e0));
+                for (int k = lane; k < n; k += 32) {
+                    S.add[0][k] = b.add[e0 + k];
+                    S.add[1][k] = b.add[ne + e0 + k];
+                }
+                __syncwarp();
+                // the float accumulations are the only dependence between
+                // epochs: lane 0 runs them alone and keeps each epoch's sums
+                if (lane == 0) {
+                    S.q[c & 1][0][0] = p1;
+                    S.q[c & 1][1][0] = p2;
+#pragma unroll 8
+                    for (int k = 0; k < n; ++k) {
+                        const double dw = (double)den + (double)S.add[0][k];
+                        const double nw = (double)num + (double)S.add[1][k];
+                        den = (float)dw;
+                        num = (float)nw;
+                        S.sum[0][k] = dw;
+                        S.sum[1][k] = nw;
+                    }
+                }
+                __syncwarp();
+                // each epoch's quotient on its own lane
+                for (int k = lane; k < n; k += 32) {
+                    const double dw = S.sum[0][k];
+                    S.defined[k] = dw != 0.0;
+                    if (dw != 0.0) {
+                        const double ratio = S.sum[1][k] / dw;
+                        S.q[c & 1][1][k + 1] = (float)ratio;
+                        S.q[c & 1][0][k + 1] = (float)((double)kScaleMultiplier * ratio);
+                    }
+                }
+                __syncwarp();
+                // an epoch without a denominator keeps the last defined pair
+                for (int k0 = 0; k0 < n; k0 += 32) {
+                    const int k = k0 + lane;
+                    const bool has = k < n && S.defined[k];
+                    const uint32_t at =
+                        __ballot_sync(0xFFFFFFFFu, has) & (0xFFFFFFFFu >> (31 - lane));
+                    const float a = has ? S.q[c & 1][0][k + 1] : 0.0f;
+                    const float d = has ? S.q[c & 1][1][k + 1] : 0.0f;
+                    const int src = at ? 31 - __clz(at) : 0;
+                    const float a1 = __shfl_sync(0xFFFFFFFFu, a, src);
+                    const float d1 = __shfl_sync(0xFFFFFFFFu, d, src);
+                    const float o1 = at ? a1 : p1, o2 = at ? d1 : p2;
+                    if (k < n) {
+                        S.q[c & 1][0][k + 1] = o1;
+                        S.q[c & 1][1][k + 1] = o2;
+                    }
+                    p1 = __shfl_sync(0xFFFFFFFFu, o1, 31);
+                    p2 = __shfl_sync(0xFFFFFFFFu, o2, 31);
+                }
+            }
+        } else {
+            if (c + 1 < chunks) load(c + 1);
+            if (c > 0) {
+                const int base = (c - 1) * kScanChunk, n = min(kScanChunk, h - base);
+                for (int k = ht; k < n; k += kScanHelpers) record(c - 1, base + k, base + k);
+                // stages h + 1 .. h + 6 repeat the last row
+                if (c == chunks && ht < 6) record(c - 1, h - 1, h + ht);
+            }
         }
-        scan_barrier();
+        __syncthreads();
     }
 }
 
-// Per-row record fields: the four float32 values the setter reads.
-__device__ __forceinline__ void row_fields(int row, int ne, const ProducerBuffers &b, int h,
-                                           float &p1, float &p2, float &mv, float &mi) {
-    const double tw = b.cum[2 * h + row];
-    if (tw != 0.0) {
-        mv = (float)(b.cum[row] / tw);
-        mi = (float)(b.cum[h + row] / tw);
-    } else {
-        mv = kInitialVisibleMean;
-        mi = kInitialInfraredMean;
-    }
-    const int done = (row + 1) / 8;  // epochs finalised at rows 7, 15, ...
-    if (done > 0 && done <= ne) {
-        p1 = b.p_epoch[done - 1];
-        p2 = b.p_epoch[ne + done - 1];
-    } else {
-        p1 = kInitialScale;
-        p2 = kInitialScale;
-    }
+template <int RB>
+static cudaError_t rows_init() {
+    return cudaFuncSetAttribute(k_producer_rows<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(RowSmem<RB>));
 }
 
-__global__ void k_stage_table(int h, int ne, float factor_b, ProducerBuffers b, fx_stage *stages,
-                              float *rows_out, uint32_t *err) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x + 1;  // stage hit
-    if (s > h + 6) return;
-    const int row = min(s - 1, h - 1);
-    float p1, p2, mv, mi;
-    row_fields(row, ne, b, h, p1, p2, mv, mi);
-    if (rows_out && s <= h) {
-        rows_out[row] = p1;
-        rows_out[h + row] = p2;
-        rows_out[2 * h + row] = mv;
-        rows_out[3 * h + row] = mi;
-    }
-    fx_stage st;
-    const int rc = setter_stage(p1, p2, mv, mi, factor_b, &st);
-    if (rc != FX_OK) {
-        raise_error(err, (uint32_t)rc);
-        st = fx_stage{0.0f, 0.0f, 0.0f, 0, 0.0f, 0.0f, 0, 0};
-    }
-    stages[s - 1] = st;
+template <int RB>
+static void launch_rows(const uint16_t *rgbi, int h, int w, int aw, int cells, const float *lut,
+                        const ProducerBuffers &b, cudaStream_t stream) {
+    k_producer_rows<RB><<<(h + RB * 8 - 1) / (RB * 8), kRowWarps * 32, sizeof(RowSmem<RB>),
+                          stream>>>(rgbi, h, w, aw, cells, lut, b);
 }
+
+static int g_producer_sms = 148;
 
 cudaError_t producer_init() {
-    const cudaError_t e = cudaFuncSetAttribute(
-        k_producer_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowSmem));
-    if (e != cudaSuccess) return e;
+    int device = 0, sms = 0;
+    if (cudaGetDevice(&device) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
+        sms > 0)
+        g_producer_sms = sms;
+    const cudaError_t e[] = {rows_init<1>(), rows_init<2>(), rows_init<3>(), rows_init<4>(),
+                             rows_init<5>()};
+    static_assert(sizeof(RowSmem<kMaxRowBlocks>) <= 232448, "one block fits an SM's shared memory");
+    for (cudaError_t x : e)
+        if (x != cudaSuccess) return x;
     return cudaFuncSetAttribute(k_producer_scan, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(ScanSmem));
 }
@@ -640,15 +610,21 @@ cudaError_t launch_producer(const uint16_t *rgbi, int h, int w, const float *lut
     b.cum = (double *)take(3 * (size_t)h * sizeof(double));
     b.add = (float *)take(2 * (size_t)ne * sizeof(float));
     b.p_epoch = (float *)take(2 * (size_t)ne * sizeof(float));
-    k_producer_rows<<<(h + kRows - 1) / kRows, kRowWarps * 32, sizeof(RowSmem), stream>>>(rgbi, h, w, aw,
-                                                                               cells, lut, b);
+    // the fewest rows per block that still give every block its own SM: a
+    // tile's time falls with its rows, and a second wave of blocks costs as
+    // much as the first
+    const int want = ((h + 7) / 8 + g_producer_sms - 1) / g_producer_sms;
+    switch (want < kMaxRowBlocks ? want : kMaxRowBlocks) {
+    case 1: launch_rows<1>(rgbi, h, w, aw, cells, lut, b, stream); break;
+    case 2: launch_rows<2>(rgbi, h, w, aw, cells, lut, b, stream); break;
+    case 3: launch_rows<3>(rgbi, h, w, aw, cells, lut, b, stream); break;
+    case 4: launch_rows<4>(rgbi, h, w, aw, cells, lut, b, stream); break;
+    default: launch_rows<5>(rgbi, h, w, aw, cells, lut, b, stream); break;
+    }
     // the scan is one block: given priority, it starts as soon as the row
     // sums are done even when other frames' kernels have blocks pending
     cudaError_t e = launch_prio(k_producer_scan, dim3(1), dim3(kScanThreads), sizeof(ScanSmem),
-                                stream, priority, h, ne, b);
-    if (e != cudaSuccess) return e;
-    e = launch_prio(k_stage_table, dim3((h + 6 + 255) / 256), dim3(256), 0, stream, priority, h,
-                    ne, 1.0f, b, stages, rows_out, err);
+                                stream, priority, h, ne, 1.0f, b, stages, rows_out, err);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
