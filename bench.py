@@ -67,7 +67,7 @@ WALK_AVG_CHUNKS = 18     # most 256-channel chunks per segment on average (kWalk
 def launches_per_frame(h: int, w: int, sms: int) -> int:
     """Kernel launches of one plain pass (the library's launch sequence):
     producer 2, planes 1, stencil 1, startup 1, chain 4, walk 1 per wave + 1
-    rewalk, apply 3.  Waves are sized from the RNG-dependent list capacity,
+    rewalk, apply 1.  Waves are sized from the RNG-dependent list capacity,
     with four window blocks per SM."""
 
     sites = 6 * w + h * w
@@ -75,7 +75,7 @@ def launches_per_frame(h: int, w: int, sms: int) -> int:
     chunks = (capacity + 255) // 256
     reach = WALK_BLOCKS_PER_SM * sms * WALK_AVG_CHUNKS
     waves = (chunks + reach - 1) // reach
-    return 13 + waves
+    return 11 + waves
 
 
 def ncu_counter(kernel: str, name: str):

@@ -22,7 +22,6 @@ constexpr int kTileH = 16;       // padded planes cover whole 16-row tiles (the
                                  // stencil runs 8- or 16-row tiles)
 constexpr int kTileW = 32;       // stencil tile cols
 constexpr int kSegment = 1024;   // chain sites per scan segment
-constexpr int kSegThreads = 256; // threads per segment block
 
 // Device error word: the first failing status wins.
 __device__ __forceinline__ void raise_error(uint32_t *err, uint32_t code) {

@@ -895,6 +895,7 @@ __global__ void __launch_bounds__(32)
     uint32_t T = t0, E = 0;
     if (n < serial_below) {  // a short chain (or the serial mode): one lane from E = 0
         if (blockIdx.x) return;
+        if (n == 0 && lane == 0) extra[0] = ExtraWord{0u, 0u};  // read by every site's lookup
         b = p == 0 ? n : 0u;
     } else {
         // pieces of segment x of a wave take the places from start(x) / 2 + x

@@ -21,9 +21,9 @@
 //   5. the walk (fx_walk.cu) visits only the RNG-dependent channels: a
 //      multiply-add, a test and a conditional LCG step per channel,
 //      parallelised over segments by speculation.  Output: the running count of extra draws.
-//   6. k_apply: every public site recomputes its exact draws and values from
-//      its own start state g^(fixed + extra before it)(s0), in parallel, and
-//      emits public RGB16 with the counters.
+//   6. k_apply: every public site computes its values from its own start
+//      state g^(fixed + extra before it)(s0), in parallel, and emits public
+//      RGB16 with the counters.
 #include <algorithm>
 
 #include "fx_internal.cuh"
@@ -40,64 +40,10 @@ struct DevCounters {
     uint32_t walk_fallbacks;
     uint32_t walk_packed;              // written together with walk_fallbacks
     unsigned long long walk_stats[3];  // candidate steps, window sum, survivor sum
-    uint32_t su_base[6], su_amb[6];    // per startup row, for the last block's prefix
-    uint32_t su_done;                  // startup rows summed
-    unsigned long long apply_next;     // k_apply's next segment
+    uint32_t su_base[6], su_amb[6];    // per startup row, for the last block's chain
+    uint32_t apply_next;               // k_apply's next ticket
+    uint32_t apply_done;               // k_apply's finished blocks
 };
-
-// ---------------------------------------------------------------------------
-// Block scan helpers (256 threads)
-// ---------------------------------------------------------------------------
-
-// Exclusive scan of 64-bit values (packed counters) over a block of NT threads.
-template <int NT>
-__device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned long long v,
-                                                                    unsigned long long &total,
-                                                                    unsigned long long *warp_sums) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long w = (lane < NT / 32) ? warp_sums[lane] : 0ull;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < NT / 32) warp_sums[lane] = w;
-    }
-    __syncthreads();
-    const unsigned long long prefix = warp ? warp_sums[warp - 1] : 0ull;
-    total = warp_sums[NT / 32 - 1];
-    __syncthreads();
-    return prefix + x - v;
-}
-
-template <int NT, typename T>
-__device__ __forceinline__ T block_sum(T v, T *scratch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    T total = 0;
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < NT / 32; ++i) total += scratch[i];
-        scratch[0] = total;
-    }
-    __syncthreads();
-    total = scratch[0];
-    __syncthreads();
-    return total;
-}
-
-constexpr int kPer = kSegment / kSegThreads;  // sites per thread
 
 // Extra draws of the first `count` RNG-dependent channels (clamped to the
 // list capacity; an overflowing frame is rerun by the host).
@@ -107,16 +53,6 @@ __device__ __forceinline__ uint32_t extra_before(const ExtraWord *extra, uint32_
     const uint32_t i = (uint32_t)((int64_t)count < capacity ? (int64_t)count : capacity);
     const uint2 w = __ldg(reinterpret_cast<const uint2 *>(extra) + (i >> 5));
     return w.x + (uint32_t)__popc(w.y & ((1u << (i & 31u)) - 1u));
-}
-
-// Packed local (base << 16 | amb) of one thread's sites.
-__device__ __forceinline__ void load_meta(const uint8_t *meta, int64_t first, int64_t sites,
-                                          uint8_t m[kPer]) {
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        const int64_t s = first + i;
-        m[i] = (s < sites) ? meta[s] : 0;
-    }
 }
 
 // (fixed draws << 16) | RNG-dependent channels of the four sites of one
@@ -295,9 +231,10 @@ __device__ __forceinline__ SiteInfo site_info(int64_t site, int w, const uint16_
     return si;
 }
 
-// Affine jump tables: g_jump[j][d] = g^(d * 64^j) in T space, so any jump
-// below 2^36 draws is six table lookups and compositions.
-constexpr int kJumpDigits = 6;
+// Affine jump tables: g_jump[j][d] = g^(d * 64^j) in T space.  States repeat
+// after 2^24 draws, so the low four base-64 digits of a draw count give its
+// map on states.
+constexpr int kJumpDigits = 4;
 __device__ Affine g_jump[kJumpDigits][64];
 
 // ---------------------------------------------------------------------------
@@ -633,89 +570,36 @@ __global__ void __launch_bounds__(256, 4) k_coef(AmbEntry *__restrict__ entries,
 }
 
 // ---------------------------------------------------------------------------
-// The serial walk (one resident warp per frame; lane 0 walks)
+// Apply + emit, counters, final state
 // ---------------------------------------------------------------------------
 
-// ---------------------------------------------------------------------------
-// Startup counters, apply + emit, final state
-// ---------------------------------------------------------------------------
-
-// Startup counters: one block per startup row sums its attempted sites,
-// fixed draws and RNG-dependent channels; the last block to finish chains
-// the six rows (the extra draws of a row come from the walk's running count
-// at the row's ends).
-__global__ void k_startup_counts(const uint8_t *__restrict__ meta, int w,
-                                 const ExtraWord *__restrict__ extra, uint32_t s0,
-                                 DevCounters *ctr, int64_t capacity,
-                                 const uint32_t *__restrict__ err) {
-    __shared__ unsigned long long scratch[8];
-    __shared__ bool last;
-    if (pass_stopped(err)) return;
-    const int k = blockIdx.x;  // startup row 0..5
-    unsigned long long att = 0, base = 0, amb = 0;
-    for (int x = threadIdx.x; x < w; x += blockDim.x) {
-        const uint8_t m = meta[(int64_t)k * w + x];
-        att += (m >> 7) & 1u;
-        base += meta_base(m);
-        amb += meta_amb(m);
-    }
-    att = block_sum<256, unsigned long long>(att, scratch);
-    base = block_sum<256, unsigned long long>(base, scratch);
-    amb = block_sum<256, unsigned long long>(amb, scratch);
-    if (threadIdx.x == 0) {
-        ctr->su_attempted[k] = att;
-        ctr->su_base[k] = (uint32_t)base;
-        ctr->su_amb[k] = (uint32_t)amb;
-        __threadfence();
-        last = atomicAdd(&ctr->su_done, 1u) == 5u;
-    }
-    __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    __threadfence();
-    const volatile DevCounters *vc = ctr;
-    uint32_t a_run = 0, p_run = 0;
-    for (int r = 0; r < 6; ++r) {
-        const uint32_t rb = vc->su_base[r], ra = vc->su_amb[r];
-        const uint32_t e_start = extra_before(extra, a_run, capacity);
-        const uint32_t a_end = a_run + ra;
-        const uint32_t e_end = extra_before(extra, a_end, capacity);
-        ctr->su_advances[r] = (unsigned long long)rb + (e_end - e_start);
-        a_run = a_end;
-        p_run += rb;
-    }
-    const uint32_t e = extra_before(extra, a_run, capacity);
-    ctr->startup_base = p_run;
-    ctr->startup_amb = a_run;
-    ctr->startup_extra = e;
-    ctr->su_final_state = lcg_jump(s0, (uint64_t)p_run + e);
-}
-
-__device__ __forceinline__ bool emit_one(float v, const uint32_t *hi, const uint32_t *lo,
-                                         uint16_t &out) {
-    if (!isfinite(v)) return false;
-    double wv = (double)v + 0.5;
-    wv = (wv < 0.0) ? 0.0 : wv;
-    wv = (wv > 65535.0) ? 65535.0 : wv;
-    const uint32_t idx = (uint32_t)wv;  // truncation (output.py:61-73)
+// Emitted value of a table index (output.py:61-73).
+__device__ __forceinline__ uint16_t emit_index(uint32_t idx, const uint32_t *hi,
+                                               const uint32_t *lo) {
     const unsigned long long prod = (unsigned long long)hi[idx >> 8] * lo[idx & 0xFFu];
-    out = (uint16_t)((prod >> 20) - 1ull);
-    return true;
+    return (uint16_t)((prod >> 20) - 1ull);
 }
 
-// Identity emits: ident[v] = emit(lut[v]), the output of a channel whose
-// value is its original (every unattempted pixel, and the comparison emit of
-// an attempted one).  *bad is set when a LUT value is not finite.
+// Table index of a finite value: trunc(v + 0.5) clipped to 0..65535.  The
+// reference adds in binary64, where the sum is exact; v's integer and
+// fractional parts are exact in binary32, so this is the same index.
+__device__ __forceinline__ uint32_t emit_index_of(float v) {
+    const float c = fminf(fmaxf(v, 0.0f), 65535.0f);
+    const uint32_t u = (uint32_t)c;
+    return u + (c - (float)u >= 0.5f ? 1u : 0u);
+}
+
+// Identity emits: ident[v] = emit(lut[v]), the output of a channel whose value
+// is its original (every unattempted pixel, and the comparison emit of an
+// attempted one).  *bad is set when a LUT value is not finite.
 __global__ void k_identity(const float *__restrict__ lut, const uint32_t *__restrict__ hi,
                            const uint32_t *__restrict__ lo, uint16_t *__restrict__ ident,
                            uint32_t *bad) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= 65536) return;
-    uint16_t e = 0;
-    if (!emit_one(lut[v], hi, lo, e)) {
-        atomicOr(bad, 1u);
-        e = 0;
-    }
-    ident[v] = e;
+    const float x = lut[v];
+    if (!isfinite(x)) atomicOr(bad, 1u);
+    ident[v] = isfinite(x) ? emit_index(emit_index_of(x), hi, lo) : (uint16_t)0;
 }
 
 cudaError_t writer_identity_table(const float *lut, const uint32_t *hi, const uint32_t *lo,
@@ -727,6 +611,10 @@ cudaError_t writer_identity_table(const float *lut, const uint32_t *hi, const ui
 
 constexpr int kApplyBlocksPerSM = 5;  // k_apply's resident blocks per SM
 static int g_apply_blocks = kApplyBlocksPerSM * 148;
+
+// Powers of the LCG step for short jumps: g_short[j][d] = g^(d * 128^j) in T
+// space, so a jump below 2^14 draws is two lookups.
+__device__ Affine g_short[2][128];
 
 cudaError_t writer_init() {
     int device = 0, sms = 0;
@@ -744,26 +632,73 @@ cudaError_t writer_init() {
         }
         step = acc;
     }
-    return cudaMemcpyToSymbol(g_jump, tab, sizeof(tab));
+    cudaError_t e = cudaMemcpyToSymbol(g_jump, tab, sizeof(tab));
+    if (e != cudaSuccess) return e;
+    Affine brief[2][128];
+    Affine one{125u, 256u};  // g^(128^j)
+    for (int j = 0; j < 2; ++j) {
+        Affine acc{1u, 0u};
+        for (int d = 0; d < 128; ++d) {
+            brief[j][d] = acc;
+            acc = affine_compose(one, acc);
+        }
+        one = acc;
+    }
+    return cudaMemcpyToSymbol(g_short, brief, sizeof(brief));
 }
 
-__device__ __forceinline__ uint32_t jump_by_table(const Affine (*tab)[64], uint32_t s,
-                                                  uint64_t n) {
-    Affine r{1u, 0u};
-#pragma unroll
-    for (int j = 0; j < kJumpDigits; ++j) r = affine_compose(tab[j][(n >> (6 * j)) & 63u], r);
-    return ((r.a * (s << 8) + r.c) >> 8) & kLcgMask;
+// Every warp takes units of 256 sites, a quarter of a chain segment, with no
+// block barrier:
+//   * the segment's meta bytes give the chain offsets before the unit and of
+//     its sites, and the attempted sites are listed in the warp's shared
+//     memory;
+//   * the sites that were not attempted are emitted, one pixel per lane
+//     (their output is the identity emit);
+//   * the list is processed densely, one attempted site per lane, from its
+//     own start state: the segment's, advanced by the draws inside it.
+// A channel's classification and the walk's bit say which of its draws
+// decides its value, so at most one is evaluated, and none where the original
+// is copied.  The first six units are the startup rows' counts; the last block
+// to finish chains the rows and writes the final state.
+// Measured on a native frame with half its pixels attempted: 505 us as blocks
+// of 256 threads with a block scan, four pixels per thread, both draws of
+// every channel and a six-digit jump per site (564 warp instructions per 32
+// pixels, 357 now); 332 us so.  The gathers' L1 decides the rest: with the
+// samples staged in shared memory five blocks took 505 us and six 866, with a
+// 128 KB emit table instead of the two factor tables 420.
+constexpr int kApplyWarps = 8;
+constexpr int kApplySites = 256;  // sites of a unit
+static_assert(kSegment == 1024 && kApplySites == 32 * 8, "32 and 8 meta bytes per lane");
+
+__device__ void apply_final(const uint32_t *seg_base, const uint32_t *seg_amb, int64_t segments,
+                            const ExtraWord *extra, uint32_t s0, DevCounters *ctr, uint32_t *err,
+                            int64_t capacity) {
+    uint32_t a_run = 0, p_run = 0;
+    for (int r = 0; r < 6; ++r) {
+        const uint32_t rb = __ldcg(&ctr->su_base[r]), ra = __ldcg(&ctr->su_amb[r]);
+        const uint32_t e_start = extra_before(extra, a_run, capacity);
+        const uint32_t e_end = extra_before(extra, a_run + ra, capacity);
+        ctr->su_advances[r] = (unsigned long long)rb + (e_end - e_start);
+        a_run += ra;
+        p_run += rb;
+    }
+    const uint32_t e_su = extra_before(extra, a_run, capacity);
+    ctr->startup_base = p_run;
+    ctr->startup_amb = a_run;
+    ctr->startup_extra = e_su;
+    ctr->su_final_state = lcg_jump(s0, (uint64_t)p_run + e_su);
+    const uint32_t p_total = seg_base[segments];
+    const uint32_t a_total = seg_amb[segments];
+    const uint32_t e_total = extra_before(extra, a_total, capacity);
+    ctr->n_amb = a_total;
+    ctr->final_state = lcg_jump(s0, (uint64_t)p_total + e_total);
+    const unsigned long long expect =
+        (unsigned long long)(p_total - p_run) + (e_total - e_su);
+    if ((int64_t)a_total <= capacity && expect != __ldcg(&ctr->public_advances))
+        raise_error(err, FX_ERR_INTERNAL);
 }
 
-// Public sites: exact draws and values, emit, counters.  A block takes
-// 1024-site segments by ticket until none is left (one resident wave of
-// blocks; the LCG jump and emit tables are loaded once per block).  Phase 1
-// emits every site that was not attempted (its output is the identity emit)
-// and lists the attempted ones in shared memory; phase 2 processes that list
-// densely, each entry from its own start state g^(fixed + extra before
-// it)(s0), and checks the draws it makes against the classification and the
-// walk.
-__global__ void __launch_bounds__(kSegThreads, kApplyBlocksPerSM)
+__global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
     k_apply(const uint8_t *__restrict__ meta, const double *__restrict__ cand, int64_t sites,
             int w, const uint16_t *__restrict__ rgbi, const float *__restrict__ lut,
             const uint32_t *__restrict__ g_high, const uint32_t *__restrict__ g_low,
@@ -772,143 +707,241 @@ __global__ void __launch_bounds__(kSegThreads, kApplyBlocksPerSM)
             const ExtraWord *__restrict__ extra, uint32_t s0, uint16_t *__restrict__ rgb_out,
             uint8_t *__restrict__ changed_out, DevCounters *ctr, uint32_t *err,
             int64_t capacity) {
-    __shared__ uint32_t hi[256], lo[256];
-    __shared__ unsigned long long s_sums[kSegThreads / 32][4];
-    __shared__ Affine s_jump[kJumpDigits][64];
-    __shared__ uint32_t s_ref[kSegment], s_p[kSegment], s_a[kSegment];
-    __shared__ unsigned long long s_seg;
-    __shared__ unsigned long long ws64[kSegThreads / 32];
+    __shared__ Affine s_jump[2][128];
+    __shared__ uint32_t hi[256], lo[256];  // emit factors
+    // attempted sites: x = site in the segment | meta << 16, y = fixed draws
+    // before it in the segment | RNG-dependent channels before it << 16
+    __shared__ uint2 s_list[kApplyWarps][kApplySites];
+    __shared__ unsigned long long s_sums[kApplyWarps][4];
+    __shared__ bool s_last;
     if (pass_stopped(err)) return;  // cancelled: the output stays untouched
-    for (int i = threadIdx.x; i < 256; i += kSegThreads) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < 256; i += kApplyWarps * 32) {
+        s_jump[i >> 7][i & 127] = g_short[i >> 7][i & 127];
         hi[i] = g_high[i];
         lo[i] = g_low[i];
     }
-    for (int i = threadIdx.x; i < kJumpDigits * 64; i += kSegThreads)
-        s_jump[i / 64][i % 64] = g_jump[i / 64][i % 64];
+    __syncthreads();
     const int64_t su = 6 * (int64_t)w;
     const int64_t segs = (sites + kSegment - 1) / kSegment;
     const DitherConst dc = dither_const(p);
+    uint2 *list = s_list[warp];
     unsigned long long att = 0, written = 0, changed = 0, draws_total = 0;
     bool ok = true;
-    // segments by ticket: the tables above are loaded once per block
-    for (;;) {
-        __syncthreads();  // the previous segment's list and ticket are consumed
-        if (threadIdx.x == 0) s_seg = atomicAdd(&ctr->apply_next, 1ull);
-        __syncthreads();
-        const int64_t seg = (int64_t)s_seg;
-        if (seg >= segs) break;
-        const int64_t seg0 = seg * kSegment;
-        const int64_t first = seg0 + threadIdx.x * kPer;
-        uint8_t m[kPer];
-        load_meta(meta, first, sites, m);
-        // one block scan gives each thread its sites' chain offsets (fixed
-        // draws, RNG-dependent channels) and its first slot in the list of
-        // attempted public sites: (fixed << 40 | channels << 20 | attempted)
-        unsigned long long mine = 0;
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            const int64_t site = first + i;
-            const bool listed = site >= su && site < sites && (m[i] & 0x80u);
-            mine += ((unsigned long long)meta_base(m[i]) << 40) |
-                    ((unsigned long long)meta_amb(m[i]) << 20) | (listed ? 1ull : 0ull);
+    const int64_t units = 6 + segs * (kSegment / kApplySites);
+    // two units per ticket on large frames (the ticket counter is one address),
+    // one on small ones
+    const int grab = units > 8 * (int64_t)gridDim.x * kApplyWarps ? 2 : 1;
+    int64_t unit = 0;
+    for (int left = 0;; --left, ++unit) {
+        if (left == 0) {
+            uint32_t ticket = 0;
+            if (lane == 0) ticket = atomicAdd(&ctr->apply_next, 1u);
+            unit = (int64_t)__shfl_sync(0xFFFFFFFFu, ticket, 0) * grab;
+            left = grab;
         }
-        unsigned long long total;
-        const unsigned long long ex = block_exclusive_scan64<kSegThreads>(mine, total, ws64);
-        uint32_t P = seg_base[seg] + (uint32_t)(ex >> 40);
-        uint32_t A = seg_amb[seg] + (uint32_t)((ex >> 20) & 0xFFFFFu);
-        const uint32_t listed = (uint32_t)(total & 0xFFFFFu);
-
-        // ---- phase 1: identity emits; list the attempted sites ---------------
-        {
-            uint32_t slot = (uint32_t)(ex & 0xFFFFFu);
+        if (unit >= units) break;
+        if (unit < 6) {  // counts of a startup row
+            uint32_t a = 0, fixed = 0, amb = 0;
+            const uint8_t *row = meta + unit * w;
+#pragma unroll 4
+            for (int x = lane; x < w; x += 32) {
+                const uint32_t m = row[x];
+                const uint32_t k = packed_word(m);
+                a += m >> 7;
+                fixed += k >> 16;
+                amb += k & 0xFFFFu;
+            }
+            a = __reduce_add_sync(0xFFFFFFFFu, a);
+            fixed = __reduce_add_sync(0xFFFFFFFFu, fixed);
+            amb = __reduce_add_sync(0xFFFFFFFFu, amb);
+            if (lane == 0) {
+                ctr->su_attempted[unit] = a;
+                ctr->su_base[unit] = fixed;
+                ctr->su_amb[unit] = amb;
+            }
+            continue;
+        }
+        const int64_t seg = (unit - 6) / (kSegment / kApplySites);
+        const int part = (int)((unit - 6) % (kSegment / kApplySites));
+        const int64_t first = seg * kSegment + part * kApplySites;
+        if (first >= sites) continue;
+        // the state at the segment's first draw
+        const uint32_t seg_a = seg_amb[seg], seg_p = seg_base[seg];
+        // ---- meta: the segment's sites before the unit, this lane's 8 sites ---
+        uint32_t sum = 0, ahead = 0;
+        uint32_t m2[2] = {0u, 0u};
+        const int64_t mine = first + lane * 8, far = seg * kSegment + lane * 32;
+        if (first + kApplySites <= sites) {
+            if (lane < part * (kApplySites / 32)) {
+                const uint4 *q = reinterpret_cast<const uint4 *>(meta + far);
+                const uint4 u = q[0], v = q[1];
+                ahead = packed_word(u.x) + packed_word(u.y) + packed_word(u.z) +
+                        packed_word(u.w) + packed_word(v.x) + packed_word(v.y) +
+                        packed_word(v.z) + packed_word(v.w);
+            }
+            const uint2 v = *reinterpret_cast<const uint2 *>(meta + mine);
+            m2[0] = v.x;
+            m2[1] = v.y;
+        } else {  // the chain's last unit
+            if (lane < part * (kApplySites / 32))
+                for (int i = 0; i < 32; ++i) ahead += packed_word(meta[far + i]);
+            for (int i = 0; i < 8; ++i)
+                if (mine + i < sites) m2[i >> 2] |= (uint32_t)meta[mine + i] << (8 * (i & 3));
+        }
+        // attempted public sites of the lane (bit i: site i)
+        const int pub = (int)(su - mine < 0 ? 0 : (su - mine > 8 ? 8 : su - mine));
+        uint32_t bits = 0;
 #pragma unroll
-            for (int i = 0; i < kPer; ++i) {
-                const int64_t site = first + i;
-                const uint8_t mi = m[i];
-                if (site >= su && site < sites) {
-                    if (mi & 0x80u) {
-                        s_ref[slot] = ((uint32_t)mi << 16) | (uint32_t)(threadIdx.x * kPer + i);
-                        s_p[slot] = P;
-                        s_a[slot] = A;
-                        ++slot;
-                    } else {
-                        const int64_t pixel = site - su;
-                        const uint2 raw = reinterpret_cast<const uint2 *>(rgbi)[pixel];
-                        uint16_t *o = rgb_out + 3 * pixel;
-                        o[0] = __ldg(ident + (raw.x & 0xFFFFu));
-                        o[1] = __ldg(ident + (raw.x >> 16));
-                        o[2] = __ldg(ident + (raw.y & 0xFFFFu));
-                        if (changed_out) changed_out[pixel] = 0;
-                    }
-                }
-                P += meta_base(mi);
-                A += meta_amb(mi);
+        for (int q = 0; q < 2; ++q) {
+            sum += packed_word(m2[q]);
+            const uint32_t hi = (m2[q] >> 7) & 0x01010101u;
+            bits |= ((hi * 0x01020408u) >> 24 & 0xFu) << (4 * q);
+        }
+        bits &= 0xFFu << pub & 0xFFu;
+        const uint32_t listed = __popc(bits);
+        // fixed << 16 | RNG-dependent fits (at most 6144 and 3072 a segment)
+        uint32_t inc = sum, slot = listed;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            const uint32_t z = __shfl_up_sync(0xFFFFFFFFu, slot, o);
+            if (lane >= o) {
+                inc += y;
+                slot += z;
             }
         }
-        __syncthreads();
-
-        // ---- phase 2: attempted sites, densely ----------------------------------
-        for (uint32_t k = threadIdx.x; k < listed; k += kSegThreads) {
-            const uint32_t r = s_ref[k];
-            const uint8_t mi = (uint8_t)(r >> 16);
-            const int64_t site = seg0 + (r & 0xFFFFu);
-            const uint32_t pixel = (uint32_t)(site - su);  // H*W < 2^31
-            const uint32_t y = pixel / (uint32_t)w;
-            const uint2 raw = reinterpret_cast<const uint2 *>(rgbi)[pixel];
-            const float orig[3] = {__ldg(lut + (raw.x & 0xFFFFu)), __ldg(lut + (raw.x >> 16)),
-                                   __ldg(lut + (raw.y & 0xFFFFu))};
-            const bool floor_enabled = p.driver_gate_primary || stages[y + 6].gate_secondary;
-            float values[3] = {orig[0], orig[1], orig[2]};
-            const uint32_t Ak = s_a[k];
-            const int amb = meta_amb(mi);
-            const uint32_t e_before = extra_before(extra, Ak, capacity);
-            const uint32_t redraws = extra_before(extra, Ak + amb, capacity) - e_before;
-            uint32_t state = jump_by_table(s_jump, s0, (uint64_t)s_p[k] + e_before);
-            const double *cd = cand + 3 * site;
-            const double c3[3] = {cd[0], cd[1], cd[2]};
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, slot, 31);
+        uint32_t run = __reduce_add_sync(0xFFFFFFFFu, ahead) + inc - sum;
+        slot -= listed;
+        __syncwarp();  // the previous list is consumed
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t m = (m2[i >> 2] >> (8 * (i & 3))) & 0xFFu;
+            if ((bits >> i) & 1u) {
+                list[slot] = make_uint2((uint32_t)(part * kApplySites + lane * 8 + i) | (m << 16),
+                                        (run >> 16) | (run << 16));
+                ++slot;
+            }
+            run += packed_word(m);
+        }
+        // ---- sites that were not attempted: identity emits -------------------
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int64_t site = first + 32 * r + lane;
+            // the bits of site's lane say whether it was attempted
+            const uint32_t b = __shfl_sync(0xFFFFFFFFu, bits, 4 * r + (lane >> 3));
+            if (site >= su && site < sites && !((b >> (lane & 7)) & 1u)) {
+                const int64_t pixel = site - su;
+                const uint2 raw = reinterpret_cast<const uint2 *>(rgbi)[pixel];
+                uint16_t *o = rgb_out + 3 * pixel;
+                o[0] = __ldg(ident + (raw.x & 0xFFFFu));
+                o[1] = __ldg(ident + (raw.x >> 16));
+                o[2] = __ldg(ident + (raw.y & 0xFFFFu));
+                if (changed_out) changed_out[pixel] = 0;
+            }
+        }
+        if (total == 0) continue;
+        const uint32_t seg_e = extra_before(extra, seg_a, capacity);
+        uint32_t seg_t = s0 << 8;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {  // states repeat after 2^24 draws
+            const Affine f = g_jump[j][((seg_p + seg_e) >> (6 * j)) & 63u];
+            seg_t = f.a * seg_t + f.c;
+        }
+        __syncwarp();  // the list is complete
+        // ---- attempted sites, densely: one round's loads are in flight while
+        // the round before is computed ------------------------------------------
+        struct Site {
+            uint2 entry, raw, words;  // list entry, samples, extra draws
+            double cand[3];
+        };
+        auto fetch = [&](uint32_t k) {
+            Site q;
+            if (k < total) {
+                q.entry = list[k];
+                const int64_t site = seg * kSegment + (q.entry.x & 0xFFFFu);
+                q.raw = reinterpret_cast<const uint2 *>(rgbi)[site - su];
+                const uint32_t a =
+                    (uint32_t)min((int64_t)(seg_a + (q.entry.y >> 16)), capacity);
+                q.words = __ldg(reinterpret_cast<const uint2 *>(extra) + (a >> 5));
+#pragma unroll
+                for (int c = 0; c < 3; ++c) q.cand[c] = cand[3 * site + c];
+            }
+            return q;
+        };
+        Site cur = fetch(lane);
+        for (uint32_t k = lane; k < total; k += 32) {
+            const Site q = cur;
+            cur = fetch(k + 32);
+            const uint8_t mi = (uint8_t)(q.entry.x >> 16);
+            // H*W < 2^31
+            const uint32_t pixel = (uint32_t)(seg * kSegment + (q.entry.x & 0xFFFFu) - su);
+            const uint32_t lanes[3] = {q.raw.x & 0xFFFFu, q.raw.x >> 16, q.raw.y & 0xFFFFu};
+            uint16_t e0[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) e0[c] = __ldg(ident + lanes[c]);
+            // the walk's bits of this site's RNG-dependent channels, and the
+            // extra draws before them
+            const uint32_t a = (uint32_t)min((int64_t)(seg_a + (q.entry.y >> 16)), capacity);
+            const uint32_t sh = a & 31u;
+            uint32_t redraw = q.words.y >> sh;
+            if (sh + (uint32_t)meta_amb(mi) > 32u)
+                redraw |= __ldg(&extra[(a >> 5) + 1].bits) << (32u - sh);
+            const uint32_t n = (q.entry.y & 0xFFFFu) + q.words.x +
+                               (uint32_t)__popc(q.words.y & ((1u << sh) - 1u)) - seg_e;
+            const Affine f0 = s_jump[0][n & 127u], f1 = s_jump[1][(n >> 7) & 127u];
+            uint32_t state = (f1.a * (f0.a * seg_t + f0.c) + f1.c) >> 8;
+            const bool floor_enabled =
+                p.driver_gate_primary || stages[pixel / (uint32_t)w + 6].gate_secondary;
             bool valid = true;
+            if ((mi & 0x3Fu) == 0u)  // no draws: all channels outside the bounds, or invalid
 #pragma unroll
-            for (int c = 0; c < 3; ++c) valid &= isfinite(c3[c]) && c3[c] > 0.0;
-            uint32_t draws = 0;
-            if (valid) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    int drew;
-                    const DitherChannel ch = dither_channel(c3[c], p.dither_scales[c], dc);
-                    const double firstd = dither_draw(ch, dc, state, drew);
-                    draws += drew;
-                    if (floor_enabled && c3[c] + firstd <= (double)orig[c]) {
-                        values[c] = orig[c];
-                    } else {
-                        double d = firstd;
-                        if (floor_enabled) {
-                            d = dither_draw(ch, dc, state, drew);
-                            draws += drew;
-                        }
-                        values[c] = (float)(c3[c] + d);
-                    }
-                }
-            }
-            if ((int64_t)(Ak + amb) <= capacity && draws != (uint32_t)meta_base(mi) + redraws)
-                raise_error(err, FX_ERR_INTERNAL);
-            att += 1;
-            draws_total += draws;
-            written += (values[0] != orig[0] || values[1] != orig[1] || values[2] != orig[2]);
-            const uint16_t e0[3] = {__ldg(ident + (raw.x & 0xFFFFu)), __ldg(ident + (raw.x >> 16)),
-                                    __ldg(ident + (raw.y & 0xFFFFu))};
-            uint16_t e[3];
+                for (int c = 0; c < 3; ++c) valid &= isfinite(q.cand[c]) && q.cand[c] > 0.0;
+            bool wrote = false, differs = false;
+            uint16_t *o = rgb_out + 3 * (int64_t)pixel;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                e[c] = e0[c];
-                if (!(values[c] == orig[c])) ok &= emit_one(values[c], hi, lo, e[c]);
+                int code = meta_code(mi, c);
+                if (code == 3) {  // one draw and a copy, or two
+                    code = (redraw & 1u) ? 2 : 1;
+                    redraw >>= 1;
+                }
+                // the draw that decides the value (the first draw copies the
+                // original where the floor gate is on)
+                if (code >= 1) state = (125u * state + 1u) & kLcgMask;
+                if (code == 2) state = (125u * state + 1u) & kLcgMask;
+                draws_total += (uint32_t)code;
+                uint16_t e = e0[c];
+                if (valid && !(code == 1 && floor_enabled)) {
+                    const double c3 = q.cand[c];
+                    float v;
+                    bool copied = false;
+                    if (code == 0) {
+                        const float orig = __ldg(lut + lanes[c]);
+                        copied = floor_enabled && c3 <= (double)orig;
+                        v = (float)c3;
+                    } else {
+                        const DitherChannel ch = dither_channel(c3, p.dither_scales[c], dc);
+                        const double d = dither_raw_delta(ch.cand, ch.envelope, ch.span, state);
+                        const double moved = ch.cand + d;
+                        v = (float)(c3 + ((dc.low < moved && moved < dc.high) ? d : 0.0));
+                    }
+                    if (!copied) {
+                        if (!isfinite(v)) ok = false;
+                        else e = emit_index(emit_index_of(v), hi, lo);
+                        // an output that differs was written; one that does not
+                        // may still come from another value
+                        wrote |= e != e0[c] || !(v == __ldg(lut + lanes[c]));
+                    }
+                }
+                differs |= e != e0[c];
+                o[c] = e;
             }
-            const bool ch = (e[0] != e0[0]) || (e[1] != e0[1]) || (e[2] != e0[2]);
-            changed += ch;
-            uint16_t *o = rgb_out + 3 * (int64_t)pixel;
-            o[0] = e[0];
-            o[1] = e[1];
-            o[2] = e[2];
-            if (changed_out) changed_out[pixel] = ch ? 1 : 0;
+            att += 1;
+            written += wrote;
+            changed += differs;
+            if (changed_out) changed_out[pixel] = differs ? 1 : 0;
         }
     }
     if (!ok) raise_error(err, FX_ERR_NONFINITE_WORK);
@@ -918,35 +951,26 @@ __global__ void __launch_bounds__(kSegThreads, kApplyBlocksPerSM)
     for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v4[q] += __shfl_down_sync(0xFFFFFFFFu, v4[q], o);
-    if ((threadIdx.x & 31) == 0)
+    if (lane == 0)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) s_sums[threadIdx.x >> 5][q] = v4[q];
+        for (int q = 0; q < 4; ++q) s_sums[warp][q] = v4[q];
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long t4[4] = {0, 0, 0, 0};
-        for (int wq = 0; wq < kSegThreads / 32; ++wq)
+        for (int wq = 0; wq < kApplyWarps; ++wq)
 #pragma unroll
             for (int q = 0; q < 4; ++q) t4[q] += s_sums[wq][q];
         if (t4[0]) atomicAdd(&ctr->attempted, t4[0]);
         if (t4[1]) atomicAdd(&ctr->written, t4[1]);
         if (t4[2]) atomicAdd(&ctr->changed, t4[2]);
         if (t4[3]) atomicAdd(&ctr->public_advances, t4[3]);
+        __threadfence();
+        s_last = atomicAdd(&ctr->apply_done, 1u) == gridDim.x - 1u;
     }
-}
-
-__global__ void k_final(const uint32_t *__restrict__ seg_base, const uint32_t *__restrict__ seg_amb,
-                        int64_t segments, const ExtraWord *__restrict__ extra, uint32_t s0,
-                        DevCounters *ctr, uint32_t *err, int64_t capacity) {
-    if (pass_stopped(err)) return;
-    const uint32_t p_total = seg_base[segments];
-    const uint32_t a_total = seg_amb[segments];
-    const uint32_t e_total = extra_before(extra, a_total, capacity);
-    ctr->n_amb = a_total;
-    ctr->final_state = lcg_jump(s0, (uint64_t)p_total + e_total);
-    const unsigned long long expect =
-        (unsigned long long)(p_total - ctr->startup_base) + (e_total - ctr->startup_extra);
-    if ((int64_t)a_total <= capacity && expect != ctr->public_advances)
-        raise_error(err, FX_ERR_INTERNAL);
+    __syncthreads();
+    if (!s_last || threadIdx.x != 0) return;
+    __threadfence();
+    apply_final(seg_base, seg_amb, segs, extra, s0, ctr, err, capacity);
 }
 
 // ---------------------------------------------------------------------------
@@ -998,13 +1022,12 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
     marks.mark(6, stream);
     e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
-    k_startup_counts<<<6, 256, 0, stream>>>(meta, g.w, b.extra, s0 & kLcgMask, ctr,
-                                            b.capacity, err);
-    k_apply<<<(unsigned)std::min<int64_t>(segs, g_apply_blocks), kSegThreads, 0, stream>>>(
-        meta, cand, g.sites, g.w, rgbi, lut, high, low, ident, stages, p, b.seg_base, b.seg_amb,
-        b.extra, s0 & kLcgMask, rgb_out, changed_out, ctr, err, b.capacity);
-    k_final<<<1, 1, 0, stream>>>(b.seg_base, b.seg_amb, segs, b.extra, s0 & kLcgMask,
-                                 ctr, err, b.capacity);
+    const int64_t apply_blocks =
+        (segs * (kSegment / kApplySites) + 6 + kApplyWarps - 1) / kApplyWarps;
+    k_apply<<<(unsigned)std::min<int64_t>(apply_blocks, g_apply_blocks), kApplyWarps * 32, 0,
+              stream>>>(meta, cand, g.sites, g.w, rgbi, lut, high, low, ident, stages, p,
+                        b.seg_base, b.seg_amb, b.extra, s0 & kLcgMask, rgb_out, changed_out, ctr,
+                        err, b.capacity);
     marks.mark(7, stream);
     return cudaGetLastError();
 }
