@@ -73,8 +73,10 @@ def launches_per_frame(h: int, w: int, sms: int) -> int:
     sites = 6 * w + h * w
     capacity = max(65536, sites // 2)
     chunks = (capacity + 255) // 256
-    reach = WALK_BLOCKS_PER_SM * sms * WALK_AVG_CHUNKS
-    waves = (chunks + reach - 1) // reach
+    per_wave = WALK_BLOCKS_PER_SM * sms
+    waves = (chunks + per_wave * WALK_AVG_CHUNKS - 1) // (per_wave * WALK_AVG_CHUNKS)
+    if chunks >= 4 * per_wave * waves:  # long segments: two spare waves for misses
+        waves += 2
     return 11 + waves
 
 

@@ -22,8 +22,10 @@
 // lists (every survivor of the first list followed through the others), and
 // the block that completes the last group chains the exact E through the
 // groups and looks up every segment's exact entry count.  When E falls
-// outside a window that segment is walked exactly, so correctness never
-// depends on the prediction.  No block waits for another.
+// outside a window the wave ends there and the next one starts at that
+// segment, its windows centred on the exact count again (the launches hold a
+// few waves in reserve; without one left the segment is walked exactly), so
+// correctness never depends on the prediction.  No block waits for another.
 //
 // Every 512 channels a block also keeps its survivors (entry count and
 // state): from them k_rewalk starts one lane per 512 channels, in parallel,
@@ -45,9 +47,10 @@ constexpr int kWinBatch = 32 * kWinSlots;           // candidates a warp walks a
 // 2.7 M channels, and a channel's variance at most 1/4, so 4.5 standard
 // deviations either side (at most 7425 + 33 candidates) always fit.
 constexpr int kWinMax = 8192;
-// The first kWinFirst channels are walked by every warp on its own share of
-// the window, in batches of kWinBatch; about a quarter of a batch is left
-// then and waits in the warp's region of the list.
+// The first kWinFirst channels (the first chunk, where too many are left then)
+// are walked by every warp on its own share of the window, in batches of
+// kWinBatch; about a quarter of a batch is left then and waits in the warp's
+// region of the list.
 constexpr uint32_t kWinFirst = 64;
 constexpr int kWinRegion = 2 * kWinBatch;
 constexpr int kWinChunk = kWalkChunk;               // channels staged per chunk
@@ -56,15 +59,17 @@ constexpr uint32_t kPiece = 512;                    // channels per kept survivo
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr uint32_t kSerialBelow = 1024;             // short chains: one serial walk
 // The window half-width is kDefaultWindowSigmas (4.5) standard deviations of
-// the predicted entry count, plus 16.  A count outside its window costs one
-// exact serial walk of that segment and never changes a result; at 4.5 sigma
-// that happens for about 7e-6 of the segments.  fx_set_walk_window narrows
-// it, so tests can force such misses.
+// the predicted entry count, plus 16.  A count outside its window never
+// changes a result: it ends the wave, or costs one exact serial walk of that
+// segment (200 us for the longest).  Heavily damaged frames drift out of 4.5
+// sigma now and then and stay out for the rest of the wave: 239 segments and
+// 51.6 ms on one frame with exact walks alone, 4.6 ms with restarts.
+// fx_set_walk_window narrows the windows, so tests can force misses.
+constexpr uint32_t kSpareWaves = 2;  // launches beyond the waves a chain needs
 
 struct WalkState {
-    uint32_t e_wave;     // exact E at the start of the current wave
-    uint32_t waves;
-    uint32_t fallbacks;  // segments resolved by an exact serial walk
+    uint32_t waves;      // waves resolved
+    uint32_t fallbacks;  // misses: waves ended early and segments walked exactly
     uint32_t packed;     // segments whose settled phase ran two candidates per lane
     unsigned long long candidate_steps;  // window-walk work, for diagnostics
     unsigned long long window_sum;       // candidates started
@@ -232,6 +237,7 @@ struct WalkBuffers {
     const uint8_t *chunk_two;
     const ChunkStat *chunk_stat;
     WalkState *st;
+    uint2 *wave;           // per wave: first chunk, exact E there (one more: its end)
     SegWindow *windows;    // per segment of the chain
     uint32_t *e_in;        // per segment: exact entry count
     SegList *lists;        // per segment of a wave
@@ -244,9 +250,9 @@ struct WalkBuffers {
     uint32_t kept_size;
 };
 
-// Segments of wave w that hold channels (the last wave may be short).
-__device__ __forceinline__ uint32_t wave_segments(const WalkPlan &plan, uint32_t w) {
-    const uint32_t c0 = w * plan.wave_chunks;
+// Segments that hold channels of a wave that starts at chunk c0 (the last
+// wave may be short).
+__device__ __forceinline__ uint32_t wave_segments(const WalkPlan &plan, uint32_t c0) {
     if (c0 >= plan.chunks) return 0u;
     const uint32_t left = plan.chunks - c0;
     if (left >= plan.wave_chunks) return plan.segs;
@@ -261,7 +267,7 @@ __device__ __forceinline__ uint32_t wave_segments(const WalkPlan &plan, uint32_t
 
 // One segment's window walk: segment x of wave w, channels [i0, i1).
 __device__ __forceinline__ void window_block(const WalkBuffers &B, WindowSmem &S, uint32_t c_wave,
-                                             uint32_t i0, uint32_t i1, uint32_t j, uint32_t x,
+                                             uint32_t e0, uint32_t i0, uint32_t i1, uint32_t j, uint32_t x,
                                              uint32_t t0, double sigmas) {
     const uint32_t tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -307,7 +313,6 @@ __device__ __forceinline__ void window_block(const WalkBuffers &B, WindowSmem &S
             S.pred[warp][1] = var;
         }
     }
-    const uint32_t e0 = B.st->e_wave;
     asm volatile("cp.async.wait_group 1;\n" ::);
     __syncthreads();  // the prediction and the first chunk
     double center = 0.0, var = 0.0;
@@ -408,7 +413,7 @@ __device__ __forceinline__ void window_block(const WalkBuffers &B, WindowSmem &S
     auto slots_for = [](uint32_t n) { return (int)((n + 31u) / 32u); };
 
     // ---- the first channels, every warp on its share of the window -----------
-    const uint32_t first = min(kWinFirst, len);
+    uint32_t first = min(kWinFirst, len);
     const uint4 *ring0 = reinterpret_cast<const uint4 *>(S.ring[0]);
     const bool two0 = B.chunk_two[i0 / kWalkChunk] != 0;
     uint32_t wlo, count;
@@ -474,9 +479,10 @@ __device__ __forceinline__ void window_block(const WalkBuffers &B, WindowSmem &S
         }
         full |= mine > (uint32_t)kWinBatch;
         if (!__syncthreads_or(full)) break;
-        // Too many are left (a stretch of channels that hardly merges): half
-        // the window, at the risk of a miss.
-        half *= 0.5;
+        // Too many are left (a stretch of channels that hardly merges): more
+        // channels first, then half the window, at the risk of a miss.
+        if (first < min((uint32_t)kWinChunk, len)) first = min((uint32_t)kWinChunk, len);
+        else half *= 0.5;
     }
 
     // ---- the rest of the segment ---------------------------------------------
@@ -557,7 +563,8 @@ __device__ __forceinline__ void window_block(const WalkBuffers &B, WindowSmem &S
     block_compact();
     if (tid == 0 && len > kPiece) S.kept_at = atomicAdd(&B.st->kept_next, live);
 
-    uint32_t next_compact = 2 * kWinFirst;  // then 256, 512, every kPiece channels
+    uint32_t next_compact = first > kWinFirst ? kPiece : 2 * kWinFirst;  // then 256, 512,
+                                                                         // every kPiece channels
     int b = 0;
     for (uint32_t c0 = i0; c0 < i1; c0 += kWinChunk) {
         const uint32_t c1 = min(i1, c0 + (uint32_t)kWinChunk);
@@ -723,6 +730,7 @@ struct FinalSmem {
     uint32_t count[kMaxGroups];              // survivors of the first list
     SegWindow win[kMaxGroups + 1];           // its window (then an empty one)
     uint32_t pick[kMaxGroups];               // survivor chosen; kNone: written already
+    uint32_t stop;                           // segments resolved
     uint16_t ein[kMaxGroups][kListMax];
     uint16_t next[kMaxGroups][kListMax];     // 0xFFFF: not in the next group's window
 };
@@ -733,8 +741,15 @@ constexpr size_t kWaveSmem =
 static_assert(kWinBlocksPerSM * (kWaveSmem + 1024) <= 228 * 1024, "window blocks per SM");
 
 __device__ void resolve_wave(const WalkBuffers &B, FinalSmem &S, const WalkPlan &plan, uint32_t n,
-                             uint32_t wave, uint32_t per_wave, uint32_t here, uint32_t t0) {
+                             uint32_t wave, uint32_t launches, uint32_t per_wave, uint32_t c_wave,
+                             uint32_t e0, uint32_t here, uint32_t t0) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // a miss at segment x ends the wave there, if the launches left can still
+    // cover the chain from it
+    const auto restarts = [&](uint32_t x) {
+        const uint32_t left = plan.chunks - (c_wave + plan.start(x));
+        return (left + plan.wave_chunks - 1u) / plan.wave_chunks <= launches - (wave + 1u);
+    };
     const uint32_t groups = (here + kGroup - 1) / kGroup;
     if (tid <= (int)groups && tid < kMaxGroups + 1) {
         uint4 head = make_uint4(0u, 1u, 0u, 0u);  // past the last: an empty window
@@ -758,9 +773,10 @@ __device__ void resolve_wave(const WalkBuffers &B, FinalSmem &S, const WalkPlan 
     }
     __syncthreads();
     if (warp == 0) {
-        uint32_t E = B.st->e_wave;
+        uint32_t E = e0;
         uint32_t fallbacks = 0;
-        for (uint32_t g = 0; g < groups; ++g) {
+        uint32_t stop = here;  // segments resolved
+        for (uint32_t g = 0; g < groups && stop == here; ++g) {
             const uint32_t x0 = g * kGroup, end = min(here, x0 + kGroup);
             const uint32_t cnt = S.count[g];
             const SegWindow win = S.win[g];
@@ -786,36 +802,44 @@ __device__ void resolve_wave(const WalkBuffers &B, FinalSmem &S, const WalkPlan 
             }
             // a miss inside the group: segment by segment
             for (uint32_t x = x0; x < end; ++x) {
-                const uint32_t j = wave * per_wave + x;
-                if (lane == 0) B.e_in[j] = E;
                 const SegList *L = B.lists + x;
                 const uint4 head = __ldcg(reinterpret_cast<const uint4 *>(L));
-                if (head.x <= (uint32_t)kListMax && head.x > 0 && E >= head.y && E <= head.z) {
+                const bool listed =
+                    head.x <= (uint32_t)kListMax && head.x > 0 && E >= head.y && E <= head.z;
+                if (!listed) {
+                    ++fallbacks;
+                    if (x > 0 && restarts(x)) {
+                        stop = x;
+                        break;
+                    }
+                }
+                if (lane == 0) B.e_in[wave * per_wave + x] = E;
+                if (listed) {
                     const uint32_t q = E - head.y;
                     uint32_t below = 0;
                     for (uint32_t k = lane; k < head.x; k += 32) below += __ldcg(L->ein + k) <= q;
                     below = __reduce_add_sync(0xFFFFFFFFu, below);
                     E = head.y + __ldcg(L->eout + below - 1u);
                 } else {
-                    const uint32_t c = wave * plan.wave_chunks + plan.start(x);
-                    const uint32_t ce = wave * plan.wave_chunks + plan.start(x + 1);
+                    const uint32_t c = c_wave + plan.start(x), ce = c_wave + plan.start(x + 1);
                     E = walk_segment_exact(B.entries, B.second, c * kWalkChunk,
                                            min(n, ce * kWalkChunk), E, t0);
-                    ++fallbacks;
                 }
             }
             if (lane == 0) S.pick[g] = kNone;
         }
         if (lane == 0) {
-            B.st->e_wave = E;
-            B.st->waves += 1;
+            const uint32_t end = min(plan.chunks, c_wave + plan.start(stop));
+            B.wave[wave + 1] = make_uint2(end, E);
+            B.st->waves = wave + 1;
             B.st->fallbacks += fallbacks;
             B.st->groups_done = 0;  // for the next wave
+            S.stop = stop;
         }
     }
     __syncthreads();
     // the other segments of a group: the exit count of the one before
-    for (uint32_t x = tid; x < here; x += kWinThreads) {
+    for (uint32_t x = tid; x < S.stop; x += kWinThreads) {
         const uint32_t k = S.pick[x / kGroup];
         if (x % kGroup && k != kNone)
             B.e_in[wave * per_wave + x] = __ldcg(B.path + (size_t)(x - 1) * kListMax + k);
@@ -825,20 +849,23 @@ __device__ void resolve_wave(const WalkBuffers &B, FinalSmem &S, const WalkPlan 
 // One wave of the speculative walk: one block per segment.
 __global__ void __launch_bounds__(kWinThreads, kWinBlocksPerSM)
     k_wave(WalkBuffers B, const uint32_t *__restrict__ n_ptr, int64_t capacity, uint32_t wave,
-           uint32_t per_wave, uint32_t t0, uint32_t serial_below, double sigmas, uint32_t *err) {
+           uint32_t launches, uint32_t per_wave, uint32_t t0, uint32_t serial_below, double sigmas, uint32_t *err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_last;
     if (pass_stopped(err)) return;
     const uint32_t n = (uint32_t)min((int64_t)*n_ptr, capacity);
     if (n < serial_below) return;  // the chain is walked serially instead
     const WalkPlan plan = walk_plan(n, per_wave);
-    const uint32_t here = wave_segments(plan, wave);
+    // where this wave starts: written by the wave before, never during this one
+    const uint2 from = __ldcg(B.wave + wave);
+    const uint32_t c_wave = from.x;
+    const uint32_t here = wave_segments(plan, c_wave);
     const uint32_t x = blockIdx.x;
+    if (here == 0 && x == 0 && threadIdx.x == 0) B.wave[wave + 1] = from;  // nothing left
     if (x >= here) return;  // past the chain
-    const uint32_t c_wave = wave * plan.wave_chunks;
     const uint32_t i0 = (c_wave + plan.start(x)) * kWalkChunk;
     const uint32_t i1 = min(n, (c_wave + plan.start(x + 1)) * kWalkChunk);
-    window_block(B, *reinterpret_cast<WindowSmem *>(smem_raw), c_wave, i0, i1,
+    window_block(B, *reinterpret_cast<WindowSmem *>(smem_raw), c_wave, from.y, i0, i1,
                  wave * per_wave + x, x, t0, sigmas);
     // the last of a group composes it; the last group resolves the wave
     const uint32_t g = x / kGroup, size = min((uint32_t)kGroup, here - g * kGroup);
@@ -857,7 +884,8 @@ __global__ void __launch_bounds__(kWinThreads, kWinBlocksPerSM)
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    resolve_wave(B, *reinterpret_cast<FinalSmem *>(smem_raw), plan, n, wave, per_wave, here, t0);
+    resolve_wave(B, *reinterpret_cast<FinalSmem *>(smem_raw), plan, n, wave, launches, per_wave,
+                 c_wave, from.y, here, t0);
 }
 
 // ---------------------------------------------------------------------------
@@ -903,7 +931,8 @@ __global__ void __launch_bounds__(32)
         const WalkPlan plan = walk_plan(n, per_wave);
         const uint32_t places = plan.wave_chunks / 2u + plan.segs;
         const uint32_t w = p / places, q = p % places;
-        if (w < plan.waves) {
+        if (w < B.st->waves) {
+            const uint32_t c_wave = B.wave[w].x, c_end = B.wave[w + 1].x;
             uint32_t l = 0, h = plan.segs;
             while (h - l > 1u) {
                 const uint32_t mid = (l + h) / 2u;
@@ -911,8 +940,8 @@ __global__ void __launch_bounds__(32)
                 else h = mid;
             }
             const uint32_t s0 = plan.start(l), m = q - (s0 / 2u + l);
-            const uint32_t c0 = w * plan.wave_chunks + s0;
-            const uint32_t c1 = min(plan.chunks, w * plan.wave_chunks + plan.start(l + 1));
+            const uint32_t c0 = c_wave + s0;
+            const uint32_t c1 = min(c_end, c_wave + plan.start(l + 1));
             const uint32_t c = c0 + m * (kPiece / kWalkChunk);
             if (c < c1) {
                 const uint32_t j = w * per_wave + l;
@@ -994,11 +1023,17 @@ __global__ void __launch_bounds__(32)
 // Host side
 // ---------------------------------------------------------------------------
 
+// Waves launched for a chain of the list's capacity: spare ones where a miss
+// is expensive (long segments).
+static uint32_t wave_launches(const WalkPlan &plan) {
+    return plan.waves + (plan.even ? 0u : kSpareWaves);
+}
+
 // Device layout of the walk scratch for lists of up to `capacity` channels;
 // returns its size.
 static size_t walk_layout(void *scratch, int64_t capacity, int per_wave, WalkBuffers *B) {
     const uint32_t n = (uint32_t)std::min<int64_t>(capacity, 0xFFFFFF00ll);
-    const size_t waves = walk_plan(n, (uint32_t)per_wave).waves;
+    const size_t waves = wave_launches(walk_plan(n, (uint32_t)per_wave));
     const size_t groups = ((size_t)per_wave + kGroup - 1) / kGroup;
     char *base = reinterpret_cast<char *>(scratch);
     size_t off = 0;
@@ -1010,6 +1045,7 @@ static size_t walk_layout(void *scratch, int64_t capacity, int per_wave, WalkBuf
     WalkBuffers b{};
     b.st = (WalkState *)take(sizeof(WalkState));
     b.group_done = (uint32_t *)take(groups * sizeof(uint32_t));
+    b.wave = (uint2 *)take((waves + 1) * sizeof(uint2));
     b.windows = (SegWindow *)take(waves * per_wave * sizeof(SegWindow));
     b.e_in = (uint32_t *)take(waves * per_wave * sizeof(uint32_t));
     b.lists = (SegList *)take((size_t)per_wave * sizeof(SegList));
@@ -1070,19 +1106,22 @@ cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
     B.chunk_stat = chunk_stat;
     const uint32_t t0 = (s0 & kLcgMask) << 8;
     const uint32_t serial_below = parallel ? kSerialBelow : 0xFFFFFFFFu;
-    // the state and the group counters, next to each other
+    // the state, the group counters and the waves' starts, next to each other
     cudaMemsetAsync(B.st, 0, (char *)B.windows - (char *)B.st, stream);
     int64_t places = 1;
     if (parallel) {
         const uint32_t cap = (uint32_t)std::min<int64_t>(capacity, 0xFFFFFF00ll);
         const WalkPlan plan = walk_plan(cap, (uint32_t)per_wave);
         const uint32_t blocks = std::min((uint32_t)per_wave, plan.chunks);
-        // chunks / 2 and per_wave places a wave, one more a wave for rounding
-        places = (int64_t)plan.chunks / 2 + (int64_t)plan.waves * (per_wave + 2);
-        for (uint32_t w = 0; w < plan.waves; ++w) {
+        const uint32_t launches = wave_launches(plan);
+        // half a wave's chunks (a shorter chain may have longer waves than the
+        // capacity's) and per_wave places a wave
+        const uint32_t reach = std::min(plan.chunks, (uint32_t)per_wave * kWalkAvgMax);
+        places = (int64_t)launches * (reach / 2 + per_wave + 2);
+        for (uint32_t w = 0; w < launches; ++w) {
             const cudaError_t e =
                 launch_prio(k_wave, dim3(blocks), dim3(kWinThreads), kWaveSmem, stream, priority,
-                            B, n_ptr, capacity, w, (uint32_t)per_wave, t0, serial_below,
+                            B, n_ptr, capacity, w, launches, (uint32_t)per_wave, t0, serial_below,
                             window_sigmas, const_cast<uint32_t *>(err));
             if (e != cudaSuccess) return e;
         }
