@@ -66,7 +66,7 @@ WALK_AVG_CHUNKS = 18     # most 256-channel chunks per segment on average (kWalk
 
 def launches_per_frame(h: int, w: int, sms: int) -> int:
     """Kernel launches of one plain pass (the library's launch sequence):
-    producer 2, planes 1, stencil 1, startup 1, chain 4, walk 1 per wave + 1
+    producer 2, planes 1, stencil 1, startup 1, chain 2, walk 1 per wave + 1
     rewalk, apply 1.  Waves are sized from the RNG-dependent list capacity,
     with four window blocks per SM."""
 
@@ -77,7 +77,7 @@ def launches_per_frame(h: int, w: int, sms: int) -> int:
     waves = (chunks + per_wave * WALK_AVG_CHUNKS - 1) // (per_wave * WALK_AVG_CHUNKS)
     if chunks >= 4 * per_wave * waves:  # long segments: two spare waves for misses
         waves += 2
-    return 11 + waves
+    return 9 + waves
 
 
 def ncu_counter(kernel: str, name: str):

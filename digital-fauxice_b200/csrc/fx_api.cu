@@ -48,7 +48,6 @@ struct Arena {
     uint32_t *seg_raw = nullptr;  // seg_raw_words(segments): per-segment and per-block sums
     AmbEntry *entries = nullptr;
     SecondInterval *second = nullptr;
-    uint32_t *pos = nullptr, *site_of = nullptr;
     ExtraWord *extra = nullptr;
     uint8_t *chunk_two = nullptr;
     ChunkStat *chunk_stat = nullptr;
@@ -58,7 +57,8 @@ struct Arena {
     uint8_t *changed = nullptr;
     void *counters = nullptr;
     uint32_t *err = nullptr;
-    void *walk = nullptr;
+    void *walk = nullptr, *walk_zero = nullptr;
+    size_t zero_bytes = 0;  // cleared for a pass, from `counters` on
     int64_t amb_capacity = 0;
 };
 
@@ -86,17 +86,18 @@ static size_t arena_layout(const Geometry &g, int64_t amb_cap, Arena *a) {
     const size_t o_sr = take(seg_raw_words(g.segments) * 4);
     const size_t o_ent = take(amb_cap * sizeof(AmbEntry));
     const size_t o_sec = take(amb_cap * sizeof(SecondInterval));
-    const size_t o_pos = take(amb_cap * 4);
-    const size_t o_site = take(amb_cap * 4);
     const size_t o_ext = take(extra_words(amb_cap) * sizeof(ExtraWord));
-    const size_t o_two = take(walk_chunks(amb_cap));
-    const size_t o_stat = take(walk_chunks(amb_cap) * sizeof(ChunkStat));
     const size_t o_prod = take(producer_bytes(g.h, g.w));
     const size_t o_rows = take(4 * (size_t)g.h * 4);
     const size_t o_out = take(px * 6);
     const size_t o_chg = take(px);
-    const size_t o_ctr = take(dev_counters_bytes());
-    const size_t o_err = take(16);
+    // what a pass clears, in one piece: counters, error block (right behind
+    // them: both come back in one copy), the walk's state and chunk tables
+    const size_t o_ctr = take(dev_counters_bytes() + 16);
+    const size_t o_wz = take(walk_zero_bytes(amb_cap));
+    const size_t o_stat = take(walk_chunks(amb_cap) * sizeof(ChunkStat));
+    const size_t o_two = take(walk_chunks(amb_cap));
+    const size_t zero_end = off;
     const size_t o_walk = take(walk_scratch_bytes(amb_cap, g_per_wave));
     if (a) {
         char *b = reinterpret_cast<char *>(a->base);
@@ -113,17 +114,17 @@ static size_t arena_layout(const Geometry &g, int64_t amb_cap, Arena *a) {
         a->seg_raw = (uint32_t *)(b + o_sr);
         a->entries = (AmbEntry *)(b + o_ent);
         a->second = (SecondInterval *)(b + o_sec);
-        a->pos = (uint32_t *)(b + o_pos);
-        a->site_of = (uint32_t *)(b + o_site);
         a->extra = (ExtraWord *)(b + o_ext);
-        a->chunk_two = (uint8_t *)(b + o_two);
-        a->chunk_stat = (ChunkStat *)(b + o_stat);
         a->producer = (void *)(b + o_prod);
         a->rows = (float *)(b + o_rows);
         a->out = (uint16_t *)(b + o_out);
         a->changed = (uint8_t *)(b + o_chg);
         a->counters = (void *)(b + o_ctr);
-        a->err = (uint32_t *)(b + o_err);
+        a->err = (uint32_t *)(b + o_ctr + dev_counters_bytes());
+        a->walk_zero = (void *)(b + o_wz);
+        a->chunk_stat = (ChunkStat *)(b + o_stat);
+        a->chunk_two = (uint8_t *)(b + o_two);
+        a->zero_bytes = zero_end - o_ctr;
         a->walk = (void *)(b + o_walk);
         a->amb_capacity = amb_cap;
     }
@@ -318,7 +319,7 @@ static int enqueue_pass(fx_context *ctx, Slot &s, const Geometry &g, const fx_pa
         ctx->pending.push_back(std::move(ev));
         marks.events = ctx->pending.back().data();
     }
-    FX_CUDA(ctx, cudaMemsetAsync(a.err, 0, 16, st));
+    FX_CUDA(ctx, cudaMemsetAsync(a.counters, 0, a.zero_bytes, st));
     marks.mark(0, st);
     if (host_stages) {
         FX_CUDA(ctx, cudaMemcpyAsync(a.stages, host_stages, (g.h + 6) * sizeof(fx_stage),
@@ -337,9 +338,8 @@ static int enqueue_pass(fx_context *ctx, Slot &s, const Geometry &g, const fx_pa
     // the walk scratch is sized for g_per_wave; a narrower wave uses part of it
     const int wave = (ctx->walk_wave > 0 && ctx->walk_wave < g_per_wave) ? ctx->walk_wave
                                                                          : g_per_wave;
-    WriterBuffers wb{a.seg_base, a.seg_amb, a.seg_raw, a.entries, a.second, a.pos,
-                     a.site_of, a.extra, a.counters,
-                     a.amb_capacity, a.walk, wave, ctx->parallel_walk, ctx->walk_sigmas, cancel,
+    WriterBuffers wb{a.seg_base, a.seg_amb, a.seg_raw, a.entries, a.second, a.extra, a.counters,
+                     a.amb_capacity, a.walk, a.walk_zero, wave, ctx->parallel_walk, ctx->walk_sigmas, cancel,
                      a.chunk_two, a.chunk_stat, ctx->use_priority ? ctx->top_priority : 0};
     FX_CUDA(ctx, launch_writer(g, a.meta, a.cand, d_in, ctx->lut, ctx->high, ctx->low, ctx->ident, a.stages,
                                p, rng, wb, d_out, d_changed, a.err, st, marks));
@@ -450,9 +450,7 @@ static int run_device(fx_context *ctx, Slot &s, const Geometry &g, const fx_para
         rc = enqueue_pass(ctx, s, g, p, stages, rng, in, out, chg, producer_rows);
         if (rc) return rc;
         char *hc = reinterpret_cast<char *>(s.h_ctr);
-        FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes(),
-                                     cudaMemcpyDeviceToHost, s.stream));
-        FX_CUDA(ctx, cudaMemcpyAsync(hc + dev_counters_bytes(), s.arena.err, 4,
+        FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes() + 4,
                                      cudaMemcpyDeviceToHost, s.stream));
         FX_CUDA(ctx, cudaStreamSynchronize(s.stream));
         uint32_t err;
@@ -795,9 +793,7 @@ FX_API int fx_process(fx_context *ctx, const fx_frame *f, fx_counters *counters)
                           s.arena.out, s.arena.changed, false);
         if (rc) return rc;
         char *hc = reinterpret_cast<char *>(s.h_ctr);
-        FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes(),
-                                     cudaMemcpyDeviceToHost, s.stream));
-        FX_CUDA(ctx, cudaMemcpyAsync(hc + dev_counters_bytes(), s.arena.err, 4,
+        FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes() + 4,
                                      cudaMemcpyDeviceToHost, s.stream));
         FX_CUDA(ctx, cudaStreamSynchronize(s.stream));
         uint32_t err;
@@ -869,9 +865,7 @@ FX_API int fx_sync_counters(fx_context *ctx, fx_counters *counters) {
     Slot &s = slot0(ctx);
     cudaStream_t st = s.last_stream ? s.last_stream : s.stream;
     char *hc = reinterpret_cast<char *>(s.h_ctr);
-    FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes(),
-                                 cudaMemcpyDeviceToHost, st));
-    FX_CUDA(ctx, cudaMemcpyAsync(hc + dev_counters_bytes(), s.arena.err, 4,
+    FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes() + 4,
                                  cudaMemcpyDeviceToHost, st));
     FX_CUDA(ctx, cudaStreamSynchronize(st));
     uint32_t err;
@@ -999,9 +993,7 @@ static int stage_host_results(fx_context *ctx, Slot &s) {
         FX_CUDA(ctx, cudaMemcpyAsync(ho + px * 10, s.arena.changed, px, cudaMemcpyDeviceToHost,
                                      s.stream));
     char *hc = reinterpret_cast<char *>(s.h_ctr);
-    FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes(),
-                                 cudaMemcpyDeviceToHost, s.stream));
-    FX_CUDA(ctx, cudaMemcpyAsync(hc + dev_counters_bytes(), s.arena.err, 4,
+    FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes() + 4,
                                  cudaMemcpyDeviceToHost, s.stream));
     return FX_OK;
 }
@@ -1091,9 +1083,7 @@ static int copy_device_results(fx_context *ctx, Slot &s) {
                                        (size_t)g.pitch * 4, (size_t)g.w * 4, g.h,
                                        cudaMemcpyDeviceToDevice, s.stream));
     char *hc = reinterpret_cast<char *>(s.h_ctr);
-    FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes(),
-                                 cudaMemcpyDeviceToHost, s.stream));
-    FX_CUDA(ctx, cudaMemcpyAsync(hc + dev_counters_bytes(), s.arena.err, 4,
+    FX_CUDA(ctx, cudaMemcpyAsync(hc, s.arena.counters, dev_counters_bytes() + 4,
                                  cudaMemcpyDeviceToHost, s.stream));
     return FX_OK;
 }

@@ -262,12 +262,11 @@ struct WriterBuffers {
     uint32_t *seg_raw;             // seg_raw_words(segments): the prefix's partial sums
     AmbEntry *entries;             // capacity
     SecondInterval *second;        // capacity, sparse
-    uint32_t *pos;                 // capacity
-    uint32_t *site_of;             // capacity: the site of each listed channel
     ExtraWord *extra;              // extra_words(capacity)
     void *counters;                // DevCounters
     int64_t capacity;
     void *walk_scratch;            // walk_scratch_bytes(capacity, per_wave)
+    void *walk_zero;               // walk_zero_bytes(capacity), cleared for the pass
     int per_wave;                  // window blocks per wave (walk_per_wave of the SM count)
     bool parallel_walk;
     double window_sigmas;          // walk window half-width in standard deviations
@@ -327,17 +326,29 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
 size_t dev_counters_bytes();
 cudaError_t walk_init();
 size_t walk_scratch_bytes(int64_t capacity, int per_wave);
+size_t walk_zero_bytes(int64_t capacity);
 int walk_per_wave(int sms);
 __host__ __device__ inline size_t walk_chunks(int64_t capacity) {
     return (size_t)((capacity + kWalkChunk - 1) / kWalkChunk) + 1;
 }
 cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
-                        const uint32_t *n_ptr, int64_t capacity, uint32_t s0, void *scratch, int per_wave,
+                        const uint32_t *n_ptr, int64_t capacity, uint32_t s0, void *scratch,
+                        void *zero, int per_wave,
                         bool parallel, double window_sigmas, const uint8_t *chunk_two,
                         const ChunkStat *chunk_stat,
-                        ExtraWord *extra, uint32_t *fallbacks_out,
-                        unsigned long long *stats_out, const uint32_t *err,
-                        cudaStream_t stream, int priority);
+                        ExtraWord *extra, const uint32_t *err, cudaStream_t stream,
+                        int priority);
+// Diagnostics of a pass's walk, at the start of its cleared scratch.
+struct WalkState {
+    uint32_t waves;      // waves resolved
+    uint32_t fallbacks;  // misses: waves ended early and segments walked exactly
+    uint32_t packed;     // segments whose settled phase ran two candidates per lane
+    uint32_t groups_done;                // groups of the current wave composed
+    unsigned long long candidate_steps;  // window-walk work
+    unsigned long long window_sum;       // candidates started
+    unsigned long long survivor_sum;     // candidates left at segment ends
+    uint32_t kept_next;                  // entries of the kept lists' pool handed out
+};
 // Stage gate: when *cancel (host-mapped) is set, stop the pass: err[1] = 1
 // and err[0] = FX_ERR_CANCELLED unless an error came first.  No launch when
 // `cancel` is null.

@@ -67,17 +67,6 @@ constexpr uint32_t kSerialBelow = 1024;             // short chains: one serial 
 // fx_set_walk_window narrows the windows, so tests can force misses.
 constexpr uint32_t kSpareWaves = 2;  // launches beyond the waves a chain needs
 
-struct WalkState {
-    uint32_t waves;      // waves resolved
-    uint32_t fallbacks;  // misses: waves ended early and segments walked exactly
-    uint32_t packed;     // segments whose settled phase ran two candidates per lane
-    unsigned long long candidate_steps;  // window-walk work, for diagnostics
-    unsigned long long window_sum;       // candidates started
-    unsigned long long survivor_sum;     // candidates left at segment ends
-    uint32_t groups_done;                // groups of the current wave composed
-    uint32_t kept_next;                  // entries of the kept lists' pool handed out
-};
-
 struct SegWindow {
     uint32_t lo, hi;  // candidate E_in range, inclusive
 };
@@ -1029,12 +1018,22 @@ static uint32_t wave_launches(const WalkPlan &plan) {
     return plan.waves + (plan.even ? 0u : kSpareWaves);
 }
 
+constexpr size_t kWalkZeroGroups = 128, kWalkZeroWaves = 256;
+static_assert(sizeof(WalkState) <= kWalkZeroGroups &&
+                  kWalkZeroGroups + kMaxGroups * sizeof(uint32_t) <= kWalkZeroWaves,
+              "the cleared part's layout");
+size_t walk_zero_bytes(int64_t capacity) {
+    // a wave has at least one segment, so at least kWalkAvgMax chunks
+    return kWalkZeroWaves +
+           (walk_chunks(capacity) / kWalkAvgMax + 2 + kSpareWaves) * sizeof(uint2);
+}
+
 // Device layout of the walk scratch for lists of up to `capacity` channels;
 // returns its size.
-static size_t walk_layout(void *scratch, int64_t capacity, int per_wave, WalkBuffers *B) {
+static size_t walk_layout(void *scratch, void *zero, int64_t capacity, int per_wave,
+                          WalkBuffers *B) {
     const uint32_t n = (uint32_t)std::min<int64_t>(capacity, 0xFFFFFF00ll);
     const size_t waves = wave_launches(walk_plan(n, (uint32_t)per_wave));
-    const size_t groups = ((size_t)per_wave + kGroup - 1) / kGroup;
     char *base = reinterpret_cast<char *>(scratch);
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -1043,9 +1042,6 @@ static size_t walk_layout(void *scratch, int64_t capacity, int per_wave, WalkBuf
         return r;
     };
     WalkBuffers b{};
-    b.st = (WalkState *)take(sizeof(WalkState));
-    b.group_done = (uint32_t *)take(groups * sizeof(uint32_t));
-    b.wave = (uint2 *)take((waves + 1) * sizeof(uint2));
     b.windows = (SegWindow *)take(waves * per_wave * sizeof(SegWindow));
     b.e_in = (uint32_t *)take(waves * per_wave * sizeof(uint32_t));
     b.lists = (SegList *)take((size_t)per_wave * sizeof(SegList));
@@ -1055,12 +1051,16 @@ static size_t walk_layout(void *scratch, int64_t capacity, int per_wave, WalkBuf
     b.kept_state = (uint32_t *)take((size_t)pool * sizeof(uint32_t));
     b.kept_ein = (uint16_t *)take((size_t)pool * sizeof(uint16_t));
     b.kept_size = (uint32_t)std::min<int64_t>(pool, 0xFFFFFFFFll);
+    // the cleared part: state, group counters, the waves' starts
+    b.st = (WalkState *)zero;
+    b.group_done = (uint32_t *)((char *)zero + kWalkZeroGroups);
+    b.wave = (uint2 *)((char *)zero + kWalkZeroWaves);
     if (B) *B = b;
     return off;
 }
 
 size_t walk_scratch_bytes(int64_t capacity, int per_wave) {
-    return walk_layout(nullptr, capacity, per_wave, nullptr);
+    return walk_layout(nullptr, nullptr, capacity, per_wave, nullptr);
 }
 
 // Segments per wave: the blocks that fit the SMs, so every block of a wave is
@@ -1094,20 +1094,17 @@ cudaError_t walk_init() {
 // lane instead of the speculative windows.
 cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
                         const uint32_t *n_ptr, int64_t capacity, uint32_t s0, void *scratch,
-                        int per_wave, bool parallel, double window_sigmas,
+                        void *zero, int per_wave, bool parallel, double window_sigmas,
                         const uint8_t *chunk_two, const ChunkStat *chunk_stat, ExtraWord *extra,
-                        uint32_t *fallbacks_out, unsigned long long *stats_out,
                         const uint32_t *err, cudaStream_t stream, int priority) {
     WalkBuffers B;
-    walk_layout(scratch, capacity, per_wave, &B);
+    walk_layout(scratch, zero, capacity, per_wave, &B);
     B.entries = entries;
     B.second = second;
     B.chunk_two = chunk_two;
     B.chunk_stat = chunk_stat;
     const uint32_t t0 = (s0 & kLcgMask) << 8;
     const uint32_t serial_below = parallel ? kSerialBelow : 0xFFFFFFFFu;
-    // the state, the group counters and the waves' starts, next to each other
-    cudaMemsetAsync(B.st, 0, (char *)B.windows - (char *)B.st, stream);
     int64_t places = 1;
     if (parallel) {
         const uint32_t cap = (uint32_t)std::min<int64_t>(capacity, 0xFFFFFF00ll);
@@ -1130,13 +1127,6 @@ cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
                                 sizeof(RewalkSmem), stream, priority, B, n_ptr, capacity,
                                 (uint32_t)per_wave, t0, extra, serial_below, err);
     if (e != cudaSuccess) return e;
-    // fallbacks_out[0] = segments walked exactly, fallbacks_out[1] = packed segments
-    if (fallbacks_out)
-        cudaMemcpyAsync(fallbacks_out, &B.st->fallbacks, 2 * sizeof(uint32_t),
-                        cudaMemcpyDeviceToDevice, stream);
-    if (stats_out)
-        cudaMemcpyAsync(stats_out, &B.st->candidate_steps, 3 * sizeof(unsigned long long),
-                        cudaMemcpyDeviceToDevice, stream);
     return cudaGetLastError();
 }
 

@@ -8,20 +8,18 @@
 // |delta|.  So:
 //   1. k_stencil / k_startup classify every channel: 0, 1 or 2 fixed draws,
 //      or "RNG-dependent" (one or two).
-//   2. k_seg_sums + k_seg_scan: exclusive prefix of fixed draws and of
-//      RNG-dependent channels along the chain (startup sites, then public
-//      sites in row-major order).
-//   3. k_amb: for each RNG-dependent channel, the set of first-draw states
-//      that copy the original, as at most two state intervals (found by
-//      binary search on the exact binary64 expressions, which are monotone
-//      in the state).
-//   4. k_coef: the interval test of each such channel as a function of the
-//      extra draws before it (the channel's fixed draws folded into an affine
-//      LCG jump).
-//   5. the walk (fx_walk.cu) visits only the RNG-dependent channels: a
+//   2. k_seg_sums: exclusive prefix of fixed draws and of RNG-dependent
+//      channels along the chain (startup sites, then public sites in
+//      row-major order).
+//   3. k_coef: lists the RNG-dependent channels and finds, for each, the set
+//      of first-draw states that copy the original, as at most two state
+//      intervals (by binary search on the exact binary64 expressions, which
+//      are monotone in the state), as a test on the extra draws before it
+//      (the channel's fixed draws folded into an affine LCG jump).
+//   4. the walk (fx_walk.cu) visits only the RNG-dependent channels: a
 //      multiply-add, a test and a conditional LCG step per channel,
 //      parallelised over segments by speculation.  Output: the running count of extra draws.
-//   6. k_apply: every public site computes its values from its own start
+//   5. k_apply: every public site computes its values from its own start
 //      state g^(fixed + extra before it)(s0), in parallel, and emits public
 //      RGB16 with the counters.
 #include <algorithm>
@@ -30,7 +28,7 @@
 
 namespace fx {
 
-struct DevCounters {
+struct alignas(16) DevCounters {
     unsigned long long attempted, written, public_advances, changed;
     unsigned long long su_attempted[6], su_advances[6];
     unsigned long long public_base, public_amb;
@@ -38,9 +36,11 @@ struct DevCounters {
     uint32_t startup_base, startup_amb, startup_extra;
     uint32_t n_amb;
     uint32_t walk_fallbacks;
-    uint32_t walk_packed;              // written together with walk_fallbacks
+    uint32_t walk_packed;
     unsigned long long walk_stats[3];  // candidate steps, window sum, survivor sum
     uint32_t su_base[6], su_amb[6];    // per startup row, for the last block's chain
+    uint32_t seg_done;                 // k_seg_sums's finished blocks
+    uint32_t coef_next;                // k_coef's next ticket
     uint32_t apply_next;               // k_apply's next ticket
     uint32_t apply_done;               // k_apply's finished blocks
 };
@@ -92,14 +92,25 @@ __device__ __forceinline__ SegRaw seg_raw_view(uint32_t *raw, int64_t segs) {
 // fixed << 16 | RNG-dependent), and of every group of eight segments: one
 // warp per segment, 32 sites per lane in two 16-byte loads (the meta array
 // starts on a 256-byte boundary and segments on multiples of 1024 sites),
-// one block per group.  The group sums go where k_seg_scan writes the
-// groups' prefixes.
+// one block per group.  The last block to finish scans the groups' sums into
+// their exclusive prefixes, over tiles of 4096 groups (a native frame has 2.8
+// k): a tile is loaded coalesced into shared memory, each thread scans 16
+// neighbouring groups, and one block scan of (fixed << 32 | RNG-dependent)
+// pairs gives the threads' offsets (the RNG-dependent total stays below 2^32:
+// at most three per site).  seg_base[segs] and seg_amb[segs] get the totals;
+// k_coef adds a segment's offset inside its group.
 __global__ void __launch_bounds__(kSegWarps * 32)
     k_seg_sums(const uint8_t *__restrict__ meta, int64_t sites, int64_t segs,
-               uint32_t *__restrict__ raw, const uint32_t *__restrict__ err) {
+               uint32_t *__restrict__ raw, uint32_t *__restrict__ seg_base,
+               uint32_t *__restrict__ seg_amb, DevCounters *ctr,
+               const uint32_t *__restrict__ err) {
+    constexpr int kPerThread = 16, kTile = kSegWarps * 32 * kPerThread;
     __shared__ uint32_t s_warp[kSegWarps];
+    __shared__ uint32_t tile[kTile];
+    __shared__ unsigned long long ws[kSegWarps];
+    __shared__ bool s_last;
     if (pass_stopped(err)) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t seg = (int64_t)blockIdx.x * kSegWarps + warp;
     const SegRaw v = seg_raw_view(raw, segs);
     uint32_t packed = 0;
@@ -112,54 +123,38 @@ __global__ void __launch_bounds__(kSegWarps * 32)
                      packed_word(w.x) + packed_word(w.y) + packed_word(w.z) + packed_word(w.w);
         } else {
             for (int i = 0; i < 32; ++i)
-                if (first + i < sites) packed += packed_site(meta[first + i]);
+                if (first + i < sites) packed += packed_word(meta[first + i]);
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) packed += __shfl_xor_sync(0xFFFFFFFFu, packed, o);
+    packed = __reduce_add_sync(0xFFFFFFFFu, packed);
     if (lane == 0) {
         if (seg < segs) v.seg[seg] = packed;
         s_warp[warp] = packed;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         uint32_t g = 0;  // at most 8 x 6144 fixed draws and 8 x 3072 channels
 #pragma unroll
         for (int k = 0; k < kSegWarps; ++k) g += s_warp[k];
-        v.grp_base[blockIdx.x] = g;
+        v.grp_amb[blockIdx.x] = g;  // the sum, until the scan below
+        __threadfence();
+        s_last = atomicAdd(&ctr->seg_done, 1u) == gridDim.x - 1u;
     }
-}
-
-// Exclusive scan of the groups' sums into the groups' prefixes; seg_base[n]
-// and seg_amb[n] get the totals (n segments).  One block of 1024 threads,
-// over tiles of 4096 groups (a native frame has 2.8 k): a tile is loaded
-// coalesced into shared memory, each thread scans four neighbouring groups,
-// and one block scan of (fixed << 32 | RNG-dependent) pairs gives the
-// threads' offsets (the RNG-dependent total stays below 2^32: at most three
-// per site).  k_amb adds a segment's offset inside its group.
-__global__ void __launch_bounds__(1024)
-    k_seg_scan(uint32_t *__restrict__ raw, int64_t n, uint32_t *__restrict__ seg_base,
-               uint32_t *__restrict__ seg_amb, const uint32_t *__restrict__ err) {
-    constexpr int kPerThread = 4, kTile = 1024 * kPerThread;
-    __shared__ uint32_t tb[kTile], ta[kTile];
-    __shared__ unsigned long long ws[32];
-    if (pass_stopped(err)) return;
-    const SegRaw v = seg_raw_view(raw, n);
-    const int64_t groups = (n + kSegGroup - 1) / kSegGroup;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const int64_t groups = gridDim.x;
     unsigned long long carry = 0;
     for (int64_t t0 = 0; t0 < groups; t0 += kTile) {
-        for (int j = tid; j < kTile; j += 1024) {
-            const int64_t i = t0 + j;
-            const uint32_t g = i < groups ? v.grp_base[i] : 0u;
-            tb[j] = g >> 16;
-            ta[j] = g & 0xFFFFu;
-        }
+        for (int j = tid; j < kTile; j += kSegWarps * 32)
+            tile[j] = t0 + j < groups ? __ldcg(v.grp_amb + t0 + j) : 0u;
         __syncthreads();
         unsigned long long mine = 0;
 #pragma unroll
-        for (int k = 0; k < kPerThread; ++k)
-            mine += ((unsigned long long)tb[kPerThread * tid + k] << 32) | ta[kPerThread * tid + k];
+        for (int k = 0; k < kPerThread; ++k) {
+            const uint32_t g = tile[kPerThread * tid + k];
+            mine += ((unsigned long long)(g >> 16) << 32) | (g & 0xFFFFu);
+        }
         unsigned long long x = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -168,67 +163,27 @@ __global__ void __launch_bounds__(1024)
         }
         if (lane == 31) ws[warp] = x;
         __syncthreads();
-        if (warp == 0) {
-            unsigned long long w = ws[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-                if (lane >= o) w += y;
-            }
-            ws[lane] = w;
+        unsigned long long run = carry + x - mine;
+        for (int k = 0; k < kSegWarps; ++k) {
+            if (k < warp) run += ws[k];
+            carry += ws[k];
         }
-        __syncthreads();
-        unsigned long long run = carry + (warp ? ws[warp - 1] : 0ull) + x - mine;
 #pragma unroll
         for (int k = 0; k < kPerThread; ++k) {
-            const int j = kPerThread * tid + k;
-            const unsigned long long val = ((unsigned long long)tb[j] << 32) | ta[j];
-            tb[j] = (uint32_t)(run >> 32);
-            ta[j] = (uint32_t)run;
-            run += val;
-        }
-        carry += ws[31];
-        __syncthreads();
-        for (int j = tid; j < kTile; j += 1024) {
-            const int64_t i = t0 + j;
+            const int64_t i = t0 + kPerThread * tid + k;
+            const uint32_t g = tile[kPerThread * tid + k];
             if (i < groups) {
-                v.grp_base[i] = tb[j];
-                v.grp_amb[i] = ta[j];
+                v.grp_base[i] = (uint32_t)(run >> 32);
+                v.grp_amb[i] = (uint32_t)run;
             }
+            run += ((unsigned long long)(g >> 16) << 32) | (g & 0xFFFFu);
         }
-        __syncthreads();
+        __syncthreads();  // the tile and the warp sums are consumed
     }
     if (tid == 0) {
-        seg_base[n] = (uint32_t)(carry >> 32);
-        seg_amb[n] = (uint32_t)carry;
+        seg_base[segs] = (uint32_t)(carry >> 32);
+        seg_amb[segs] = (uint32_t)carry;
     }
-}
-
-struct SiteInfo {
-    float orig[3];
-    bool floor_enabled;
-};
-
-__device__ __forceinline__ SiteInfo site_info(int64_t site, int w, const uint16_t *rgbi,
-                                              const float *lut, const fx_stage *stages,
-                                              const fx_params &p) {
-    SiteInfo si;
-    const int64_t su = 6 * (int64_t)w;
-    int64_t pixel;
-    int stage_index;
-    if (site < su) {
-        pixel = site % w;  // startup originals are row 0 (startup.py:327-336)
-        stage_index = (int)(site / w);
-    } else {
-        pixel = site - su;
-        stage_index = (int)(pixel / w) + 6;
-    }
-    const uint2 raw = reinterpret_cast<const uint2 *>(rgbi)[pixel];
-    si.orig[0] = __ldg(lut + (raw.x & 0xFFFFu));
-    si.orig[1] = __ldg(lut + (raw.x >> 16));
-    si.orig[2] = __ldg(lut + (raw.y & 0xFFFFu));
-    si.floor_enabled = p.driver_gate_primary || stages[stage_index].gate_secondary;
-    return si;
 }
 
 // Affine jump tables: g_jump[j][d] = g^(d * 64^j) in T space.  States repeat
@@ -236,6 +191,10 @@ __device__ __forceinline__ SiteInfo site_info(int64_t site, int w, const uint16_
 // map on states.
 constexpr int kJumpDigits = 4;
 __device__ Affine g_jump[kJumpDigits][64];
+
+// Powers of the LCG step for short jumps: g_short[j][d] = g^(d * 128^j) in T
+// space, so a jump below 2^14 draws is two lookups.
+__device__ Affine g_short[2][128];
 
 // ---------------------------------------------------------------------------
 // Copy intervals of one RNG-dependent channel
@@ -246,58 +205,54 @@ struct ChannelView {
     float span;
     DitherConst dc;
     __device__ double raw(uint32_t s1) const { return dither_raw_delta(cd, env, span, s1); }
-    __device__ bool low_ok(uint32_t s1) const { return dc.low < cd + raw(s1); }
-    __device__ bool high_ok(uint32_t s1) const { return cd + raw(s1) < dc.high; }
-    __device__ bool floor_test(uint32_t s1) const { return cand + raw(s1) <= od; }
-    __device__ bool copies(uint32_t s1) const {
-        const double d = raw(s1);
-        const double changed = cd + d;
-        const double eff = (dc.low < changed && changed < dc.high) ? d : 0.0;
-        return cand + eff <= od;
-    }
+    __device__ bool low_ok(double d) const { return dc.low < cd + d; }
+    __device__ bool high_ok(double d) const { return cd + d < dc.high; }
+    __device__ bool floor_test(double d) const { return cand + d <= od; }
 };
 
-// First state where a monotone predicate differs from its value at 0
-// (2^24 when it never does).  `guess` estimates that state; the search
-// gallops from it to a bracket checked on the exact predicate and bisects
-// inside, so the estimate changes only the cost, never the result.
+// Estimate of the state s1 at which base + raw(s1) reaches target (the delta
+// is affine in s1 before rounding), inside [1, 2^24 - 2].  `inverse` is 1 /
+// (env * span) to about 2^-45; the search checks the exact predicate, so the
+// estimate changes only its cost.
+__device__ __forceinline__ uint32_t crossing(double base, double target, double inverse) {
+    constexpr double kScale = 1.0 / kNormalization, kOffset = 0.5 / kNormalization - 1.0;
+    const double guess = (target - base) * (inverse * kScale) + kOffset;
+    // the conversion saturates, and gives 0 for NaN
+    return min(max(__double2uint_rz(guess), 1u), kLcgMask - 1u);
+}
+
+// First state where a monotone predicate differs from its value p0 at state 0
+// (it does differ at 2^24 - 1).  Two probes around the estimate x settle
+// nearly every search; otherwise the search gallops from x to a bracket and
+// bisects inside.
 template <class F>
-__device__ __forceinline__ uint32_t switch_point(F pred, double guess) {
-    const bool p0 = pred(0u);
-    if (pred(kLcgMask) == p0) return kLcgMask + 1u;
+__device__ __forceinline__ uint32_t switch_point(F pred, bool p0, uint32_t x) {
+    const bool px = pred(x), py = pred(x + 1u);
+    if (px == p0 && py != p0) return x + 1u;
     // invariant: pred(lo) == p0, pred(hi) != p0, lo < hi
     uint32_t lo = 0u, hi = kLcgMask;
-    uint32_t x = kLcgMask / 2u;
-    if (guess == guess) {  // not NaN
-        const double top = (double)(kLcgMask - 1u);
-        x = (uint32_t)(guess < 1.0 ? 1.0 : (guess > top ? top : guess));
-    }
     uint32_t step = 1u;
-    if (pred(x) == p0) {
-        lo = x;
-        while (hi - lo > 1u) {
-            if (hi - lo <= step) break;
+    if (px == p0) {
+        lo = x + 1u;
+        while (hi - lo > step) {
             const uint32_t y = lo + step;
-            if (pred(y) == p0) {
-                lo = y;
-                step <<= 1;
-            } else {
+            if (pred(y) != p0) {
                 hi = y;
                 break;
             }
+            lo = y;
+            step <<= 1;
         }
     } else {
         hi = x;
-        while (hi - lo > 1u) {
-            if (hi - lo <= step) break;
+        while (hi - lo > step) {
             const uint32_t y = hi - step;
-            if (pred(y) != p0) {
-                hi = y;
-                step <<= 1;
-            } else {
+            if (pred(y) == p0) {
                 lo = y;
                 break;
             }
+            hi = y;
+            step <<= 1;
         }
     }
     while (hi - lo > 1u) {
@@ -308,264 +263,283 @@ __device__ __forceinline__ uint32_t switch_point(F pred, double guess) {
     return hi;
 }
 
-// The state s1 at which base + raw(s1) would reach `target` if the delta
-// were computed exactly (it is affine in s1): a starting point for
-// switch_point.
-__device__ __forceinline__ double crossing(const ChannelView &cv, double base, double target) {
-    const double scale = cv.env * (double)cv.span;
-    return ((target - base) / scale + 0.5) / kNormalization - 1.0;
-}
-
 // Copy set of one channel in T space: copy iff (T - l1) <= w1 or
 // (T - l2) <= w2 (modulo 2^32); l = 0x80 marks an empty interval.
 struct CopySet {
     uint32_t l1, w1, l2, w2;
 };
 
-__device__ void copy_intervals(const ChannelView &cv, CopySet &e, uint32_t *err) {
-    uint32_t b[3] = {
-        switch_point([&](uint32_t s) { return cv.low_ok(s); }, crossing(cv, cv.cd, cv.dc.low)),
-        switch_point([&](uint32_t s) { return cv.high_ok(s); }, crossing(cv, cv.cd, cv.dc.high)),
-        switch_point([&](uint32_t s) { return cv.floor_test(s); }, crossing(cv, cv.cand, cv.od))};
-    // sort the three breakpoints
-    if (b[0] > b[1]) { const uint32_t t = b[0]; b[0] = b[1]; b[1] = t; }
-    if (b[1] > b[2]) { const uint32_t t = b[1]; b[1] = b[2]; b[2] = t; }
-    if (b[0] > b[1]) { const uint32_t t = b[0]; b[0] = b[1]; b[1] = t; }
-    uint32_t starts[4];
-    int n = 0;
-    starts[n++] = 0u;
-    for (int i = 0; i < 3; ++i)
-        if (b[i] <= kLcgMask && b[i] != starts[n - 1]) starts[n++] = b[i];
-    uint32_t lo[2], hi[2];
-    int intervals = 0;
-    bool open = false;
-    for (int i = 0; i < n; ++i) {
-        const uint32_t first = starts[i];
-        const uint32_t last = (i + 1 < n) ? starts[i + 1] - 1u : kLcgMask;
-        const bool c = cv.copies(first);
-        if (c) {
-            if (open) {
-                hi[intervals - 1] = last;
-            } else {
-                if (intervals == 2) { raise_error(err, FX_ERR_INTERNAL); return; }
-                lo[intervals] = first;
-                hi[intervals] = last;
-                ++intervals;
-                open = true;
-            }
-        } else {
-            open = false;
-        }
-    }
+// A state copies when its delta, or none if the delta leaves (low, high),
+// passes the floor test.  Each of the three tests is monotone in the state,
+// so its values at both ends and its switch point give it everywhere.
+__device__ __forceinline__ void copy_intervals(const ChannelView &cv, CopySet &e, uint32_t *err) {
+    constexpr uint32_t kNever = kLcgMask + 1u;
+    const double d0 = cv.raw(0u), d1 = cv.raw(kLcgMask);
+    const bool low0 = cv.low_ok(d0), low1 = cv.low_ok(d1);
+    const bool high0 = cv.high_ok(d0), high1 = cv.high_ok(d1);
+    const bool floor0 = cv.floor_test(d0), floor1 = cv.floor_test(d1);
+    // one Newton step on the binary32 reciprocal; out of its range (and for
+    // 0) the estimates are infinite or NaN and the searches gallop
+    const double scale = cv.env * (double)cv.span;
+    const double r = (double)__frcp_rn((float)scale);
+    const double inverse = r * (2.0 - scale * r);
+    uint32_t bf = kNever;
+    if (floor0 != floor1)
+        bf = switch_point([&](uint32_t s) { return cv.floor_test(cv.raw(s)); }, floor0,
+                          crossing(cv.cand, cv.od, inverse));
     // empty interval: l = 0x80 can never match a T value (low byte zero)
     e.l1 = 0x80u; e.w1 = 0u; e.l2 = 0x80u; e.w2 = 0u;
-    if (intervals == 2 && lo[0] == 0u && hi[1] == kLcgMask) {
-        // [0, hi0] and [lo1, 2^24 - 1] meet across the wrap: one cyclic
-        // interval from lo1 (the test (T - l) <= w wraps modulo 2^32)
-        e.l1 = lo[1] << 8;
-        e.w1 = (hi[0] - lo[1]) << 8;
+    if (low0 && low1 && high0 && high1) {
+        // every delta stays in range (all but a few channels): the floor test
+        // alone decides, on the states up to or from its switch point
+        const uint32_t lo = floor0 ? 0u : bf, hi = floor0 ? bf - 1u : kLcgMask;
+        if (lo <= hi) { e.l1 = lo << 8; e.w1 = (hi - lo) << 8; }
         return;
     }
-    if (intervals >= 1) { e.l1 = lo[0] << 8; e.w1 = (hi[0] - lo[0]) << 8; }
-    if (intervals == 2) { e.l2 = lo[1] << 8; e.w2 = (hi[1] - lo[1]) << 8; }
+    const uint32_t bl = low0 == low1 ? kNever
+                                     : switch_point(
+                                           [&](uint32_t s) { return cv.low_ok(cv.raw(s)); }, low0,
+                                           crossing(cv.cd, cv.dc.low, inverse));
+    const uint32_t bh = high0 == high1 ? kNever
+                                       : switch_point(
+                                             [&](uint32_t s) { return cv.high_ok(cv.raw(s)); },
+                                             high0, crossing(cv.cd, cv.dc.high, inverse));
+    const bool still = cv.floor_test(0.0);  // no delta
+    // the pieces between the sorted switch points, in order
+    const uint32_t b0 = min(min(bl, bh), bf), b2 = max(max(bl, bh), bf);
+    const uint32_t b1 = max(min(bl, bh), min(max(bl, bh), bf));
+    uint32_t lo0 = 0u, hi0 = 0u, lo1 = 0u, hi1 = 0u, first = 0u;
+    int intervals = 0;
+    bool open = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t end = i == 0 ? b0 : (i == 1 ? b1 : (i == 2 ? b2 : kNever));
+        if (end == first) continue;  // empty piece
+        const bool low = low0 != (first >= bl), high = high0 != (first >= bh);
+        const bool copy = low && high ? floor0 != (first >= bf) : still;
+        if (copy) {
+            if (!open) {
+                if (intervals == 0) lo0 = first;
+                else if (intervals == 1) lo1 = first;
+                else { raise_error(err, FX_ERR_INTERNAL); return; }
+                ++intervals;
+            }
+            if (intervals == 1) hi0 = end - 1u;
+            else hi1 = end - 1u;
+        }
+        open = copy;
+        first = end;
+    }
+    if (intervals == 2 && lo0 == 0u && hi1 == kLcgMask) {
+        // [0, hi0] and [lo1, 2^24 - 1] meet across the wrap: one cyclic
+        // interval from lo1 (the test (T - l) <= w wraps modulo 2^32)
+        e.l1 = lo1 << 8;
+        e.w1 = (hi0 - lo1) << 8;
+        return;
+    }
+    if (intervals >= 1) { e.l1 = lo0 << 8; e.w1 = (hi0 - lo0) << 8; }
+    if (intervals == 2) { e.l2 = lo1 << 8; e.w2 = (hi1 - lo1) << 8; }
 }
 
-// Lists every RNG-dependent channel in chain order: entry a gets its site
-// (site_of[a], a compact array so the writes coalesce) and its draw
-// position; k_coef fills in the intervals and jumps.  One warp per segment,
-// in 16 rounds of 64 consecutive sites, two neighbouring sites per lane (all
-// the segment's meta loads issued first); a round's offsets come from one
-// warp scan, so a round's entries are written by consecutive lanes to
-// consecutive list positions.
-__global__ void __launch_bounds__(kSegWarps * 32)
-    k_amb(const uint8_t *__restrict__ meta, int64_t sites, int64_t segs,
-          uint32_t *__restrict__ raw, uint32_t *__restrict__ seg_base,
-          uint32_t *__restrict__ seg_amb, uint32_t *__restrict__ site_of,
-          uint32_t *__restrict__ pos_out, int64_t capacity, const uint32_t *__restrict__ err) {
+// Copy test and state map of every RNG-dependent channel.  Every warp takes
+// units of 256 sites, a quarter of a chain segment: the segment's meta bytes
+// give the chain offsets of the unit's sites, the channels are listed in the
+// warp's shared memory (at most three per site), and the list is processed
+// densely, one channel per lane, written to consecutive entries.  One
+// round's candidates and samples are in flight while the round before
+// searches.
+//
+// Bound: instruction issue (binary64 probes, list building), with the first
+// candidates of a unit waiting on memory.  A native frame's 9.3 M channels
+// take 173 us, at 5% coverage 17.4 M take 250.  Listing the channels in a
+// kernel of its own, through memory, and evaluating every piece between the
+// switch points anew took 300 and 500.  Five blocks per SM at 48 registers:
+// four at 60 registers measured 6% more, six (with spills) 5% more.
+constexpr int kCoefWarps = 8, kCoefBlocksPerSM = 5;
+constexpr int kUnitSites = 256;
+static_assert(kSegment == 1024 && kUnitSites == 32 * 8, "32 and 8 meta bytes per lane");
+
+// Meta bytes of a unit: this lane's 8 sites, and the packed sums (fixed << 16
+// | RNG-dependent) of the segment's sites before the unit on this lane.
+struct UnitMeta {
+    uint32_t word[2];
+    uint32_t ahead;
+};
+__device__ __forceinline__ UnitMeta unit_meta(const uint8_t *__restrict__ meta, int64_t sites,
+                                              int64_t seg, int part) {
+    const int lane = threadIdx.x & 31;
+    const int64_t first = seg * kSegment + part * kUnitSites;
+    const int64_t mine = first + lane * 8, far = seg * kSegment + lane * 32;
+    UnitMeta u{{0u, 0u}, 0u};
+    if (first + kUnitSites <= sites) {
+        if (lane < part * (kUnitSites / 32)) {
+            const uint4 *q = reinterpret_cast<const uint4 *>(meta + far);
+            const uint4 a = q[0], b = q[1];
+            u.ahead = packed_word(a.x) + packed_word(a.y) + packed_word(a.z) + packed_word(a.w) +
+                      packed_word(b.x) + packed_word(b.y) + packed_word(b.z) + packed_word(b.w);
+        }
+        const uint2 v = *reinterpret_cast<const uint2 *>(meta + mine);
+        u.word[0] = v.x;
+        u.word[1] = v.y;
+    } else {  // the chain's last unit
+        if (lane < part * (kUnitSites / 32))
+            for (int i = 0; i < 32; ++i) u.ahead += packed_word(meta[far + i]);
+        for (int i = 0; i < 8; ++i)
+            if (mine + i < sites) u.word[i >> 2] |= (uint32_t)meta[mine + i] << (8 * (i & 3));
+    }
+    return u;
+}
+
+__global__ void __launch_bounds__(kCoefWarps * 32, kCoefBlocksPerSM)
+    k_coef(AmbEntry *__restrict__ entries, SecondInterval *__restrict__ second, int64_t capacity,
+           const uint8_t *__restrict__ meta, int64_t sites, int64_t segs,
+           uint32_t *__restrict__ raw, uint32_t *__restrict__ seg_base,
+           uint32_t *__restrict__ seg_amb, const double *__restrict__ cand, int w,
+           const uint16_t *__restrict__ rgbi, const float *__restrict__ lut, fx_params p,
+           uint8_t *__restrict__ chunk_two, ChunkStat *__restrict__ chunk_stat, DevCounters *ctr,
+           uint32_t *err) {
+    __shared__ Affine s_jump[2][128];
+    // listed channels: site in the unit | channel << 8 | fixed draws before it
+    // in the segment << 10
+    __shared__ uint32_t s_list[kCoefWarps][3 * kUnitSites];
     if (pass_stopped(err)) return;
     const int lane = threadIdx.x & 31;
-    const int64_t seg = (int64_t)blockIdx.x * kSegWarps + (threadIdx.x >> 5);
-    if (seg >= segs) return;
-    const int64_t first = seg * kSegment + 2 * lane;  // sites first + 64 r, + 1
-    uint32_t m2[16];  // the two meta bytes of round r
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const int64_t s0 = first + 64 * r;
-        if (s0 + 1 < sites)
-            m2[r] = *reinterpret_cast<const uint16_t *>(meta + s0);  // even offset
-        else
-            m2[r] = s0 < sites ? meta[s0] : 0u;
-    }
-    // the segment's prefix: its group's, plus the segments before it in the
-    // group (fewer than eight, so the packed halves cannot carry); written
-    // for the kernels after the walk
+    for (int i = threadIdx.x; i < 256; i += kCoefWarps * 32)
+        s_jump[i >> 7][i & 127] = g_short[i >> 7][i & 127];
+    __syncthreads();
+    uint32_t *list = s_list[threadIdx.x >> 5];
+    const DitherConst dc = dither_const(p);
+    const int64_t su = 6 * (int64_t)w;
     const SegRaw v = seg_raw_view(raw, segs);
-    const int64_t grp = seg / kSegGroup, k0 = grp * kSegGroup;
-    uint32_t before = (k0 + lane < seg) ? v.seg[k0 + lane] : 0u;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
-    before = __shfl_sync(0xFFFFFFFFu, before, 0);
-    uint32_t P = v.grp_base[grp] + (before >> 16), A = v.grp_amb[grp] + (before & 0xFFFFu);
-    if (lane == 0) {
-        seg_base[seg] = P;
-        seg_amb[seg] = A;
-    }
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const uint8_t mb[2] = {(uint8_t)(m2[r] & 0xFFu), (uint8_t)(m2[r] >> 8)};
-        const uint32_t x0 = packed_site(mb[0]), x = x0 + packed_site(mb[1]);
-        uint32_t inc = x;
+    const int64_t units = segs * (kSegment / kUnitSites);
+    // two units per ticket on large frames (the counter is one address)
+    const int grab = units > 8 * (int64_t)gridDim.x * kCoefWarps ? 2 : 1;
+    int64_t unit = 0;
+    for (int left = 0;; --left, ++unit) {
+        if (left == 0) {
+            uint32_t ticket = 0;
+            if (lane == 0) ticket = atomicAdd(&ctr->coef_next, 1u);
+            unit = (int64_t)__shfl_sync(0xFFFFFFFFu, ticket, 0) * grab;
+            left = grab;
+        }
+        if (unit >= units) break;
+        const int64_t seg = unit / (kSegment / kUnitSites);
+        const int part = (int)(unit % (kSegment / kUnitSites));
+        const int64_t first = seg * kSegment + part * kUnitSites;
+        if (first >= sites) continue;
+        const UnitMeta u = unit_meta(meta, sites, seg, part);
+        // the segment's prefix: its group's, plus the segments before it in
+        // the group (fewer than eight, so the packed halves cannot carry);
+        // its first unit writes it for the kernels after the walk
+        const int64_t grp = seg / kSegGroup, k0 = grp * kSegGroup;
+        const uint32_t before =
+            __reduce_add_sync(0xFFFFFFFFu, (k0 + lane < seg) ? v.seg[k0 + lane] : 0u);
+        const uint32_t seg_p = v.grp_base[grp] + (before >> 16);
+        const uint32_t seg_a = v.grp_amb[grp] + (before & 0xFFFFu);
+        if (part == 0 && lane == 0) {
+            seg_base[seg] = seg_p;
+            seg_amb[seg] = seg_a;
+        }
+        const uint32_t sum = packed_word(u.word[0]) + packed_word(u.word[1]);
+        uint32_t inc = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
             if (lane >= o) inc += y;
         }
-        const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 31);
-        if (x & 0xFFFFu) {
-            const uint32_t ex = inc - x;
-            uint32_t pos = P + (ex >> 16), a = A + (ex & 0xFFFFu);
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 31) & 0xFFFFu;
+        const uint32_t ahead = __reduce_add_sync(0xFFFFFFFFu, u.ahead);
+        if (total == 0) continue;
+        __syncwarp();  // the previous list is consumed
+        {
+            uint32_t slot = (inc - sum) & 0xFFFFu;
+            uint32_t pos = (ahead + inc - sum) >> 16;  // fixed draws, relative to the segment
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint8_t mi = mb[h];
-                pos = P + ((ex + (h ? x0 : 0u)) >> 16);
+            for (int i = 0; i < 8; ++i) {
+                const uint8_t mi = (uint8_t)(u.word[i >> 2] >> (8 * (i & 3)));
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const int code = meta_code(mi, c);
-                    if (code == 3) {
-                        if ((int64_t)a < capacity) {
-                            site_of[a] = (uint32_t)(first + 64 * r + h);
-                            pos_out[a] = pos;
-                        }
-                        ++a;
-                        pos += 1u;
-                    } else {
-                        pos += (uint32_t)code;
-                    }
+                    if (code == 3) list[slot++] = (uint32_t)(lane * 8 + i) | (c << 8) | (pos << 10);
+                    pos += code == 3 ? 1u : (uint32_t)code;
                 }
             }
         }
-        P += total >> 16;
-        A += total & 0xFFFFu;
-    }
-}
-
-// k_coef's inputs of one entry, gathered in two dependent steps: the list
-// (coalesced) gives the site, the site gives its meta, pixel and candidates.
-struct CoefList {
-    uint32_t site, pos;  // pos: fixed draws before the channel
-    int k;               // this entry is the k-th of its site
-};
-struct CoefSite {
-    uint8_t meta;
-    uint2 raw;
-    double cand[3];
-};
-
-__device__ __forceinline__ CoefList coef_list(const uint32_t *__restrict__ site_of,
-                                              const uint32_t *__restrict__ pos, uint32_t i,
-                                              uint32_t n) {
-    CoefList l{0u, 0u, 0};
-    if (i >= n) return l;
-    l.site = site_of[i];
-    // a site's RNG-dependent channels are listed in channel order
-    l.k = (i >= 1 && site_of[i - 1] == l.site) ? ((i >= 2 && site_of[i - 2] == l.site) ? 2 : 1)
-                                                : 0;
-    l.pos = pos[i];
-    return l;
-}
-
-__device__ __forceinline__ CoefSite coef_site(const CoefList &l, bool live, int64_t su, int w,
-                                              const uint8_t *__restrict__ meta,
-                                              const double *__restrict__ cand,
-                                              const uint16_t *__restrict__ rgbi) {
-    CoefSite c{};
-    if (!live) return c;
-    const int64_t site = l.site;
-    const int64_t pixel = site < su ? site % w : site - su;
-    c.meta = meta[site];
-    c.raw = reinterpret_cast<const uint2 *>(rgbi)[pixel];
-    c.cand[0] = cand[3 * site];
-    c.cand[1] = cand[3 * site + 1];
-    c.cand[2] = cand[3 * site + 2];
-    return c;
-}
-
-// Copy intervals and state map of every RNG-dependent channel.  A thread's
-// entries i, i + stride, ... run through a three-stage software pipeline:
-// while entry i's interval search computes, the site of entry i + 2 stride
-// and the meta, pixel and candidates of entry i + stride are in flight, so
-// the dependent gathers overlap the arithmetic instead of stalling it.
-__global__ void __launch_bounds__(256, 4) k_coef(AmbEntry *__restrict__ entries, SecondInterval *__restrict__ second,
-                       const uint32_t *__restrict__ pos,
-                       const uint32_t *__restrict__ n_amb_ptr, int64_t capacity,
-                       const uint32_t *__restrict__ site_of, const uint8_t *__restrict__ meta,
-                       const double *__restrict__ cand, int w, const uint16_t *__restrict__ rgbi,
-                       const float *__restrict__ lut, fx_params p, uint32_t *err,
-                       uint8_t *__restrict__ chunk_two, ChunkStat *__restrict__ chunk_stat) {
-    // powers of the LCG step: states repeat after 2^24 draws, so the four
-    // low base-64 digits of a draw count give its map on states
-    __shared__ Affine s_jump[4][64];
-    if (pass_stopped(err)) return;
-    for (int j = threadIdx.x; j < 4 * 64; j += blockDim.x) s_jump[j / 64][j % 64] = g_jump[j / 64][j % 64];
-    __syncthreads();
-    const uint32_t n = (uint32_t)min((int64_t)*n_amb_ptr, capacity);
-    const DitherConst dc = dither_const(p);
-    const int64_t su = 6 * (int64_t)w;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    CoefList l0 = coef_list(site_of, pos, i, n);
-    CoefSite s0 = coef_site(l0, i < n, su, w, meta, cand, rgbi);
-    CoefList l1 = coef_list(site_of, pos, i + stride, n);
-    for (; i < n; i += stride) {
-        const uint32_t i1 = i + stride, i2 = i1 + stride;
-        const CoefSite s1 = coef_site(l1, i1 < n && i1 > i, su, w, meta, cand, rgbi);
-        const CoefList l2 = coef_list(site_of, pos, i2 > i1 ? i2 : n, n);
-        const uint8_t mi = s0.meta;
-        int c = 0;
-        for (int seen = 0; c < 3; ++c)
-            if (meta_code(mi, c) == 3 && seen++ == l0.k) break;
-        const uint2 raw = s0.raw;
-        const uint32_t lane = c == 0 ? (raw.x & 0xFFFFu) : (c == 1 ? (raw.x >> 16) : (raw.y & 0xFFFFu));
-        ChannelView cv;
-        cv.cand = c == 0 ? s0.cand[0] : (c == 1 ? s0.cand[1] : s0.cand[2]);
-        cv.cd = (double)(float)cv.cand;
-        cv.dc = dc;
-        cv.env = ((dc.high - cv.cd) * (cv.cd - dc.low)) * dc.coefficient;
-        cv.span = (float)((double)p.dither_scales[c] * cv.cd);
-        cv.od = (double)__ldg(lut + lane);
-        CopySet e;
-        copy_intervals(cv, e, err);
-        // a chunk of walk channels with a two-interval entry steps with both
-        // interval tests (every other chunk with one)
-        if (e.l2 != 0x80u) chunk_two[i / kWalkChunk] = 1;
-        // the walk's prediction: m copying states of 2^24 (an extra draw with
-        // probability p = 1 - m / 2^24), summed per chunk with the spread
-        // p (1 - p).  A warp holds 32 consecutive entries of one chunk; the
-        // lanes past the chain's end have left the loop.
-        {
-            uint32_t m = 0;
-            if (e.l1 != 0x80u) m += (e.w1 >> 8) + 1u;
-            if (e.l2 != 0x80u) m += (e.w2 >> 8) + 1u;
-            const uint32_t q = (uint32_t)(((unsigned long long)m * ((1u << 24) - m)) >> 23);
-            const uint32_t lane = threadIdx.x & 31, live = n - (i - lane);
-            const uint32_t mask = live >= 32u ? 0xFFFFFFFFu : ((1u << live) - 1u);
-            const uint32_t ms = __reduce_add_sync(mask, m >> 1), qs = __reduce_add_sync(mask, q);
-            if (lane == 0) {
-                atomicAdd(&chunk_stat[i / kWalkChunk].copy, ms);
-                atomicAdd(&chunk_stat[i / kWalkChunk].spread, qs);
+        __syncwarp();
+        // G^(draws before the segment + 1): a channel's map starts there
+        Affine base{1u, 0u};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            base = affine_compose(g_jump[j][((seg_p + 1u) >> (6 * j)) & 63u], base);
+        const uint32_t a0 = seg_a + (ahead & 0xFFFFu);  // list index of the unit's first
+        struct Channel {
+            uint32_t item, sample;
+            double cand;
+        };
+        auto fetch = [&](uint32_t k) {
+            Channel q{0u, 0u, 1.0};
+            if (k < total) {
+                q.item = list[k];
+                const int64_t site = first + (q.item & 0xFFu);
+                const int c = (q.item >> 8) & 3;
+                const int64_t pixel = site < su ? site % w : site - su;  // startup rows: row 0
+                q.sample = rgbi[4 * pixel + c];
+                q.cand = cand[3 * site + c];
+            }
+            return q;
+        };
+        Channel cur = fetch(lane);
+        for (uint32_t k = 0; k < total; k += 32) {
+            const Channel q = cur;
+            cur = fetch(k + 32 + lane);
+            const uint32_t i = a0 + k + lane;
+            const bool live = k + lane < total && (int64_t)i < capacity;
+            uint32_t m = 0;  // copying states
+            if (live) {
+                const int c = (q.item >> 8) & 3;
+                ChannelView cv;
+                cv.cand = q.cand;
+                cv.cd = (double)(float)cv.cand;
+                cv.dc = dc;
+                cv.env = ((dc.high - cv.cd) * (cv.cd - dc.low)) * dc.coefficient;
+                cv.span = (float)((double)p.dither_scales[c] * cv.cd);
+                cv.od = (double)__ldg(lut + q.sample);
+                CopySet e;
+                copy_intervals(cv, e, err);
+                // a chunk of walk channels with a two-interval entry steps with
+                // both interval tests (every other chunk with one)
+                if (e.l2 != 0x80u) chunk_two[i / kWalkChunk] = 1;
+                if (e.l1 != 0x80u) m += (e.w1 >> 8) + 1u;
+                if (e.l2 != 0x80u) m += (e.w2 >> 8) + 1u;
+                // G^(pos + 1) less the first interval's start
+                const uint32_t pos = q.item >> 10;
+                const Affine f = affine_compose(
+                    s_jump[1][pos >> 7], affine_compose(s_jump[0][pos & 127u], base));
+                entries[i] = AmbEntry{f.a, f.c - e.l1, e.w1, e.l2 != 0x80u ? 1u : 0u};
+                if (e.l2 != 0x80u) second[i] = SecondInterval{e.l1 - e.l2, e.w2};
+            }
+            // the walk's prediction: m copying states of 2^24 (an extra draw
+            // with probability p = 1 - m / 2^24), summed per chunk with the
+            // spread p (1 - p); a round's entries lie in one or two chunks
+            const uint32_t spread =
+                live ? (uint32_t)(((unsigned long long)m * ((1u << 24) - m)) >> 23) : 0u;
+            const uint32_t chunk = (a0 + k) / kWalkChunk;
+            const bool next = live && i / kWalkChunk != chunk;
+            uint32_t ms = __reduce_add_sync(0xFFFFFFFFu, next ? 0u : m >> 1);
+            uint32_t qs = __reduce_add_sync(0xFFFFFFFFu, next ? 0u : spread);
+            if (lane == 0 && ms + qs) {
+                atomicAdd(&chunk_stat[chunk].copy, ms);
+                atomicAdd(&chunk_stat[chunk].spread, qs);
+            }
+            if (__any_sync(0xFFFFFFFFu, next)) {
+                ms = __reduce_add_sync(0xFFFFFFFFu, next ? m >> 1 : 0u);
+                qs = __reduce_add_sync(0xFFFFFFFFu, next ? spread : 0u);
+                if (lane == 0) {
+                    atomicAdd(&chunk_stat[chunk + 1].copy, ms);
+                    atomicAdd(&chunk_stat[chunk + 1].spread, qs);
+                }
             }
         }
-        // G^(pos + 1) less the first interval's start
-        const uint32_t draws = l0.pos + 1u;
-        Affine f = s_jump[0][draws & 63u];
-#pragma unroll
-        for (int j = 1; j < 4; ++j)
-            f = affine_compose(s_jump[j][(draws >> (6 * j)) & 63u], f);
-        entries[i] = AmbEntry{f.a, f.c - e.l1, e.w1, e.l2 != 0x80u ? 1u : 0u};
-        if (e.l2 != 0x80u) second[i] = SecondInterval{e.l1 - e.l2, e.w2};
-        l0 = l1;
-        s0 = s1;
-        l1 = l2;
     }
 }
 
@@ -611,17 +585,16 @@ cudaError_t writer_identity_table(const float *lut, const uint32_t *hi, const ui
 
 constexpr int kApplyBlocksPerSM = 5;  // k_apply's resident blocks per SM
 static int g_apply_blocks = kApplyBlocksPerSM * 148;
-
-// Powers of the LCG step for short jumps: g_short[j][d] = g^(d * 128^j) in T
-// space, so a jump below 2^14 draws is two lookups.
-__device__ Affine g_short[2][128];
+static int g_coef_blocks = kCoefBlocksPerSM * 148;
 
 cudaError_t writer_init() {
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
-        sms > 0)
+        sms > 0) {
         g_apply_blocks = kApplyBlocksPerSM * sms;
+        g_coef_blocks = kCoefBlocksPerSM * sms;
+    }
     Affine tab[kJumpDigits][64];
     Affine step{125u, 256u};  // g^(64^j)
     for (int j = 0; j < kJumpDigits; ++j) {
@@ -667,12 +640,10 @@ cudaError_t writer_init() {
 // samples staged in shared memory five blocks took 505 us and six 866, with a
 // 128 KB emit table instead of the two factor tables 420.
 constexpr int kApplyWarps = 8;
-constexpr int kApplySites = 256;  // sites of a unit
-static_assert(kSegment == 1024 && kApplySites == 32 * 8, "32 and 8 meta bytes per lane");
 
 __device__ void apply_final(const uint32_t *seg_base, const uint32_t *seg_amb, int64_t segments,
-                            const ExtraWord *extra, uint32_t s0, DevCounters *ctr, uint32_t *err,
-                            int64_t capacity) {
+                            const ExtraWord *extra, uint32_t s0, DevCounters *ctr,
+                            const WalkState *walk, uint32_t *err, int64_t capacity) {
     uint32_t a_run = 0, p_run = 0;
     for (int r = 0; r < 6; ++r) {
         const uint32_t rb = __ldcg(&ctr->su_base[r]), ra = __ldcg(&ctr->su_amb[r]);
@@ -691,6 +662,11 @@ __device__ void apply_final(const uint32_t *seg_base, const uint32_t *seg_amb, i
     const uint32_t a_total = seg_amb[segments];
     const uint32_t e_total = extra_before(extra, a_total, capacity);
     ctr->n_amb = a_total;
+    ctr->walk_fallbacks = walk->fallbacks;
+    ctr->walk_packed = walk->packed;
+    ctr->walk_stats[0] = walk->candidate_steps;
+    ctr->walk_stats[1] = walk->window_sum;
+    ctr->walk_stats[2] = walk->survivor_sum;
     ctr->final_state = lcg_jump(s0, (uint64_t)p_total + e_total);
     const unsigned long long expect =
         (unsigned long long)(p_total - p_run) + (e_total - e_su);
@@ -705,13 +681,13 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
             const uint16_t *__restrict__ ident, const fx_stage *__restrict__ stages, fx_params p,
             const uint32_t *__restrict__ seg_base, const uint32_t *__restrict__ seg_amb,
             const ExtraWord *__restrict__ extra, uint32_t s0, uint16_t *__restrict__ rgb_out,
-            uint8_t *__restrict__ changed_out, DevCounters *ctr, uint32_t *err,
-            int64_t capacity) {
+            uint8_t *__restrict__ changed_out, DevCounters *ctr,
+            const WalkState *__restrict__ walk, uint32_t *err, int64_t capacity) {
     __shared__ Affine s_jump[2][128];
     __shared__ uint32_t hi[256], lo[256];  // emit factors
     // attempted sites: x = site in the segment | meta << 16, y = fixed draws
     // before it in the segment | RNG-dependent channels before it << 16
-    __shared__ uint2 s_list[kApplyWarps][kApplySites];
+    __shared__ uint2 s_list[kApplyWarps][kUnitSites];
     __shared__ unsigned long long s_sums[kApplyWarps][4];
     __shared__ bool s_last;
     if (pass_stopped(err)) return;  // cancelled: the output stays untouched
@@ -728,7 +704,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
     uint2 *list = s_list[warp];
     unsigned long long att = 0, written = 0, changed = 0, draws_total = 0;
     bool ok = true;
-    const int64_t units = 6 + segs * (kSegment / kApplySites);
+    const int64_t units = 6 + segs * (kSegment / kUnitSites);
     // two units per ticket on large frames (the ticket counter is one address),
     // one on small ones
     const int grab = units > 8 * (int64_t)gridDim.x * kApplyWarps ? 2 : 1;
@@ -762,33 +738,17 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
             }
             continue;
         }
-        const int64_t seg = (unit - 6) / (kSegment / kApplySites);
-        const int part = (int)((unit - 6) % (kSegment / kApplySites));
-        const int64_t first = seg * kSegment + part * kApplySites;
+        const int64_t seg = (unit - 6) / (kSegment / kUnitSites);
+        const int part = (int)((unit - 6) % (kSegment / kUnitSites));
+        const int64_t first = seg * kSegment + part * kUnitSites;
         if (first >= sites) continue;
         // the state at the segment's first draw
         const uint32_t seg_a = seg_amb[seg], seg_p = seg_base[seg];
         // ---- meta: the segment's sites before the unit, this lane's 8 sites ---
-        uint32_t sum = 0, ahead = 0;
-        uint32_t m2[2] = {0u, 0u};
-        const int64_t mine = first + lane * 8, far = seg * kSegment + lane * 32;
-        if (first + kApplySites <= sites) {
-            if (lane < part * (kApplySites / 32)) {
-                const uint4 *q = reinterpret_cast<const uint4 *>(meta + far);
-                const uint4 u = q[0], v = q[1];
-                ahead = packed_word(u.x) + packed_word(u.y) + packed_word(u.z) +
-                        packed_word(u.w) + packed_word(v.x) + packed_word(v.y) +
-                        packed_word(v.z) + packed_word(v.w);
-            }
-            const uint2 v = *reinterpret_cast<const uint2 *>(meta + mine);
-            m2[0] = v.x;
-            m2[1] = v.y;
-        } else {  // the chain's last unit
-            if (lane < part * (kApplySites / 32))
-                for (int i = 0; i < 32; ++i) ahead += packed_word(meta[far + i]);
-            for (int i = 0; i < 8; ++i)
-                if (mine + i < sites) m2[i >> 2] |= (uint32_t)meta[mine + i] << (8 * (i & 3));
-        }
+        const UnitMeta um = unit_meta(meta, sites, seg, part);
+        const uint32_t *m2 = um.word;
+        const int64_t mine = first + lane * 8;
+        uint32_t sum = 0;
         // attempted public sites of the lane (bit i: site i)
         const int pub = (int)(su - mine < 0 ? 0 : (su - mine > 8 ? 8 : su - mine));
         uint32_t bits = 0;
@@ -812,14 +772,14 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
             }
         }
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, slot, 31);
-        uint32_t run = __reduce_add_sync(0xFFFFFFFFu, ahead) + inc - sum;
+        uint32_t run = __reduce_add_sync(0xFFFFFFFFu, um.ahead) + inc - sum;
         slot -= listed;
         __syncwarp();  // the previous list is consumed
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const uint32_t m = (m2[i >> 2] >> (8 * (i & 3))) & 0xFFu;
             if ((bits >> i) & 1u) {
-                list[slot] = make_uint2((uint32_t)(part * kApplySites + lane * 8 + i) | (m << 16),
+                list[slot] = make_uint2((uint32_t)(part * kUnitSites + lane * 8 + i) | (m << 16),
                                         (run >> 16) | (run << 16));
                 ++slot;
             }
@@ -970,7 +930,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
     __syncthreads();
     if (!s_last || threadIdx.x != 0) return;
     __threadfence();
-    apply_final(seg_base, seg_amb, segs, extra, s0, ctr, err, capacity);
+    apply_final(seg_base, seg_amb, segs, extra, s0, ctr, walk, err, capacity);
 }
 
 // ---------------------------------------------------------------------------
@@ -985,8 +945,7 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
                           uint8_t *changed_out, uint32_t *err, cudaStream_t stream,
                           const Marks &marks) {
     const int64_t segs = g.segments;
-    DevCounters *ctr = reinterpret_cast<DevCounters *>(b.counters);
-    cudaMemsetAsync(ctr, 0, sizeof(DevCounters), stream);
+    DevCounters *ctr = reinterpret_cast<DevCounters *>(b.counters);  // cleared, as b.walk_zero
     cudaError_t e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
     // the chain and the walk are latency-bound: launched with b.priority, so
@@ -996,38 +955,31 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
     const int pr = b.priority;
     const unsigned seg_blocks = (unsigned)((segs + kSegWarps - 1) / kSegWarps);
     e = launch_prio(k_seg_sums, dim3(seg_blocks), dim3(kSegWarps * 32), 0, stream, pr, meta,
-                    g.sites, segs, b.seg_raw, err);
-    if (e != cudaSuccess) return e;
-    e = launch_prio(k_seg_scan, dim3(1), dim3(1024), 0, stream, pr, b.seg_raw, segs, b.seg_base,
-                    b.seg_amb, err);
-    if (e != cudaSuccess) return e;
-    e = launch_prio(k_amb, dim3(seg_blocks), dim3(kSegWarps * 32), 0, stream, pr, meta, g.sites,
-                    segs, b.seg_raw, b.seg_base, b.seg_amb, b.site_of, b.pos, b.capacity,
-                    err);
+                    g.sites, segs, b.seg_raw, b.seg_base, b.seg_amb, ctr, err);
     if (e != cudaSuccess) return e;
     const uint32_t *n_amb = b.seg_amb + segs;
-    cudaMemsetAsync(b.chunk_two, 0, walk_chunks(b.capacity), stream);
-    cudaMemsetAsync(b.chunk_stat, 0, walk_chunks(b.capacity) * sizeof(ChunkStat), stream);
-    e = launch_prio(k_coef, dim3(1184), dim3(256), 0, stream, pr, b.entries, b.second, b.pos, n_amb,
-                    b.capacity, b.site_of, meta, cand, g.w, rgbi, lut, p, err, b.chunk_two,
-                    b.chunk_stat);
+    const int64_t unit_blocks = (segs * (kSegment / kUnitSites) + kCoefWarps - 1) / kCoefWarps;
+    e = launch_prio(k_coef, dim3((unsigned)std::min<int64_t>(unit_blocks, g_coef_blocks)),
+                    dim3(kCoefWarps * 32), 0, stream, pr, b.entries, b.second, b.capacity, meta,
+                    g.sites, segs, b.seg_raw, b.seg_base, b.seg_amb, cand, g.w, rgbi, lut, p,
+                    b.chunk_two, b.chunk_stat, ctr, err);
     if (e != cudaSuccess) return e;
     marks.mark(5, stream);
     e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
-    e = launch_walk(b.entries, b.second, n_amb, b.capacity, s0, b.walk_scratch, b.per_wave,
-                    b.parallel_walk, b.window_sigmas, b.chunk_two, b.chunk_stat, b.extra,
-                    &ctr->walk_fallbacks, ctr->walk_stats, err, stream, pr);
+    e = launch_walk(b.entries, b.second, n_amb, b.capacity, s0, b.walk_scratch, b.walk_zero,
+                    b.per_wave, b.parallel_walk, b.window_sigmas, b.chunk_two, b.chunk_stat,
+                    b.extra, err, stream, pr);
     if (e != cudaSuccess) return e;
     marks.mark(6, stream);
     e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
     const int64_t apply_blocks =
-        (segs * (kSegment / kApplySites) + 6 + kApplyWarps - 1) / kApplyWarps;
+        (segs * (kSegment / kUnitSites) + 6 + kApplyWarps - 1) / kApplyWarps;
     k_apply<<<(unsigned)std::min<int64_t>(apply_blocks, g_apply_blocks), kApplyWarps * 32, 0,
               stream>>>(meta, cand, g.sites, g.w, rgbi, lut, high, low, ident, stages, p,
                         b.seg_base, b.seg_amb, b.extra, s0 & kLcgMask, rgb_out, changed_out, ctr,
-                        err, b.capacity);
+                        reinterpret_cast<const WalkState *>(b.walk_zero), err, b.capacity);
     marks.mark(7, stream);
     return cudaGetLastError();
 }
