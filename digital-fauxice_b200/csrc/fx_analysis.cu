@@ -261,14 +261,17 @@ __device__ __forceinline__ float rgb_candidate(double avg, const Reciprocals &rc
 }
 
 // The combiner's and writer's float32 profile constants, widened once on the
-// host (the widening is exact).
+// host (the widening is exact), and the writer's dither constants (the same
+// IEEE operations, one division per frame instead of one per pixel).
 struct CombineConst {
     double band_scale[3], factor_a[9], factor_b[9], coarse_slope[3], strength[3];
     double dither_scale[3];
+    DitherConst dither;
 };
 
 static CombineConst combine_const(const fx_params &p) {
     CombineConst c;
+    c.dither = dither_const(p);
     for (int i = 0; i < 3; ++i) {
         c.band_scale[i] = (double)p.band_scales[i];
         c.coarse_slope[i] = (double)p.coarse_slopes[i];
@@ -282,49 +285,73 @@ static CombineConst combine_const(const fx_params &p) {
     return c;
 }
 
-// combine_recovered_candidate (reconstruction.py:807-887).  feats[r][l].
-__device__ bool combine(const float cand[3][3], const float source[3], const float weights[4],
-                        const float feats[5][4], int records, float coarse_reference,
-                        const fx_params &p, const CombineConst &cc, double out[3]) {
-    bool finite = true;
+// Band ranges of a feature record set (reconstruction.py:807-887): the
+// extremes of the records' differences of neighbouring features, rounded to
+// binary32.  The rounding is monotone, so the extremes of the rounded
+// differences are the same values.
+struct BandRanges {
+    float first;             // the centre record's first feature
+    float lo[3], hi[3];
+    bool finite;             // every feature is finite
+};
+
+// One record's rounded differences.
+__device__ __forceinline__ void band_differences(const float f[4], float d[3]) {
+    const double a0 = (double)f[0], a1 = (double)f[1], a2 = (double)f[2], a3 = (double)f[3];
+    d[0] = (float)(a1 - a0);
+    d[1] = (float)(a2 - a1);
+    d[2] = (float)(a3 - a2);
+}
+
+// x * 0 is NaN for an infinite or NaN x and a zero otherwise.
+__device__ __forceinline__ float nonfinite(float x, float seen) { return fmaf(x, 0.0f, seen); }
+
+__device__ BandRanges band_ranges(const float feats[5][4], int records) {
+    BandRanges o;
+    float seen = 0.0f;
+    o.first = feats[0][0];
+    band_differences(feats[0], o.lo);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) o.hi[t] = o.lo[t];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) seen = nonfinite(feats[0][l], seen);
+    for (int r = 1; r < records; ++r) {
+        float d[3];
+        band_differences(feats[r], d);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            o.lo[t] = fminf(o.lo[t], d[t]);
+            o.hi[t] = fmaxf(o.hi[t], d[t]);
+        }
+#pragma unroll
+        for (int l = 0; l < 4; ++l) seen = nonfinite(feats[r][l], seen);
+    }
+    o.finite = seen == 0.0f;
+    return o;
+}
+
+// combine_recovered_candidate (reconstruction.py:807-887).
+__device__ __forceinline__ bool combine(const float cand[3][3], const float source[3],
+                                        const float weights[4], const BandRanges &band,
+                                        float coarse_reference, const fx_params &p,
+                                        const CombineConst &cc, double out[3]) {
+    float seen = 0.0f;
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) finite &= isfinite(cand[k][c]);
+        for (int c = 0; c < 3; ++c) seen = nonfinite(cand[k][c], seen);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) finite &= isfinite(source[c]);
+    for (int c = 0; c < 3; ++c) seen = nonfinite(source[c], seen);
 #pragma unroll
-    for (int l = 0; l < 4; ++l) finite &= isfinite(weights[l]);
-    for (int r = 0; r < records; ++r)
-#pragma unroll
-        for (int l = 0; l < 4; ++l) finite &= isfinite(feats[r][l]);
-    if (!finite) return false;
+    for (int l = 0; l < 4; ++l) seen = nonfinite(weights[l], seen);
+    if (!(band.finite && seen == 0.0f)) return false;
 
-    // band ranges: each record's four values widened once
     double rmin[3], rmax[3];
-    double f00;
-    {
-        const double a0 = (double)feats[0][0], a1 = (double)feats[0][1];
-        const double a2 = (double)feats[0][2], a3 = (double)feats[0][3];
-        f00 = a0;
-        rmin[0] = rmax[0] = a1 - a0;
-        rmin[1] = rmax[1] = a2 - a1;
-        rmin[2] = rmax[2] = a3 - a2;
-    }
-    for (int r = 1; r < records; ++r) {
-        const double a0 = (double)feats[r][0], a1 = (double)feats[r][1];
-        const double a2 = (double)feats[r][2], a3 = (double)feats[r][3];
-        const double d[3] = {a1 - a0, a2 - a1, a3 - a2};
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            rmin[t] = (d[t] < rmin[t]) ? d[t] : rmin[t];
-            rmax[t] = (d[t] > rmax[t]) ? d[t] : rmax[t];
-        }
-    }
+    const double f00 = (double)band.first;
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
-        rmin[t] = (double)(float)rmin[t];
-        rmax[t] = (double)(float)rmax[t];
+        rmin[t] = (double)band.lo[t];
+        rmax[t] = (double)band.hi[t];
     }
     double strengths[3];
     if (p.configured_strengths[0] == 0.0f) {
@@ -388,7 +415,8 @@ __device__ bool combine(const float cand[3][3], const float source[3], const flo
 // reconstruction.py:916-982).  Per channel: 0 = no draw, 1 = one draw,
 // 2 = two draws, 3 = one or two draws depending on the state.
 __device__ uint8_t classify_site(const double cand[3], const float orig[3], bool floor_enabled,
-                                 const CombineConst &cc, const DitherConst &dc, uint32_t *err) {
+                                 const CombineConst &cc, uint32_t *err) {
+    const DitherConst &dc = cc.dither;
     uint8_t meta = 0x80;
     bool valid = true;
 #pragma unroll
@@ -448,19 +476,18 @@ struct Tile {
     static constexpr int BLOCKS_PER_SM = TH == 8 ? 4 : 2;
 };
 
-// A feature record of the stencil (streaming.py:236-308): the four feature
-// values (one 16-byte vector, read by a consumer pixel in one load) and the
-// W of its score patch (the consumer's weights when it is the centre
-// record), kept in three separate planes.  A lane that takes the consumer
-// row's fallback value holds kFallbackBits, a NaN: the feature values are
-// quotients and aux values of finite planes, never NaN, so the marker
-// cannot collide with a value.
+// A feature record of the stencil (streaming.py:236-308) as its consumer
+// pixels use it: the first feature and the three rounded differences (one
+// 16-byte vector) and the W of its score patch (the consumer's weights when
+// it is the centre record), kept in three separate planes.  A record that
+// takes the consumer row's fallback value in a lane, or has a lane that is not
+// finite, holds NaN in its first difference; a pixel that reads one computes
+// its records' features again.
 template <int CR, int RECC>
 struct StencilRecords {
     float4 a[CR][RECC];
     float w[3][CR][RECC];
 };
-constexpr uint32_t kFallbackBits = 0x7FC0FB00u;
 
 // The tiles staged with 16-byte cp.async (hs, hwa, hwr, auxt) start on
 // 16-byte boundaries (checked below); the other members follow them.
@@ -511,6 +538,79 @@ static_assert(sizeof(float) * Tile<8>::RR * Tile<8>::SW >=
               "the attempted list fits in the aux tile");
 static_assert(kTileH % 16 == 0, "padded planes cover whole tiles of either height");
 
+// The features and weights of the record at (r, c) of a tile, from its column
+// sums; `inside` its column is in the row, `aux` its point aux.  Lanes without
+// a value take `fallback`; returns whether there are none.
+template <int TH>
+__device__ __forceinline__ bool record_features(const StencilSmem<TH> &S, int r, int c,
+                                                bool inside, float aux, float fallback,
+                                                float f[4], float rw[3]) {
+    using T = Tile<TH>;
+    if (!inside) {
+        // horizontal guard records stay zero (streaming.py:281-282)
+        f[0] = f[1] = f[2] = f[3] = 0.0f;
+        rw[0] = rw[1] = rw[2] = 0.0f;
+        return true;
+    }
+    double wq[3], nq[3];
+#pragma unroll
+    for (int src = 0; src < 2; ++src) {
+        const float(*s3)[T::CC] = S.cs[src][0];
+        const float(*s5)[T::CC] = S.cs[src][1];
+        const float(*s7)[T::CC] = S.cs[src][2];
+        const float(*s9)[T::CC] = S.cs[src][3];
+        const float(*bb)[T::CC] = S.cs[src][4];
+        double q69, q21;
+        q69_q21([&](int k) { return s3[r][c + k]; }, [&](int k) { return s5[r][c + k]; },
+                [&](int k) { return s7[r][c + k]; }, [&](int k) { return s9[r][c + k]; }, q69,
+                q21);
+        const double q16 = q16_wa([&](int k) { return bb[r][c + k]; });
+        double *dst = src ? nq : wq;
+        dst[0] = q69;
+        dst[1] = q21;
+        dst[2] = q16;
+    }
+    const float point_score = S.hs[r + 4][c + 4];
+    bool regular = point_score > 0.0f;
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+        regular &= wq[l] > 0.0;
+        f[l] = wq[l] > 0.0 ? (float)(nq[l] / wq[l]) : fallback;
+        rw[l] = (float)wq[l];
+    }
+    f[3] = point_score > 0.0f ? aux : fallback;
+    return regular;
+}
+
+// The band ranges of a pixel with an irregular record (score patches that sum
+// to zero, values that are not finite): its records' features once more, with
+// the pixel row's fallback.  Out of the way of the other pixels' registers.
+template <int TH>
+__device__ __noinline__ BandRanges irregular_ranges(const StencilSmem<TH> &S,
+                                                    const float *__restrict__ auxp, int pitch,
+                                                    int w, int ty, int tx, int records,
+                                                    float fallback) {
+    float feats[5][4];
+    for (int k = 0; k < records; ++k) {
+        const int r = ty + (k < 3 ? 1 : (k == 3 ? 0 : 2));
+        const int c = tx + (k == 1 ? 0 : (k == 2 ? 2 : 1));
+        const int xx = (int)blockIdx.x * Tile<TH>::TW - 1 + c;
+        const bool inside = xx >= 0 && xx < w;
+        // the staged aux tile starts at padded row y0 + 1, column x0
+        const float aux = auxp[(int64_t)(blockIdx.y * TH + 1 + r + 3) * pitch +
+                               blockIdx.x * Tile<TH>::TW + c + 3 + Tile<TH>::RO];
+        float rw[3];
+        record_features<TH>(S, r, c, inside, aux, fallback, feats[k], rw);
+    }
+    return band_ranges(feats, records);
+}
+
+// Bound: instruction issue (64 registers and 57 KB per block keep 32 warps on
+// an SM; the conversions' pipe has room: widening the taps with integer
+// multiplies halved its use and saved nothing).  Native frame 1.24 ms, at 5%
+// coverage 1.13.  With four widened features per record and pixel, a fresh
+// row and column division per staged vector and listed record, and the
+// dither constants' division per pixel it took 1.375 and 1.253.
 template <int TH>
 __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
     k_stencil(const uint16_t *__restrict__ rgbi, Geometry g, const float *__restrict__ lut,
@@ -541,37 +641,30 @@ __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
     // 16-byte copies, 11 per staged row, in two groups: first what the
     // decision reads (PR score rows from padded row y0, RR aux rows from
     // padded row y0+1), then the waux rows and the 3 x RR rgb rows.  The
-    // decision runs while the second group is in flight.
+    // decision runs while the second group is in flight.  A thread copies the
+    // same vector of the same rows of every plane, so its addresses differ
+    // by constants.  (Bulk copies of one row each took 300 us more on a native
+    // frame.)
     {
-        constexpr int kVec = T::SW / 4;
-        const int64_t col = x0;
-        constexpr int kRowsA = PR + RR, kRowsB = PR + 3 * RR;
-        for (int i = tid; i < kRowsA * kVec; i += NT) {
-            const int row = i / kVec, v = i % kVec;
-            const bool score = row < PR;
-            const int r = score ? row : row - PR;
-            const float *src = (score ? hs + (int64_t)(y0 + r) * g.pitch
-                                      : auxp + (int64_t)(y0 + 1 + r) * g.pitch) + col;
-            float *dst = score ? S.hs[r] : S.auxt[r];
-            const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + 4 * v);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + 4 * v));
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-        for (int i = tid; i < kRowsB * kVec; i += NT) {
-            const int row = i / kVec, v = i % kVec;
-            const float *src;
-            float *dst;
-            if (row < PR) {
-                src = hwa + (int64_t)(y0 + row) * g.pitch + col;
-                dst = S.hwa[row];
-            } else {
-                const int q = row - PR, k = q / RR, r = q % RR;  // rgb plane k
-                src = hwr + k * plane + (int64_t)(y0 + 1 + r) * g.pitch + col;
-                dst = S.hwr[k][r];
+        constexpr int kVec = T::SW / 4, kStep = NT / kVec;
+        const int row0 = tid / kVec, v = tid % kVec;
+        const int64_t origin = (int64_t)(y0 + row0) * g.pitch + x0 + 4 * v;
+        auto stage = [&](float(*dst)[T::SW], const float *src, int rows) {
+#pragma unroll
+            for (int r = 0; r < rows; r += kStep) {
+                const uint32_t d =
+                    (uint32_t)__cvta_generic_to_shared(dst[0] + (row0 + r) * T::SW + 4 * v);
+                if (row0 < kStep && row0 + r < rows)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d),
+                                 "l"(src + (int64_t)r * g.pitch));
             }
-            const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + 4 * v);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + 4 * v));
-        }
+        };
+        stage(S.hs, hs + origin, PR);
+        stage(S.auxt, auxp + origin + g.pitch, RR);
+        asm volatile("cp.async.commit_group;\n" ::);
+        stage(S.hwa, hwa + origin, PR);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) stage(S.hwr[k], hwr + k * plane + origin + g.pitch, RR);
         asm volatile("cp.async.commit_group;\n" ::);
         asm volatile("cp.async.wait_group 1;\n" ::);  // the first group
     }
@@ -636,21 +729,32 @@ __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
         return;
     }
 
-    // The record positions an attempted pixel reads, listed densely (any
-    // order: each record is computed alone): record row r is the centre row
-    // of pixel row r-1 and the cross neighbour of pixel rows r and r-2.
-    // (A warp-ordered list, by ballot and one atomic per warp, measured 2%
-    // more instructions and no fewer shared-memory bank conflicts.)
-    for (int i = tid; i < CR * RECC; i += NT) {
-        const int r = i / RECC, c = i % RECC;
-        unsigned long long need = 0;
-        if (r >= 1 && r <= TH) {
-            const unsigned long long b = S.rowbal[r - 1];
-            need |= b | (b << 1) | (b << 2);
+    // The record positions an attempted pixel reads, listed densely (row << 8 |
+    // column; rows in any order: each record is computed alone): record row r
+    // is the centre row of pixel row r-1 and the cross neighbour of pixel rows
+    // r and r-2.  A warp lists a row.
+    {
+        const int lane = tid & 31;
+        static_assert(RECC <= 64, "two columns per lane");
+        for (int r = tid >> 5; r < CR; r += NT / 32) {
+            unsigned long long need = 0;
+            if (r >= 1 && r <= TH) {
+                const unsigned long long b = S.rowbal[r - 1];
+                need |= b | (b << 1) | (b << 2);
+            }
+            if (r < TH) need |= (unsigned long long)S.rowbal[r] << 1;
+            if (r >= 2) need |= (unsigned long long)S.rowbal[r - 2] << 1;
+            const uint32_t low = (uint32_t)need, high = (uint32_t)(need >> 32);
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&S.nrec, __popc(low) + __popc(high));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            const uint32_t before = (1u << lane) - 1u;
+            if ((low >> lane) & 1u)
+                S.reclist[at + __popc(low & before)] = (uint16_t)(r << 8 | lane);
+            if ((high >> lane) & 1u)
+                S.reclist[at + __popc(low) + __popc(high & before)] =
+                    (uint16_t)(r << 8 | (32 + lane));
         }
-        if (r < TH) need |= (unsigned long long)S.rowbal[r] << 1;
-        if (r >= 2) need |= (unsigned long long)S.rowbal[r - 2] << 1;
-        if ((need >> c) & 1ull) S.reclist[atomicAdd(&S.nrec, 1)] = (uint16_t)i;
     }
 
     asm volatile("cp.async.wait_group 0;\n" ::);  // the waux and rgb rows
@@ -704,42 +808,17 @@ __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
     const int nrec = S.nrec;
     for (int k = tid; k < nrec; k += NT) {
         const int i = S.reclist[k];
-        const int r = i / RECC, c = i % RECC;
+        const int r = i >> 8, c = i & 0xFF;
         const int xx = x0 - 1 + c;
-        float ra[4], rw[3];
-        if (xx < 0 || xx >= w) {
-            // horizontal guard records stay zero (streaming.py:281-282)
-            ra[0] = ra[1] = ra[2] = ra[3] = 0.0f;
-            rw[0] = rw[1] = rw[2] = 0.0f;
-        } else {
-            double wq[3], nq[3];
+        float f[4], d[3], rw[3];
+        const bool regular = record_features<TH>(S, r, c, xx >= 0 && xx < w,
+                                                 S.auxt[r + 3][c + 3 + RO], 0.0f, f, rw);
+        band_differences(f, d);
+        float seen = 0.0f;
 #pragma unroll
-            for (int src = 0; src < 2; ++src) {
-                const float(*s3)[CC] = S.cs[src][0];
-                const float(*s5)[CC] = S.cs[src][1];
-                const float(*s7)[CC] = S.cs[src][2];
-                const float(*s9)[CC] = S.cs[src][3];
-                const float(*bb)[CC] = S.cs[src][4];
-                double q69, q21;
-                q69_q21([&](int k) { return s3[r][c + k]; }, [&](int k) { return s5[r][c + k]; },
-                        [&](int k) { return s7[r][c + k]; }, [&](int k) { return s9[r][c + k]; },
-                        q69, q21);
-                const double q16 = q16_wa([&](int k) { return bb[r][c + k]; });
-                double *dst = src ? nq : wq;
-                dst[0] = q69;
-                dst[1] = q21;
-                dst[2] = q16;
-            }
-            const float point_score = S.hs[r + 4][c + 4];
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-                ra[l] = wq[l] > 0.0 ? (float)(nq[l] / wq[l]) : __uint_as_float(kFallbackBits);
-                rw[l] = (float)wq[l];
-            }
-            ra[3] = point_score > 0.0f ? S.auxt[r + 3][c + 3 + RO]  // xx is inside the row
-                                       : __uint_as_float(kFallbackBits);
-        }
-        S.rec.a[r][c] = make_float4(ra[0], ra[1], ra[2], ra[3]);
+        for (int l = 0; l < 4; ++l) seen = nonfinite(f[l], seen);
+        if (!regular || seen != 0.0f) d[0] = __uint_as_float(0x7FC00000u);
+        S.rec.a[r][c] = make_float4(f[0], d[0], d[1], d[2]);
         S.rec.w[0][r][c] = rw[0];
         S.rec.w[1][r][c] = rw[1];
         S.rec.w[2][r][c] = rw[2];
@@ -781,15 +860,31 @@ __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
 
     const float fallback = ws.coarse;
     const int records = p.cross_neighbor ? 5 : 1;
-    float feats[5][4];
-    const int rr[5] = {ty + 1, ty + 1, ty + 1, ty, ty + 2};
-    const int rc[5] = {tx + 1, tx, tx + 2, tx + 1, tx + 1};
-    for (int k = 0; k < records; ++k) {
-        const float4 q = S.rec.a[rr[k]][rc[k]];
-        const float rec_a[4] = {q.x, q.y, q.z, q.w};
+    BandRanges band;
+    {
+        const float4 q = S.rec.a[ty + 1][tx + 1];
+        bool regular = q.y == q.y;
+        band.first = q.x;
+        band.lo[0] = band.hi[0] = q.y;
+        band.lo[1] = band.hi[1] = q.z;
+        band.lo[2] = band.hi[2] = q.w;
+        if (records == 5) {
 #pragma unroll
-        for (int l = 0; l < 4; ++l)
-            feats[k][l] = __float_as_uint(rec_a[l]) == kFallbackBits ? fallback : rec_a[l];
+            for (int k = 1; k < 5; ++k) {
+                const float4 n = S.rec.a[ty + (k < 3 ? 1 : (k == 3 ? 0 : 2))]
+                                        [tx + (k == 1 ? 0 : (k == 2 ? 2 : 1))];
+                regular &= n.y == n.y;
+                band.lo[0] = fminf(band.lo[0], n.y);
+                band.hi[0] = fmaxf(band.hi[0], n.y);
+                band.lo[1] = fminf(band.lo[1], n.z);
+                band.hi[1] = fmaxf(band.hi[1], n.z);
+                band.lo[2] = fminf(band.lo[2], n.w);
+                band.hi[2] = fmaxf(band.hi[2], n.w);
+            }
+        }
+        band.finite = true;
+        if (!regular)
+            band = irregular_ranges<TH>(S, auxp, g.pitch, w, ty, tx, records, fallback);
     }
     // W of the centre record (record row ty + 1, column tx + 1): the score
     // patch averages its record phase computed, and the point score
@@ -829,13 +924,12 @@ __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
         }
     }
     double combined[3];
-    if (!combine(cand, orig, weights, feats, records, ws.coarse, p, cc, combined)) {
+    if (!combine(cand, orig, weights, band, ws.coarse, p, cc, combined)) {
         raise_error(err, FX_ERR_COMBINER_INPUT);
         meta_out[site] = 0;
         return;
     }
-    const DitherConst dc = dither_const(p);
-    meta_out[site] = classify_site(combined, orig, floor_enabled, cc, dc, err);
+    meta_out[site] = classify_site(combined, orig, floor_enabled, cc, err);
     double *dst = cand_out + 3 * site;
     dst[0] = combined[0];
     dst[1] = combined[1];
@@ -982,13 +1076,12 @@ __global__ void k_startup(const uint16_t *__restrict__ rgbi, StartupView v,
     const float orig[3] = {__ldg(lut + (raw.x & 0xFFFFu)), __ldg(lut + (raw.x >> 16)),
                            __ldg(lut + (raw.y & 0xFFFFu))};
     double combined[3];
-    if (!combine(cand, orig, weights, feats, records, act.coarse, p, cc, combined)) {
+    if (!combine(cand, orig, weights, band_ranges(feats, records), act.coarse, p, cc, combined)) {
         raise_error(err, FX_ERR_COMBINER_INPUT);
         meta_out[site] = 0;
         return;
     }
-    const DitherConst dc = dither_const(p);
-    meta_out[site] = classify_site(combined, orig, floor_enabled, cc, dc, err);
+    meta_out[site] = classify_site(combined, orig, floor_enabled, cc, err);
     double *dst = cand_out + 3 * site;
     dst[0] = combined[0];
     dst[1] = combined[1];

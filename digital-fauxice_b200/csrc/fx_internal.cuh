@@ -136,7 +136,7 @@ struct DitherConst {
     int low_lt_high;
 };
 
-__device__ __forceinline__ DitherConst dither_const(const fx_params &p) {
+__host__ __device__ __forceinline__ DitherConst dither_const(const fx_params &p) {
     DitherConst d;
     d.low = (double)p.dither_low;
     d.high = (double)p.dither_high;
