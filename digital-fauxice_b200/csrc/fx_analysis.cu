@@ -965,113 +965,155 @@ __device__ __forceinline__ float su_raw(const StartupView &v, int y, int xp) {
     return y >= 0 ? src[w - 1] : 0.0f;
 }
 
-// startup.py:131-183 (weights are only needed for the centre record).
-__device__ void su_record(const StartupView &v, int ly, int x, float fallback, float weights[4],
-                          float feature[4]) {
-    if (ly <= -6 || x < 0 || x >= v.g.w) {
-#pragma unroll
-        for (int l = 0; l < 4; ++l) weights[l] = feature[l] = 0.0f;
-        return;
-    }
-    ColumnSums sc[9], wc[9];
-#pragma unroll
-    for (int j = 0; j < 9; ++j) {
-        float a[9], b[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            a[i] = su_plane(v, v.hs, ly - 4 + i, x - 4 + j);
-            b[i] = su_plane(v, v.hwa, ly - 4 + i, x - 4 + j);
-        }
-        sc[j] = column_sums(a);
-        wc[j] = column_sums(b);
-    }
-    double wq[3], nq[3];
-    q69_q21([&](int k) { return sc[k].s3; }, [&](int k) { return sc[k].s5; },
-            [&](int k) { return sc[k].s7; }, [&](int k) { return sc[k].s9; }, wq[0], wq[1]);
-    wq[2] = q16_wa([&](int k) { return sc[k].b16; });
-    q69_q21([&](int k) { return wc[k].s3; }, [&](int k) { return wc[k].s5; },
-            [&](int k) { return wc[k].s7; }, [&](int k) { return wc[k].s9; }, nq[0], nq[1]);
-    nq[2] = q16_wa([&](int k) { return wc[k].b16; });
-    weights[0] = (float)wq[0];
-    weights[1] = (float)wq[1];
-    weights[2] = (float)wq[2];
-    weights[3] = su_plane(v, v.hs, ly, x);
-#pragma unroll
-    for (int l = 0; l < 3; ++l) feature[l] = (wq[l] > 0.0) ? (float)(nq[l] / wq[l]) : fallback;
-    feature[3] = (weights[3] > 0.0f) ? su_raw(v, ly, x + 4) : fallback;
-}
-
 __device__ __forceinline__ int max1(int v) { return v < 1 ? 1 : v; }
 
-__global__ void k_startup(const uint16_t *__restrict__ rgbi, StartupView v,
-                          const float *__restrict__ lut, const fx_stage *__restrict__ stages,
-                          fx_params p, CombineConst cc, double *__restrict__ cand_out,
-                          uint8_t *__restrict__ meta_out, uint32_t *err) {
+// One block computes 32 columns of one hidden stage in four steps: column
+// sums of the three record rows' score and waux patches and of the centre
+// row's RGB patches, with the decision bars (one item per column and plane,
+// per pixel and bar); the records; the RGB candidates, a thread per pixel and
+// channel; the combination, a thread per pixel.
+//
+// Bound: latency (6 W sites).  A thread per site, with all of its five
+// records' sums in 255 registers, took 55 us on every frame; only frames
+// whose stencil is longer hid it.
+constexpr int kSuCols = 32, kSuThreads = 256;
+struct StartupSmem {
+    float cs[2][5][3][kSuCols + 10];  // [score|waux][S3,S5,S7,S9,B16][row][column x0-5 ..]
+    float rcs[3][4][kSuCols + 8];     // [channel][S3,S5,S7,S9][column x0-4 ..]
+    float feature[3][kSuCols + 2][4]; // [row][column x0-1 ..]
+    float weight[4][kSuCols];         // of the centre row's records
+    float cand[3][3][kSuCols];
+    uint8_t bar[4][kSuCols];          // the bar counts more than the limit
+};
+
+__global__ void __launch_bounds__(kSuThreads)
+    k_startup(const uint16_t *__restrict__ rgbi, StartupView v, const float *__restrict__ lut,
+              const fx_stage *__restrict__ stages, fx_params p, CombineConst cc,
+              double *__restrict__ cand_out, uint8_t *__restrict__ meta_out, uint32_t *err) {
+    __shared__ StartupSmem S;
     if (pass_stopped(err)) return;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int CC = kSuCols + 10, RC = kSuCols + 8, RECC = kSuCols + 2;
+    const int tid = threadIdx.x;
+    const int x0 = blockIdx.x * kSuCols, w = v.g.w;
     const int k = blockIdx.y;  // stage hit k+1, centre k-6
-    const int w = v.g.w;
-    if (x >= w) return;
-    const int64_t site = (int64_t)k * w + x;
     const int hit = k + 1, center = k - 6;
+    const int rows = p.cross_neighbor ? 3 : 1;  // record rows: the centre first
+    auto record_row = [&](int i) { return center + (i == 0 ? 0 : (i == 1 ? -1 : 1)); };
+
+    const int sums = 2 * rows * CC, rgb = 3 * RC, bars = 4 * kSuCols;
+    for (int it = tid; it < sums + rgb + bars; it += kSuThreads) {
+        if (it < sums + rgb) {
+            const bool wa = it < sums;
+            const int q = wa ? it : it - sums;
+            const int line = wa ? q / CC : q / RC, c = wa ? q % CC : q % RC;
+            const int src = line / rows, row = line % rows;
+            const float *pl = wa ? (src ? v.hwa : v.hs) : v.hwr + line * v.plane;
+            const int y = wa ? record_row(row) : center, x = x0 + c - (wa ? 5 : 4);
+            float a[9];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) a[i] = su_plane(v, pl, y - 4 + i, x);
+            const ColumnSums o = column_sums(a);
+            if (wa) {
+                S.cs[src][0][row][c] = o.s3;
+                S.cs[src][1][row][c] = o.s5;
+                S.cs[src][2][row][c] = o.s7;
+                S.cs[src][3][row][c] = o.s9;
+                S.cs[src][4][row][c] = o.b16;
+            } else {
+                S.rcs[line][0][c] = o.s3;
+                S.rcs[line][1][c] = o.s5;
+                S.rcs[line][2][c] = o.s7;
+                S.rcs[line][3][c] = o.s9;
+            }
+        } else {
+            const int q = it - sums - rgb, gi = q / kSuCols, c = q % kSuCols;
+            const int r = p.radius;
+            int count = 0;
+#pragma unroll
+            for (int s = 0; s < 9; ++s) {
+                const int axis = s - 4;
+                const int dy = (gi == 0 || gi == 2) ? axis : (gi == 1 ? -r : r);
+                const int dx = (gi == 0) ? -r : (gi == 2 ? r : axis);
+                count += su_raw(v, center + dy, x0 + c + 4 + dx) < p.decision_threshold;
+            }
+            S.bar[gi][c] = count > p.count_limit;
+        }
+    }
+    __syncthreads();
+
+    // records (startup.py:131-183); the centre row's neighbours too
+    for (int it = tid; it < rows * RECC; it += kSuThreads) {
+        const int row = it / RECC, c = it % RECC;
+        const int ly = record_row(row), x = x0 - 1 + c;
+        float f[4] = {0.0f, 0.0f, 0.0f, 0.0f}, weights[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (ly > -6 && x >= 0 && x < w) {
+            const float fallback = stages[max1(ly + 6) - 1].coarse;
+            double wq[3], nq[3];
+#pragma unroll
+            for (int src = 0; src < 2; ++src) {
+                double *dst = src ? nq : wq;
+                const auto &t = S.cs[src];
+                q69_q21([&](int j) { return t[0][row][c + j]; },
+                        [&](int j) { return t[1][row][c + j]; },
+                        [&](int j) { return t[2][row][c + j]; },
+                        [&](int j) { return t[3][row][c + j]; }, dst[0], dst[1]);
+                dst[2] = q16_wa([&](int j) { return t[4][row][c + j]; });
+            }
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                weights[l] = (float)wq[l];
+                f[l] = (wq[l] > 0.0) ? (float)(nq[l] / wq[l]) : fallback;
+            }
+            weights[3] = su_plane(v, v.hs, ly, x);
+            f[3] = (weights[3] > 0.0f) ? su_raw(v, ly, x + 4) : fallback;
+        }
+#pragma unroll
+        for (int l = 0; l < 4; ++l) S.feature[row][c][l] = f[l];
+        if (row == 0 && c >= 1 && c <= kSuCols)
+#pragma unroll
+            for (int l = 0; l < 4; ++l) S.weight[l][c - 1] = weights[l];
+    }
+    __syncthreads();
+
+    if (tid < 3 * kSuCols) {
+        const int ch = tid / kSuCols, c = tid % kSuCols;
+        const float weights[4] = {S.weight[0][c], S.weight[1][c], S.weight[2][c], S.weight[3][c]};
+        const Reciprocals rcp = weight_reciprocals(weights);
+        const float *pl = v.hwr + ch * v.plane;
+        const auto &t = S.rcs[ch];
+        double q69, q21;
+        q69_q21([&](int j) { return t[0][c + j]; }, [&](int j) { return t[1][c + j]; },
+                [&](int j) { return t[2][c + j]; }, [&](int j) { return t[3][c + j]; }, q69, q21);
+        const double q16 = q16_rgb(
+            [&](int i, int j) { return su_plane(v, pl, center - 1 + i, x0 + c - 1 + j); });
+        S.cand[0][ch][c] = rgb_candidate(q69, rcp, 0);
+        S.cand[1][ch][c] = rgb_candidate(q21, rcp, 1);
+        S.cand[2][ch][c] = rgb_candidate(q16, rcp, 2);
+    }
+    __syncthreads();
+
+    const int c = tid, x = x0 + c;
+    if (c >= kSuCols || x >= w) return;
+    const int64_t site = (int64_t)k * w + x;
     const fx_stage act = stages[hit - 1];
     const bool floor_enabled = p.driver_gate_primary || act.gate_secondary;
     const int writer_width = (p.cross_neighbor && hit <= 2) ? w - 4 : w;
-    if (x >= writer_width) {
+    const float weights[4] = {S.weight[0][c], S.weight[1][c], S.weight[2][c], S.weight[3][c]};
+    if (x >= writer_width || S.bar[0][c] || S.bar[1][c] || S.bar[2][c] || S.bar[3][c] ||
+        act.row_gate != 0 || (floor_enabled && weights[3] >= 1.0f)) {
         meta_out[site] = 0;
         return;
     }
-    const int r = p.radius;
-    bool fallback_hit = false;
-    for (int gi = 0; gi < 4 && !fallback_hit; ++gi) {
-        int count = 0;
-        for (int s = 0; s < 9; ++s) {
-            const int axis = s - 4;
-            const int dy = (gi == 0 || gi == 2) ? axis : (gi == 1 ? -r : r);
-            const int dx = (gi == 0) ? -r : (gi == 2 ? r : axis);
-            count += su_raw(v, center + dy, x + 4 + dx) < p.decision_threshold;
-        }
-        if (count > p.count_limit) fallback_hit = true;
-    }
-    const float fb_center = stages[max1(center + 6) - 1].coarse;
-    float weights[4], feats[5][4];
-    su_record(v, center, x, fb_center, weights, feats[0]);
-    if (fallback_hit || act.row_gate != 0 || (floor_enabled && weights[3] >= 1.0f)) {
-        meta_out[site] = 0;
-        return;
-    }
-    const Reciprocals rcp = weight_reciprocals(weights);
-    float cand[3][3];
+    float cand[3][3], feats[5][4];
 #pragma unroll
-    for (int ch = 0; ch < 3; ++ch) {
-        const float *pl = v.hwr + ch * v.plane;
-        ColumnSums cs[9];
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            float a[9];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) a[i] = su_plane(v, pl, center - 4 + i, x - 4 + j);
-            cs[j] = column_sums(a);
-        }
-        double q69, q21;
-        q69_q21([&](int kk) { return cs[kk].s3; }, [&](int kk) { return cs[kk].s5; },
-                [&](int kk) { return cs[kk].s7; }, [&](int kk) { return cs[kk].s9; }, q69, q21);
-        const double q16 = q16_rgb(
-            [&](int i, int j) { return su_plane(v, pl, center - 1 + i, x - 1 + j); });
-        cand[0][ch] = rgb_candidate(q69, rcp, 0);
-        cand[1][ch] = rgb_candidate(q21, rcp, 1);
-        cand[2][ch] = rgb_candidate(q16, rcp, 2);
-    }
+        for (int ch = 0; ch < 3; ++ch) cand[i][ch] = S.cand[i][ch][c];
     const int records = p.cross_neighbor ? 5 : 1;
-    if (records == 5) {
-        float wn[4];
-        const float fb_up = stages[max1(center + 5) - 1].coarse;
-        const float fb_down = stages[max1(center + 7) - 1].coarse;
-        su_record(v, center, x - 1, fb_center, wn, feats[1]);
-        su_record(v, center, x + 1, fb_center, wn, feats[2]);
-        su_record(v, center - 1, x, fb_up, wn, feats[3]);
-        su_record(v, center + 1, x, fb_down, wn, feats[4]);
-    }
+    for (int i = 0; i < records; ++i)  // centre, left, right, up, down
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            feats[i][l] = S.feature[i < 3 ? 0 : i - 2][c + (i == 1 ? 0 : (i == 2 ? 2 : 1))][l];
     const uint2 raw = reinterpret_cast<const uint2 *>(rgbi)[x];  // row 0
     const float orig[3] = {__ldg(lut + (raw.x & 0xFFFFu)), __ldg(lut + (raw.x >> 16)),
                            __ldg(lut + (raw.y & 0xFFFFu))};
@@ -1109,7 +1151,7 @@ cudaError_t launch_analysis(const uint16_t *rgbi, const Geometry &g, const float
     // GPU) runs on `side` beside the stencil: both only read the planes and
     // they write disjoint sites (startup sites 0 .. 6W-1, public ones after)
     StartupView v{g, aux, hs, hwa, hwr, plane, p.cross_neighbor ? 5 : 4};
-    const dim3 su_block(128), su_grid((g.w + 127) / 128, 6);
+    const dim3 su_block(kSuThreads), su_grid((g.w + kSuCols - 1) / kSuCols, 6);
     if (side) {
         cudaError_t e = cudaEventRecord(fork, stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
