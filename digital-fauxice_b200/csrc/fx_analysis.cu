@@ -18,105 +18,136 @@ namespace fx {
 // Planes
 // ---------------------------------------------------------------------------
 
-// The auxiliary value of one pixel (x3a.py:193-221): stage y+1's alpha and
-// offset, visible lane and IR lane through the LUT, binary64 then float.
-__device__ __forceinline__ float aux_value(const uint2 raw, const fx_stage &st, int visible,
-                                           const float *__restrict__ lut, uint32_t *err) {
-    float a;
-    if (st.alpha == 1.0f) {
-        if (!st.replacement_valid) raise_error(err, FX_ERR_ALPHA_ONE_UNBOUND);
-        a = st.replacement;
-    } else {
-        const uint32_t lanes[4] = {raw.x & 0xFFFFu, raw.x >> 16, raw.y & 0xFFFFu, raw.y >> 16};
-        const double vis = (double)__ldg(lut + lanes[visible]);
-        const double ir = (double)__ldg(lut + lanes[3]);
-        const double alpha = (double)st.alpha;
-        const double offset = (double)st.offset;
-        a = (float)((ir - alpha * vis) / (1.0 - alpha) - offset);
+// The auxiliary value of one row's pixels (x3a.py:193-221): stage y+1's alpha
+// and offset, visible lane and IR lane through the LUT, binary64 then float.
+struct AuxRow {
+    double alpha, offset, divisor, reciprocal;
+    float replacement;
+    bool replaced;
+    __device__ explicit AuxRow(const fx_stage &st, uint32_t *err)
+        : alpha((double)st.alpha), offset((double)st.offset), divisor(1.0 - alpha),
+          reciprocal(1.0 / divisor), replacement(st.replacement), replaced(st.alpha == 1.0f) {
+        if (replaced && !st.replacement_valid) raise_error(err, FX_ERR_ALPHA_ONE_UNBOUND);
     }
-    if (!isfinite(a)) raise_error(err, FX_ERR_NONFINITE_AUX);
-    return a;
-}
+    // x / divisor, correctly rounded: Markstein's theorem (a faithful quotient
+    // corrected by its exact remainder times the correctly rounded reciprocal
+    // rounds to the quotient).  The first correction makes the product with the
+    // reciprocal faithful.  Nothing underflows: x is 0 or at least 2^-298 (a
+    // difference of binary32 values and products of two) and the divisor at
+    // most 2^129.
+    __device__ __forceinline__ double quotient(double x) const {
+        double q = x * reciprocal;
+        q = fma(fma(-divisor, q, x), reciprocal, q);
+        return fma(fma(-divisor, q, x), reciprocal, q);
+    }
+    __device__ __forceinline__ float value(float visible, float ir) const {
+        if (replaced) return replacement;
+        return (float)(quotient((double)ir - alpha * (double)visible) - offset);
+    }
+};
+
+// x * 0 is NaN for an infinite or NaN x and a zero otherwise.
+__device__ __forceinline__ float nonfinite(float x, float seen) { return fmaf(x, 0.0f, seen); }
 
 // One padded row segment of the history planes (streaming.py:111-147,
-// 201-233), with the auxiliary plane computed on the way.  A block of 256
-// threads covers kPlaneCols = 254 columns: thread t computes the aux of
-// column base + t - 1, so the first and last thread compute only the
-// segment's outer neighbours for the horizontal minimum and every thread
-// computes one aux value.  History planes: rows above the
-// image take the pseudo row, rows below repeat the last row, columns outside
-// are zero.  The auxiliary plane is written padded too, but edge-replicated
-// (the decision bars clamp their indices, streaming.py:166-198): padded
-// (y, x) holds the aux of (clamp(y), clamp(x)).
-constexpr int kPlaneCols = 254;  // output columns per 256-thread k_planes block
+// 201-233), with the auxiliary plane computed on the way.  A thread computes
+// four neighbouring columns of the padded row and writes 16 bytes to each
+// plane; the horizontal minimum takes the neighbours' aux values from the
+// lanes beside it, and a warp's first and last lane compute one more.
+// History planes: rows above the image take the pseudo row, rows below repeat
+// the last row, columns outside are zero.  The auxiliary plane is written
+// padded too, but edge-replicated (the decision bars clamp their indices,
+// streaming.py:166-198): padded (y, x) holds the aux of (clamp(y), clamp(x)).
+//
+// Bound: wavefronts in L1 (the four LUT gathers per pixel; 61% of its peak)
+// and the planes' bytes (32 per position, 4 TB/s).  Native frame 159 us;
+// one column per thread, each with its own binary64 division and a fifth
+// gather, took 217.  Stores that stay in L2 (no .cs) 165; a column per lane
+// and four rounds 168; eight columns per thread 213; 64 warps per SM at 32
+// registers 178 (the table has to share L1 with more rows).
+constexpr int kPlaneThreads = 128, kPlaneRun = 4;
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kPlaneThreads)
     k_planes(const uint16_t *__restrict__ rgbi, Geometry g, const float *__restrict__ lut,
              const fx_stage *__restrict__ stages, fx_params p, float *__restrict__ auxp,
              float *__restrict__ hs, float *__restrict__ hwa, float *__restrict__ hwr,
              int64_t plane, uint32_t *err) {
-    __shared__ float s_aux[256];  // aux of columns base-1 .. base+254 of the segment
     if (pass_stopped(err)) return;
-    const int t = threadIdx.x;
-    const bool owner = t >= 1 && t <= kPlaneCols;  // threads 0 and 255: neighbours only
-    const int px = blockIdx.x * kPlaneCols + t - 1;
+    const int t = threadIdx.x, lane = t & 31;
+    const int px = (blockIdx.x * kPlaneThreads + t) * kPlaneRun;
     const int py = blockIdx.y;
-    const int y = py - kPad, x = px - kPad;
+    const int y = py - kPad, x0 = px - kPad;
     const bool live = y >= -1;  // rows above the pseudo row are zero
     const int r = y < 0 ? 0 : (y < g.h ? y : g.h - 1);
-    const int64_t row0 = (int64_t)r * g.w;
-    const fx_stage ast = stages[r];  // stage y+1 (stage_parameters.py:207-212)
-    const bool inside = x >= 0 && x < g.w;
-    const bool own = live && px >= 0 && px < g.pitch && inside;
-    uint2 raw = make_uint2(0u, 0u);
-    float a = 0.0f;
-    if (px >= 0 && px < g.pitch) {
-        // the aux of (clamp(y), clamp(x)), for the edge-replicated plane
-        const int xc = x < 0 ? 0 : (x < g.w ? x : g.w - 1);
-        const uint2 rc = reinterpret_cast<const uint2 *>(rgbi)[row0 + xc];
-        const float ac = aux_value(rc, ast, p.visible_channel, lut, err);
-        if (owner) auxp[(int64_t)py * g.pitch + px] = ac;
-        if (own) {
-            raw = rc;
-            a = ac;
-        }
+    const uint2 *row = reinterpret_cast<const uint2 *>(rgbi) + (int64_t)r * g.w;
+    const AuxRow aux(stages[r], err);  // stage y+1 (stage_parameters.py:207-212)
+    const int visible = p.visible_channel;
+    float seen = 0.0f;
+    // a column's LUT values and the aux of its clamped column
+    auto column = [&](int x, float rgb[3]) {
+        const uint2 raw = row[min(max(x, 0), g.w - 1)];
+        rgb[0] = __ldg(lut + (raw.x & 0xFFFFu));
+        rgb[1] = __ldg(lut + (raw.x >> 16));
+        rgb[2] = __ldg(lut + (raw.y & 0xFFFFu));
+        const float ir = __ldg(lut + (raw.y >> 16));
+        const float vis = visible == 0 ? rgb[0] : (visible == 1 ? rgb[1] : rgb[2]);
+        const float a = aux.value(vis, ir);
+        seen = nonfinite(a, seen);
+        return a;
+    };
+    const bool inside_row = px < g.pitch;
+    float rgb[kPlaneRun][3], a[kPlaneRun], outer = 0.0f;
+    if (inside_row) {
+#pragma unroll
+        for (int j = 0; j < kPlaneRun; ++j) a[j] = column(x0 + j, rgb[j]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < kPlaneRun; ++j) a[j] = rgb[j][0] = rgb[j][1] = rgb[j][2] = 0.0f;
     }
-    s_aux[t] = a;  // 0 outside the row, as the horizontal minimum's guard needs
-    __syncthreads();
-    if (!owner || px < 0 || px >= g.pitch) return;
+    if (p.horizontal_minimum && (lane == 0 || lane == 31)) {
+        float unused[3];
+        outer = column(lane == 0 ? x0 - 1 : x0 + kPlaneRun, unused);
+    }
+    float left = __shfl_up_sync(0xFFFFFFFFu, a[kPlaneRun - 1], 1);
+    float right = __shfl_down_sync(0xFFFFFFFFu, a[0], 1);
+    if (lane == 0) left = outer;
+    if (lane == 31) right = outer;
+    if (!inside_row) return;
+    if (seen != 0.0f) raise_error(err, FX_ERR_NONFINITE_AUX);  // also when it is NaN
+
     const float floor = p.score_floor;
-    float s = 0.0f, wa = 0.0f, wr[3] = {0.0f, 0.0f, 0.0f};
-    if (own) {
-        const float rgb[3] = {__ldg(lut + (raw.x & 0xFFFFu)), __ldg(lut + (raw.x >> 16)),
-                              __ldg(lut + (raw.y & 0xFFFFu))};
-        if (y == -1) {
-            // the pseudo row above the image (streaming.py:218-228)
-            s = floor;
-            wa = a * floor;
-            for (int c = 0; c < 3; ++c) wr[c] = rgb[c] * floor;
-        } else {
-            float sample = a;
-            if (p.horizontal_minimum && g.w > 2 && x > 0 && x < g.w - 1) {
-                const float l = s_aux[t - 1], rr = s_aux[t + 1];
-                const float m = (l < a) ? l : a;
-                sample = (m < rr) ? m : rr;
-            }
-            const double primary = (double)stages[r + 1].score_base;  // stage y+2
-            double sc = (((primary + (double)p.score_addend) - (double)sample) *
-                         (double)p.score_scale) + (double)p.score_offset;
-            sc = (sc > 1.0) ? 1.0 : sc;
-            sc = (sc < (double)floor) ? (double)floor : sc;
-            s = (float)sc;
-            wa = s * a;
-            for (int c = 0; c < 3; ++c) wr[c] = s * rgb[c];
+    const double base = (double)stages[r + 1].score_base + (double)p.score_addend;  // stage y+2
+    const double scale = (double)p.score_scale, offset = (double)p.score_offset;
+    float s[kPlaneRun], wa[kPlaneRun], wr[3][kPlaneRun];
+#pragma unroll
+    for (int j = 0; j < kPlaneRun; ++j) {
+        const int x = x0 + j;
+        const float l = j == 0 ? left : a[j - 1], rr = j == kPlaneRun - 1 ? right : a[j + 1];
+        float sample = a[j];
+        if (p.horizontal_minimum && x > 0 && x < g.w - 1) {
+            const float m = (l < a[j]) ? l : a[j];
+            sample = (m < rr) ? m : rr;
         }
+        // clipped to [floor, 1] after the rounding, which is monotone
+        float v = (float)(((base - (double)sample) * scale) + offset);
+        v = (v > 1.0f) ? 1.0f : v;
+        v = (v < floor) ? floor : v;
+        if (y < 0) v = floor;  // the pseudo row above the image (streaming.py:218-228)
+        const bool own = live && x >= 0 && x < g.w;
+        s[j] = own ? v : 0.0f;
+        wa[j] = own ? v * a[j] : 0.0f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) wr[c][j] = own ? v * rgb[j][c] : 0.0f;
     }
     const int64_t o = (int64_t)py * g.pitch + px;
-    hs[o] = s;
-    hwa[o] = wa;
-    hwr[o] = wr[0];
-    hwr[o + plane] = wr[1];
-    hwr[o + 2 * plane] = wr[2];
+    auto put = [&](float *dst, const float q[kPlaneRun]) {
+        __stcs(reinterpret_cast<float4 *>(dst + o), make_float4(q[0], q[1], q[2], q[3]));
+    };
+    put(auxp, a);
+    put(hs, s);
+    put(hwa, wa);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) put(hwr + c * plane, wr[c]);
 }
 
 // ---------------------------------------------------------------------------
@@ -302,9 +333,6 @@ __device__ __forceinline__ void band_differences(const float f[4], float d[3]) {
     d[1] = (float)(a2 - a1);
     d[2] = (float)(a3 - a2);
 }
-
-// x * 0 is NaN for an infinite or NaN x and a zero otherwise.
-__device__ __forceinline__ float nonfinite(float x, float seen) { return fmaf(x, 0.0f, seen); }
 
 __device__ BandRanges band_ranges(const float feats[5][4], int records) {
     BandRanges o;
@@ -1142,9 +1170,10 @@ cudaError_t launch_analysis(const uint16_t *rgbi, const Geometry &g, const float
                             cudaEvent_t join) {
     const CombineConst cc = combine_const(p);
     {
-        dim3 block(256), grid((g.pitch + kPlaneCols - 1) / kPlaneCols, g.prow);
-        k_planes<<<grid, block, 0, stream>>>(rgbi, g, lut, stages, p, aux, hs, hwa, hwr, plane,
-                                             err);
+        constexpr int kColumns = kPlaneThreads * kPlaneRun;
+        const dim3 grid((g.pitch + kColumns - 1) / kColumns, g.prow);
+        k_planes<<<grid, kPlaneThreads, 0, stream>>>(rgbi, g, lut, stages, p, aux, hs, hwa, hwr,
+                                                     plane, err);
     }
     marks.mark(2, stream);
     // k_startup (the six hidden stages, 6 W sites: too few blocks to fill the
