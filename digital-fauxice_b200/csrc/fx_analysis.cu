@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(kPlaneThreads)
              const fx_stage *__restrict__ stages, fx_params p, float *__restrict__ auxp,
              float *__restrict__ hs, float *__restrict__ hwa, float *__restrict__ hwr,
              int64_t plane, uint32_t *err) {
+    grid_dependency();
     if (pass_stopped(err)) return;
     const int t = threadIdx.x, lane = t & 31;
     const int px = (blockIdx.x * kPlaneThreads + t) * kPlaneRun;
@@ -651,6 +652,7 @@ __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
     constexpr int RECC = T::RECC, RO = T::RO, NT = T::THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StencilSmem<TH> &S = *reinterpret_cast<StencilSmem<TH> *>(smem_raw);
+    grid_dependency();
     if (pass_stopped(err)) return;
     const int tid = threadIdx.x;
     const int y0 = blockIdx.y * TH, x0 = blockIdx.x * T::TW;
@@ -1019,6 +1021,7 @@ __global__ void __launch_bounds__(kSuThreads)
               const fx_stage *__restrict__ stages, fx_params p, CombineConst cc,
               double *__restrict__ cand_out, uint8_t *__restrict__ meta_out, uint32_t *err) {
     __shared__ StartupSmem S;
+    grid_dependency();
     if (pass_stopped(err)) return;
     constexpr int CC = kSuCols + 10, RC = kSuCols + 8, RECC = kSuCols + 2;
     const int tid = threadIdx.x;
@@ -1172,8 +1175,9 @@ cudaError_t launch_analysis(const uint16_t *rgbi, const Geometry &g, const float
     {
         constexpr int kColumns = kPlaneThreads * kPlaneRun;
         const dim3 grid((g.pitch + kColumns - 1) / kColumns, g.prow);
-        k_planes<<<grid, kPlaneThreads, 0, stream>>>(rgbi, g, lut, stages, p, aux, hs, hwa, hwr,
-                                                     plane, err);
+        const cudaError_t e = launch_chained(k_planes, grid, dim3(kPlaneThreads), 0, stream, 0,
+                                             rgbi, g, lut, stages, p, aux, hs, hwa, hwr, plane, err);
+        if (e != cudaSuccess) return e;
     }
     marks.mark(2, stream);
     // k_startup (the six hidden stages, 6 W sites: too few blocks to fill the
@@ -1189,15 +1193,15 @@ cudaError_t launch_analysis(const uint16_t *rgbi, const Geometry &g, const float
         e = cudaEventRecord(join, side);
         if (e != cudaSuccess) return e;
     }
-    if (tile_rows == 16) {
-        dim3 grid(g.tw, g.hp / 16);
-        k_stencil<16><<<grid, Tile<16>::THREADS, sizeof(StencilSmem<16>), stream>>>(
-            rgbi, g, lut, stages, p, cc, aux, hs, hwa, hwr, plane, cand, meta, err);
-    } else {
-        dim3 grid(g.tw, g.hp / 8);
-        k_stencil<8><<<grid, Tile<8>::THREADS, sizeof(StencilSmem<8>), stream>>>(
-            rgbi, g, lut, stages, p, cc, aux, hs, hwa, hwr, plane, cand, meta, err);
-    }
+    const cudaError_t launched =
+        tile_rows == 16
+            ? launch_chained(k_stencil<16>, dim3(g.tw, g.hp / 16), dim3(Tile<16>::THREADS),
+                             sizeof(StencilSmem<16>), stream, 0, rgbi, g, lut, stages, p, cc, aux,
+                             hs, hwa, hwr, plane, cand, meta, err)
+            : launch_chained(k_stencil<8>, dim3(g.tw, g.hp / 8), dim3(Tile<8>::THREADS),
+                             sizeof(StencilSmem<8>), stream, 0, rgbi, g, lut, stages, p, cc, aux,
+                             hs, hwa, hwr, plane, cand, meta, err);
+    if (launched != cudaSuccess) return launched;
     marks.mark(3, stream);
     if (side) {
         const cudaError_t e = cudaStreamWaitEvent(stream, join, 0);

@@ -186,6 +186,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1)
                     const float *__restrict__ lut, ProducerBuffers b) {
     using Smem = RowSmem<RB>;
     constexpr int kRows = Smem::kRows, kCells = Smem::kCells;
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem &S = *reinterpret_cast<Smem *>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -416,6 +417,7 @@ struct ScanSmem {
 __global__ void __launch_bounds__(kScanThreads)
     k_producer_scan(int h, int ne, float factor_b, ProducerBuffers b, fx_stage *stages,
                     float *rows_out, uint32_t *err) {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ScanSmem &S = *reinterpret_cast<ScanSmem *>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -559,8 +561,8 @@ static cudaError_t rows_init() {
 template <int RB>
 static void launch_rows(const uint16_t *rgbi, int h, int w, int aw, int cells, const float *lut,
                         const ProducerBuffers &b, cudaStream_t stream) {
-    k_producer_rows<RB><<<(h + RB * 8 - 1) / (RB * 8), kRowWarps * 32, sizeof(RowSmem<RB>),
-                          stream>>>(rgbi, h, w, aw, cells, lut, b);
+    launch_chained(k_producer_rows<RB>, dim3((h + RB * 8 - 1) / (RB * 8)), dim3(kRowWarps * 32),
+                   sizeof(RowSmem<RB>), stream, 0, rgbi, h, w, aw, cells, lut, b);
 }
 
 static int g_producer_sms = 148;
@@ -623,7 +625,7 @@ cudaError_t launch_producer(const uint16_t *rgbi, int h, int w, const float *lut
     }
     // the scan is one block: given priority, it starts as soon as the row
     // sums are done even when other frames' kernels have blocks pending
-    cudaError_t e = launch_prio(k_producer_scan, dim3(1), dim3(kScanThreads), sizeof(ScanSmem),
+    cudaError_t e = launch_chained(k_producer_scan, dim3(1), dim3(kScanThreads), sizeof(ScanSmem),
                                 stream, priority, h, ne, 1.0f, b, stages, rows_out, err);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();

@@ -841,6 +841,7 @@ __global__ void __launch_bounds__(kWinThreads, kWinBlocksPerSM)
            uint32_t launches, uint32_t per_wave, uint32_t t0, uint32_t serial_below, double sigmas, uint32_t *err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_last;
+    grid_dependency();
     if (pass_stopped(err)) return;
     const uint32_t n = (uint32_t)min((int64_t)*n_ptr, capacity);
     if (n < serial_below) return;  // the chain is walked serially instead
@@ -904,6 +905,7 @@ __global__ void __launch_bounds__(32)
              const uint32_t *__restrict__ err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     RewalkSmem &S = *reinterpret_cast<RewalkSmem *>(smem_raw);
+    grid_dependency();
     if (pass_stopped(err)) return;
     const int lane = threadIdx.x;
     const uint32_t n = (uint32_t)min((int64_t)*n_ptr, capacity);
@@ -1117,13 +1119,13 @@ cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
         places = (int64_t)launches * (reach / 2 + per_wave + 2);
         for (uint32_t w = 0; w < launches; ++w) {
             const cudaError_t e =
-                launch_prio(k_wave, dim3(blocks), dim3(kWinThreads), kWaveSmem, stream, priority,
+                launch_chained(k_wave, dim3(blocks), dim3(kWinThreads), kWaveSmem, stream, priority,
                             B, n_ptr, capacity, w, launches, (uint32_t)per_wave, t0, serial_below,
                             window_sigmas, const_cast<uint32_t *>(err));
             if (e != cudaSuccess) return e;
         }
     }
-    cudaError_t e = launch_prio(k_rewalk, dim3((unsigned)((places + 31) / 32)), dim3(32),
+    cudaError_t e = launch_chained(k_rewalk, dim3((unsigned)((places + 31) / 32)), dim3(32),
                                 sizeof(RewalkSmem), stream, priority, B, n_ptr, capacity,
                                 (uint32_t)per_wave, t0, extra, serial_below, err);
     if (e != cudaSuccess) return e;

@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(kSegWarps * 32)
     __shared__ uint32_t tile[kTile];
     __shared__ unsigned long long ws[kSegWarps];
     __shared__ bool s_last;
+    grid_dependency();
     if (pass_stopped(err)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t seg = (int64_t)blockIdx.x * kSegWarps + warp;
@@ -402,6 +403,7 @@ __global__ void __launch_bounds__(kCoefWarps * 32, kCoefBlocksPerSM)
     // listed channels: site in the unit | channel << 8 | fixed draws before it
     // in the segment << 10
     __shared__ uint32_t s_list[kCoefWarps][3 * kUnitSites];
+    grid_dependency();
     if (pass_stopped(err)) return;
     const int lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < 256; i += kCoefWarps * 32)
@@ -690,6 +692,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
     __shared__ uint2 s_list[kApplyWarps][kUnitSites];
     __shared__ unsigned long long s_sums[kApplyWarps][4];
     __shared__ bool s_last;
+    grid_dependency();
     if (pass_stopped(err)) return;  // cancelled: the output stays untouched
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < 256; i += kApplyWarps * 32) {
@@ -954,12 +957,12 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
     // leave idle
     const int pr = b.priority;
     const unsigned seg_blocks = (unsigned)((segs + kSegWarps - 1) / kSegWarps);
-    e = launch_prio(k_seg_sums, dim3(seg_blocks), dim3(kSegWarps * 32), 0, stream, pr, meta,
+    e = launch_chained(k_seg_sums, dim3(seg_blocks), dim3(kSegWarps * 32), 0, stream, pr, meta,
                     g.sites, segs, b.seg_raw, b.seg_base, b.seg_amb, ctr, err);
     if (e != cudaSuccess) return e;
     const uint32_t *n_amb = b.seg_amb + segs;
     const int64_t unit_blocks = (segs * (kSegment / kUnitSites) + kCoefWarps - 1) / kCoefWarps;
-    e = launch_prio(k_coef, dim3((unsigned)std::min<int64_t>(unit_blocks, g_coef_blocks)),
+    e = launch_chained(k_coef, dim3((unsigned)std::min<int64_t>(unit_blocks, g_coef_blocks)),
                     dim3(kCoefWarps * 32), 0, stream, pr, b.entries, b.second, b.capacity, meta,
                     g.sites, segs, b.seg_raw, b.seg_base, b.seg_amb, cand, g.w, rgbi, lut, p,
                     b.chunk_two, b.chunk_stat, ctr, err);
@@ -976,10 +979,12 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
     if (e != cudaSuccess) return e;
     const int64_t apply_blocks =
         (segs * (kSegment / kUnitSites) + 6 + kApplyWarps - 1) / kApplyWarps;
-    k_apply<<<(unsigned)std::min<int64_t>(apply_blocks, g_apply_blocks), kApplyWarps * 32, 0,
-              stream>>>(meta, cand, g.sites, g.w, rgbi, lut, high, low, ident, stages, p,
-                        b.seg_base, b.seg_amb, b.extra, s0 & kLcgMask, rgb_out, changed_out, ctr,
-                        reinterpret_cast<const WalkState *>(b.walk_zero), err, b.capacity);
+    e = launch_chained(k_apply, dim3((unsigned)std::min<int64_t>(apply_blocks, g_apply_blocks)),
+                       dim3(kApplyWarps * 32), 0, stream, 0, meta, cand, g.sites, g.w, rgbi, lut,
+                       high, low, ident, stages, p, b.seg_base, b.seg_amb, b.extra, s0 & kLcgMask,
+                       rgb_out, changed_out, ctr,
+                       reinterpret_cast<const WalkState *>(b.walk_zero), err, b.capacity);
+    if (e != cudaSuccess) return e;
     marks.mark(7, stream);
     return cudaGetLastError();
 }
