@@ -357,40 +357,53 @@ __device__ __forceinline__ void copy_intervals(const ChannelView &cv, CopySet &e
 // switch points anew took 300 and 500.  Five blocks per SM at 48 registers:
 // four at 60 registers measured 6% more, six (with spills) 5% more.
 constexpr int kCoefWarps = 8, kCoefBlocksPerSM = 5;
-constexpr int kUnitSites = 256;
+constexpr int kUnitSites = 256;  // most sites of a unit
 static_assert(kSegment == 1024 && kUnitSites == 32 * 8, "32 and 8 meta bytes per lane");
 
-// Meta bytes of a unit: this lane's 8 sites, and the packed sums (fixed << 16
-// | RNG-dependent) of the segment's sites before the unit on this lane.
+// Sites of a unit of k_coef and k_apply (template instances).  256 keep a
+// warp's lists dense; where 64 still give every resident warp at most one
+// unit, the frame is bound by one unit's latency and 64 are faster: a 256x256
+// frame's chain 29 -> 19 us and apply 24 -> 20.
+static int unit_sites(int64_t segments, int resident_warps) {
+    return segments * (kSegment / 64) <= resident_warps ? 64 : kUnitSites;
+}
+
+// Meta bytes of a unit of US sites: this lane's 8 sites (US / 8 lanes have
+// any), and the packed sums (fixed << 16 | RNG-dependent) of the segment's
+// sites before the unit on this lane.
 struct UnitMeta {
     uint32_t word[2];
     uint32_t ahead;
 };
+template <int US>
 __device__ __forceinline__ UnitMeta unit_meta(const uint8_t *__restrict__ meta, int64_t sites,
                                               int64_t seg, int part) {
     const int lane = threadIdx.x & 31;
-    const int64_t first = seg * kSegment + part * kUnitSites;
+    const int64_t first = seg * kSegment + part * US;
     const int64_t mine = first + lane * 8, far = seg * kSegment + lane * 32;
     UnitMeta u{{0u, 0u}, 0u};
-    if (first + kUnitSites <= sites) {
-        if (lane < part * (kUnitSites / 32)) {
+    if (first + US <= sites) {
+        if (lane < part * (US / 32)) {
             const uint4 *q = reinterpret_cast<const uint4 *>(meta + far);
             const uint4 a = q[0], b = q[1];
             u.ahead = packed_word(a.x) + packed_word(a.y) + packed_word(a.z) + packed_word(a.w) +
                       packed_word(b.x) + packed_word(b.y) + packed_word(b.z) + packed_word(b.w);
         }
-        const uint2 v = *reinterpret_cast<const uint2 *>(meta + mine);
-        u.word[0] = v.x;
-        u.word[1] = v.y;
+        if (lane < US / 8) {
+            const uint2 v = *reinterpret_cast<const uint2 *>(meta + mine);
+            u.word[0] = v.x;
+            u.word[1] = v.y;
+        }
     } else {  // the chain's last unit
-        if (lane < part * (kUnitSites / 32))
+        if (lane < part * (US / 32))
             for (int i = 0; i < 32; ++i) u.ahead += packed_word(meta[far + i]);
         for (int i = 0; i < 8; ++i)
-            if (mine + i < sites) u.word[i >> 2] |= (uint32_t)meta[mine + i] << (8 * (i & 3));
+            if (lane < US / 8 && mine + i < sites) u.word[i >> 2] |= (uint32_t)meta[mine + i] << (8 * (i & 3));
     }
     return u;
 }
 
+template <int US>
 __global__ void __launch_bounds__(kCoefWarps * 32, kCoefBlocksPerSM)
     k_coef(AmbEntry *__restrict__ entries, SecondInterval *__restrict__ second, int64_t capacity,
            const uint8_t *__restrict__ meta, int64_t sites, int64_t segs,
@@ -402,7 +415,7 @@ __global__ void __launch_bounds__(kCoefWarps * 32, kCoefBlocksPerSM)
     __shared__ Affine s_jump[2][128];
     // listed channels: site in the unit | channel << 8 | fixed draws before it
     // in the segment << 10
-    __shared__ uint32_t s_list[kCoefWarps][3 * kUnitSites];
+    __shared__ uint32_t s_list[kCoefWarps][3 * US];
     grid_dependency();
     if (pass_stopped(err)) return;
     const int lane = threadIdx.x & 31;
@@ -413,7 +426,8 @@ __global__ void __launch_bounds__(kCoefWarps * 32, kCoefBlocksPerSM)
     const DitherConst dc = dither_const(p);
     const int64_t su = 6 * (int64_t)w;
     const SegRaw v = seg_raw_view(raw, segs);
-    const int64_t units = segs * (kSegment / kUnitSites);
+    constexpr int kPerSegment = kSegment / US;
+    const int64_t units = segs * kPerSegment;
     // two units per ticket on large frames (the counter is one address)
     const int grab = units > 8 * (int64_t)gridDim.x * kCoefWarps ? 2 : 1;
     int64_t unit = 0;
@@ -425,11 +439,11 @@ __global__ void __launch_bounds__(kCoefWarps * 32, kCoefBlocksPerSM)
             left = grab;
         }
         if (unit >= units) break;
-        const int64_t seg = unit / (kSegment / kUnitSites);
-        const int part = (int)(unit % (kSegment / kUnitSites));
-        const int64_t first = seg * kSegment + part * kUnitSites;
+        const int64_t seg = unit / kPerSegment;
+        const int part = (int)(unit % kPerSegment);
+        const int64_t first = seg * kSegment + part * US;
         if (first >= sites) continue;
-        const UnitMeta u = unit_meta(meta, sites, seg, part);
+        const UnitMeta u = unit_meta<US>(meta, sites, seg, part);
         // the segment's prefix: its group's, plus the segments before it in
         // the group (fewer than eight, so the packed halves cannot carry);
         // its first unit writes it for the kernels after the walk
@@ -676,6 +690,7 @@ __device__ void apply_final(const uint32_t *seg_base, const uint32_t *seg_amb, i
         raise_error(err, FX_ERR_INTERNAL);
 }
 
+template <int US>
 __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
     k_apply(const uint8_t *__restrict__ meta, const double *__restrict__ cand, int64_t sites,
             int w, const uint16_t *__restrict__ rgbi, const float *__restrict__ lut,
@@ -689,7 +704,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
     __shared__ uint32_t hi[256], lo[256];  // emit factors
     // attempted sites: x = site in the segment | meta << 16, y = fixed draws
     // before it in the segment | RNG-dependent channels before it << 16
-    __shared__ uint2 s_list[kApplyWarps][kUnitSites];
+    __shared__ uint2 s_list[kApplyWarps][US];
     __shared__ unsigned long long s_sums[kApplyWarps][4];
     __shared__ bool s_last;
     grid_dependency();
@@ -707,7 +722,8 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
     uint2 *list = s_list[warp];
     unsigned long long att = 0, written = 0, changed = 0, draws_total = 0;
     bool ok = true;
-    const int64_t units = 6 + segs * (kSegment / kUnitSites);
+    constexpr int kPerSegment = kSegment / US;
+    const int64_t units = 6 + segs * kPerSegment;
     // two units per ticket on large frames (the ticket counter is one address),
     // one on small ones
     const int grab = units > 8 * (int64_t)gridDim.x * kApplyWarps ? 2 : 1;
@@ -741,14 +757,14 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
             }
             continue;
         }
-        const int64_t seg = (unit - 6) / (kSegment / kUnitSites);
-        const int part = (int)((unit - 6) % (kSegment / kUnitSites));
-        const int64_t first = seg * kSegment + part * kUnitSites;
+        const int64_t seg = (unit - 6) / kPerSegment;
+        const int part = (int)((unit - 6) % kPerSegment);
+        const int64_t first = seg * kSegment + part * US;
         if (first >= sites) continue;
         // the state at the segment's first draw
         const uint32_t seg_a = seg_amb[seg], seg_p = seg_base[seg];
         // ---- meta: the segment's sites before the unit, this lane's 8 sites ---
-        const UnitMeta um = unit_meta(meta, sites, seg, part);
+        const UnitMeta um = unit_meta<US>(meta, sites, seg, part);
         const uint32_t *m2 = um.word;
         const int64_t mine = first + lane * 8;
         uint32_t sum = 0;
@@ -782,7 +798,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
         for (int i = 0; i < 8; ++i) {
             const uint32_t m = (m2[i >> 2] >> (8 * (i & 3))) & 0xFFu;
             if ((bits >> i) & 1u) {
-                list[slot] = make_uint2((uint32_t)(part * kUnitSites + lane * 8 + i) | (m << 16),
+                list[slot] = make_uint2((uint32_t)(part * US + lane * 8 + i) | (m << 16),
                                         (run >> 16) | (run << 16));
                 ++slot;
             }
@@ -790,7 +806,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
         }
         // ---- sites that were not attempted: identity emits -------------------
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
+        for (int r = 0; r < US / 32; ++r) {
             const int64_t site = first + 32 * r + lane;
             // the bits of site's lane say whether it was attempted
             const uint32_t b = __shfl_sync(0xFFFFFFFFu, bits, 4 * r + (lane >> 3));
@@ -961,8 +977,11 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
                     g.sites, segs, b.seg_raw, b.seg_base, b.seg_amb, ctr, err);
     if (e != cudaSuccess) return e;
     const uint32_t *n_amb = b.seg_amb + segs;
-    const int64_t unit_blocks = (segs * (kSegment / kUnitSites) + kCoefWarps - 1) / kCoefWarps;
-    e = launch_chained(k_coef, dim3((unsigned)std::min<int64_t>(unit_blocks, g_coef_blocks)),
+    const int us = unit_sites(segs, std::min(g_coef_blocks * kCoefWarps,
+                                             g_apply_blocks * kApplyWarps));
+    const int64_t unit_blocks = (segs * (kSegment / us) + kCoefWarps - 1) / kCoefWarps;
+    e = launch_chained(us == 64 ? k_coef<64> : k_coef<kUnitSites>,
+                    dim3((unsigned)std::min<int64_t>(unit_blocks, g_coef_blocks)),
                     dim3(kCoefWarps * 32), 0, stream, pr, b.entries, b.second, b.capacity, meta,
                     g.sites, segs, b.seg_raw, b.seg_base, b.seg_amb, cand, g.w, rgbi, lut, p,
                     b.chunk_two, b.chunk_stat, ctr, err);
@@ -978,8 +997,9 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
     e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
     const int64_t apply_blocks =
-        (segs * (kSegment / kUnitSites) + 6 + kApplyWarps - 1) / kApplyWarps;
-    e = launch_chained(k_apply, dim3((unsigned)std::min<int64_t>(apply_blocks, g_apply_blocks)),
+        (segs * (kSegment / us) + 6 + kApplyWarps - 1) / kApplyWarps;
+    e = launch_chained(us == 64 ? k_apply<64> : k_apply<kUnitSites>,
+                       dim3((unsigned)std::min<int64_t>(apply_blocks, g_apply_blocks)),
                        dim3(kApplyWarps * 32), 0, stream, 0, meta, cand, g.sites, g.w, rgbi, lut,
                        high, low, ident, stages, p, b.seg_base, b.seg_amb, b.extra, s0 & kLcgMask,
                        rgb_out, changed_out, ctr,

@@ -4,7 +4,8 @@ The profile's amplitudes keep every delta inside the dither bounds, so the
 floor test alone decides.  With larger amplitudes and tighter bounds the delta
 leaves them on some states and a channel's copy set gets up to three
 breakpoints and two intervals; sizes around the units of 256 sites and the
-segments of 1024 that list the channels (6 w + h w sites).
+segments of 1024 that list the channels (6 w + h w sites; units of 64 on the
+smaller frames).
 """
 
 from __future__ import annotations
@@ -22,7 +23,8 @@ pytestmark = pytest.mark.gpu
 BOUNDS = ox.dither_bounds(ox.tables()[0])
 
 
-@pytest.mark.parametrize("h, w", [(16, 16), (74, 16), (58, 16), (26, 40), (57, 65), (130, 211)])
+@pytest.mark.parametrize("h, w", [(16, 16), (74, 16), (58, 16), (26, 40), (57, 65), (130, 211),
+                                  (620, 651)])
 @pytest.mark.parametrize("scales, margin", [
     ((0.015, 0.025, 0.015), 0.0), ((0.4, 0.9, 2.0), 0.0), ((30.0, 4.0, 300.0), 0.0),
     ((0.02, 1.5, 8.0), 0.05), ((1e-7, 1e-12, 1e5), 0.02)])
