@@ -634,12 +634,13 @@ __device__ __noinline__ BandRanges irregular_ranges(const StencilSmem<TH> &S,
     return band_ranges(feats, records);
 }
 
-// Bound: instruction issue (64 registers and 57 KB per block keep 32 warps on
-// an SM; the conversions' pipe has room: widening the taps with integer
-// multiplies halved its use and saved nothing).  Native frame 1.24 ms, at 5%
-// coverage 1.13.  With four widened features per record and pixel, a fresh
-// row and column division per staged vector and listed record, and the
-// dither constants' division per pixel it took 1.375 and 1.253.
+// Bound: instruction issue (36 warp instructions per pixel, 58% of the slots;
+// 64 registers and 57 KB per block keep 32 warps on an SM) with the pipe of the
+// binary32/64 conversions at 60%; widening the taps with integer multiplies
+// took that to 30% and saved nothing.  Native frame 1.23 ms, at 5% coverage
+// 1.12.  With four widened features per record and pixel, a fresh row and
+// column division per staged vector and listed record, and the dither
+// constants' division per pixel it took 1.375 and 1.253.
 template <int TH>
 __global__ void __launch_bounds__(Tile<TH>::THREADS, Tile<TH>::BLOCKS_PER_SM)
     k_stencil(const uint16_t *__restrict__ rgbi, Geometry g, const float *__restrict__ lut,

@@ -343,7 +343,7 @@ __device__ __forceinline__ void copy_intervals(const ChannelView &cv, CopySet &e
 }
 
 // Copy test and state map of every RNG-dependent channel.  Every warp takes
-// units of 256 sites, a quarter of a chain segment: the segment's meta bytes
+// units of 256 sites, a quarter of a chain segment (or 64, see unit_sites): the segment's meta bytes
 // give the chain offsets of the unit's sites, the channels are listed in the
 // warp's shared memory (at most three per site), and the list is processed
 // densely, one channel per lane, written to consecutive entries.  One
@@ -636,8 +636,8 @@ cudaError_t writer_init() {
     return cudaMemcpyToSymbol(g_short, brief, sizeof(brief));
 }
 
-// Every warp takes units of 256 sites, a quarter of a chain segment, with no
-// block barrier:
+// Every warp takes units of 256 sites, a quarter of a chain segment (64 on
+// small frames: unit_sites), with no block barrier:
 //   * the segment's meta bytes give the chain offsets before the unit and of
 //     its sites, and the attempted sites are listed in the warp's shared
 //     memory;

@@ -86,7 +86,7 @@ def reserve_frames(ctx: _lib.Context, max_height: int, max_width: int) -> None:
 
 
 def set_walk_wave(ctx: _lib.Context, segments: int) -> None:
-    """Segments per speculative walk wave (0: the default, three per SM)."""
+    """Segments per speculative walk wave (0: the default, four per SM)."""
 
     with ctx.lock:
         _check(ctx, _lib.load().fx_set_walk_wave(ctx.handle, int(segments)))

@@ -206,13 +206,13 @@ FX_API int fx_set_slots(fx_context *ctx, int32_t slots);
 /* 1 (default): the speculative parallel walk; 0: one warp walks the whole
  * chain (leaves the rest of the GPU to other frames' kernels). */
 FX_API int fx_set_parallel_walk(fx_context *ctx, int enable);
-/* Segments of 4096 RNG-dependent channels walked speculatively per wave
- * (0, the default: three per SM).  Fewer segments per wave mean narrower
+/* Segments of RNG-dependent channels walked speculatively per wave (0, the
+ * default: four per SM).  Fewer segments per wave mean narrower
  * candidate windows (less total work, for throughput when several frames
  * are in flight) and more waves (longer latency for one frame). */
 FX_API int fx_set_walk_wave(fx_context *ctx, int32_t segments);
 /* 1 (default): the latency-bound kernels of a pass (the producer's scan, the
- * writer's prefix, interval and jump kernels, the walk) are launched at the
+ * writer's prefix and interval kernels, the walk) are launched at the
  * device's greatest execution priority, so that with several frames in
  * flight their blocks are dispatched ahead of other frames' stencil and
  * emit blocks; 0: every launch at the default priority.  No effect on
