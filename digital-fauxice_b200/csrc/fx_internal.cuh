@@ -57,14 +57,6 @@ struct Geometry {
 // Per-site meta byte: bit 7 attempted, bits 2c..2c+1 draw code of channel c
 // (0: no draw, 1: one draw, 2: two draws, 3: RNG-dependent: one or two).
 __host__ __device__ __forceinline__ int meta_code(uint8_t m, int c) { return (m >> (2 * c)) & 3; }
-__host__ __device__ __forceinline__ int meta_base(uint8_t m) {
-    int b = 0;
-    for (int c = 0; c < 3; ++c) {
-        const int k = meta_code(m, c);
-        b += (k == 3) ? 1 : k;
-    }
-    return b;
-}
 __host__ __device__ __forceinline__ int meta_amb(uint8_t m) {
     int a = 0;
     for (int c = 0; c < 3; ++c) a += meta_code(m, c) == 3;

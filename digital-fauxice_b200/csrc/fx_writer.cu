@@ -66,10 +66,6 @@ __device__ __forceinline__ uint32_t packed_word(uint32_t w) {
     return (base << 16) | amb;
 }
 
-__device__ __forceinline__ uint32_t packed_site(uint8_t m) {
-    return ((uint32_t)meta_base(m) << 16) | (uint32_t)meta_amb(m);
-}
-
 constexpr int kSegWarps = 8;  // segments per block of the chain kernels (one per warp)
 
 static_assert(kSegWarps == kSegGroup, "a k_seg_sums block sums one group of segments");
