@@ -62,7 +62,7 @@ struct Arena {
     int64_t amb_capacity = 0;
 };
 
-static int g_per_wave = 591;  // window blocks per wave: walk_per_wave(SM count)
+static int g_per_wave = 592;  // most segments per wave: walk_per_wave(SM count)
 
 static size_t arena_layout(const Geometry &g, int64_t amb_cap, Arena *a) {
     size_t off = 0;
@@ -296,6 +296,12 @@ static int check_frame(fx_context *ctx, const fx_params *p, int h, int w) {
     return FX_OK;
 }
 
+// Segments per wave of a pass with `requested` (0: as many as fit the SMs);
+// the walk scratch holds any of them.
+static int pass_wave(int requested) {
+    return requested > 0 && requested < g_per_wave ? requested : g_per_wave;
+}
+
 // Enqueue the whole pass for one frame whose input already sits in
 // s.arena.rgbi (or `d_in`).  Outputs land in the arena (or `d_out`).
 // `cancellable` passes (fx_submit, fx_submit_device) get stage gates that
@@ -335,11 +341,9 @@ static int enqueue_pass(fx_context *ctx, Slot &s, const Geometry &g, const fx_pa
     FX_CUDA(ctx, launch_analysis(d_in, g, ctx->lut, a.stages, p, a.aux, a.hs, a.hwa, a.hwr,
                                  (int64_t)g.prow * g.pitch, a.cand, a.meta, a.err, st, marks,
                                  ctx->stencil_rows, s.side, s.fork, s.join));
-    // the walk scratch is sized for g_per_wave; a narrower wave uses part of it
-    const int wave = (ctx->walk_wave > 0 && ctx->walk_wave < g_per_wave) ? ctx->walk_wave
-                                                                         : g_per_wave;
+    const int wave = pass_wave(ctx->walk_wave);
     WriterBuffers wb{a.seg_base, a.seg_amb, a.seg_raw, a.entries, a.second, a.extra, a.counters,
-                     a.amb_capacity, a.walk, a.walk_zero, wave, ctx->parallel_walk, ctx->walk_sigmas, cancel,
+                     a.amb_capacity, a.walk, a.walk_zero, g_per_wave, wave, ctx->parallel_walk, ctx->walk_sigmas, cancel,
                      a.chunk_two, a.chunk_stat, ctx->use_priority ? ctx->top_priority : 0};
     FX_CUDA(ctx, launch_writer(g, a.meta, a.cand, d_in, ctx->lut, ctx->high, ctx->low, ctx->ident, a.stages,
                                p, rng, wb, d_out, d_changed, a.err, st, marks));
@@ -912,6 +916,14 @@ FX_API int fx_set_walk_wave(fx_context *ctx, int32_t segments) {
     if (!ctx || segments < 0) return FX_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lock(ctx->mu);
     ctx->walk_wave = segments;
+    return FX_OK;
+}
+
+FX_API int fx_walk_segments(int64_t channels, int32_t segments, int64_t *used,
+                            int64_t *reserved) {
+    if (channels < 1 || segments < 0 || !used || !reserved) return FX_ERR_INVALID_ARGUMENT;
+    *used = walk_segments(channels, pass_wave(segments));
+    *reserved = walk_segments_reserved(channels, g_per_wave);
     return FX_OK;
 }
 

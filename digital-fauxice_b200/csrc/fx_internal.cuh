@@ -257,9 +257,10 @@ struct WriterBuffers {
     ExtraWord *extra;              // extra_words(capacity)
     void *counters;                // DevCounters
     int64_t capacity;
-    void *walk_scratch;            // walk_scratch_bytes(capacity, per_wave)
+    void *walk_scratch;            // walk_scratch_bytes(capacity, widest_wave)
     void *walk_zero;               // walk_zero_bytes(capacity), cleared for the pass
-    int per_wave;                  // window blocks per wave (walk_per_wave of the SM count)
+    int widest_wave;               // most segments per wave (walk_per_wave of the SM count)
+    int per_wave;                  // segments per wave, at most widest_wave
     bool parallel_walk;
     double window_sigmas;          // walk window half-width in standard deviations
     const uint32_t *cancel;        // host-mapped cancel word read by the stage gates, or null
@@ -334,7 +335,9 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
                           const Marks &marks);
 size_t dev_counters_bytes();
 cudaError_t walk_init();
-size_t walk_scratch_bytes(int64_t capacity, int per_wave);
+size_t walk_scratch_bytes(int64_t capacity, int widest);
+int64_t walk_segments(int64_t capacity, int per_wave);
+int64_t walk_segments_reserved(int64_t capacity, int widest);
 size_t walk_zero_bytes(int64_t capacity);
 int walk_per_wave(int sms);
 __host__ __device__ inline size_t walk_chunks(int64_t capacity) {
@@ -342,7 +345,7 @@ __host__ __device__ inline size_t walk_chunks(int64_t capacity) {
 }
 cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
                         const uint32_t *n_ptr, int64_t capacity, uint32_t s0, void *scratch,
-                        void *zero, int per_wave,
+                        void *zero, int widest, int per_wave,
                         bool parallel, double window_sigmas, const uint8_t *chunk_two,
                         const ChunkStat *chunk_stat,
                         ExtraWord *extra, const uint32_t *err, cudaStream_t stream,

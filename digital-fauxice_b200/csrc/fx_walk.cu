@@ -227,7 +227,7 @@ struct WalkBuffers {
     const ChunkStat *chunk_stat;
     WalkState *st;
     uint2 *wave;           // per wave: first chunk, exact E there (one more: its end)
-    SegWindow *windows;    // per segment of the chain
+    SegWindow *windows;    // per segment of every wave
     uint32_t *e_in;        // per segment: exact entry count
     SegList *lists;        // per segment of a wave
     uint32_t *path;        // per segment of a wave: kListMax exit counts, one per survivor
@@ -1030,12 +1030,32 @@ size_t walk_zero_bytes(int64_t capacity) {
            (walk_chunks(capacity) / kWalkAvgMax + 2 + kSpareWaves) * sizeof(uint2);
 }
 
-// Device layout of the walk scratch for lists of up to `capacity` channels;
-// returns its size.
-static size_t walk_layout(void *scratch, void *zero, int64_t capacity, int per_wave,
+static uint32_t walk_channels(int64_t capacity) {
+    return (uint32_t)std::min<int64_t>(capacity, 0xFFFFFF00ll);
+}
+
+// Segment records (window, entry count) of a walk in waves of `per_wave`.
+int64_t walk_segments(int64_t capacity, int per_wave) {
+    const WalkPlan plan = walk_plan(walk_channels(capacity), (uint32_t)per_wave);
+    return (int64_t)wave_launches(plan) * per_wave;
+}
+
+// Segment records that hold a walk in waves of any number of segments up to
+// `widest`: c chunks in waves of s segments are ceil(c / (kWalkAvgMax s))
+// waves (at least one) and kSpareWaves more, so at most c / kWalkAvgMax +
+// (1 + kSpareWaves) s records.  A narrower wave can need more records than the
+// widest: one of 591 segments ramps from 2364 chunks on, with spare waves, one
+// of 592 from 2368 on.
+int64_t walk_segments_reserved(int64_t capacity, int widest) {
+    const WalkPlan plan = walk_plan(walk_channels(capacity), (uint32_t)widest);
+    return plan.chunks / kWalkAvgMax + (int64_t)(1u + kSpareWaves) * widest;
+}
+
+// Device layout of the walk scratch for lists of up to `capacity` channels and
+// waves of up to `widest` segments; returns its size.
+static size_t walk_layout(void *scratch, void *zero, int64_t capacity, int widest,
                           WalkBuffers *B) {
-    const uint32_t n = (uint32_t)std::min<int64_t>(capacity, 0xFFFFFF00ll);
-    const size_t waves = wave_launches(walk_plan(n, (uint32_t)per_wave));
+    const size_t segments = (size_t)walk_segments_reserved(capacity, widest);
     char *base = reinterpret_cast<char *>(scratch);
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -1044,10 +1064,10 @@ static size_t walk_layout(void *scratch, void *zero, int64_t capacity, int per_w
         return r;
     };
     WalkBuffers b{};
-    b.windows = (SegWindow *)take(waves * per_wave * sizeof(SegWindow));
-    b.e_in = (uint32_t *)take(waves * per_wave * sizeof(uint32_t));
-    b.lists = (SegList *)take((size_t)per_wave * sizeof(SegList));
-    b.path = (uint32_t *)take((size_t)per_wave * kListMax * sizeof(uint32_t));
+    b.windows = (SegWindow *)take(segments * sizeof(SegWindow));
+    b.e_in = (uint32_t *)take(segments * sizeof(uint32_t));
+    b.lists = (SegList *)take((size_t)widest * sizeof(SegList));
+    b.path = (uint32_t *)take((size_t)widest * kListMax * sizeof(uint32_t));
     b.kept = (KeptHead *)take(walk_chunks(capacity) * sizeof(KeptHead));
     const int64_t pool = kept_pool(capacity);
     b.kept_state = (uint32_t *)take((size_t)pool * sizeof(uint32_t));
@@ -1061,8 +1081,8 @@ static size_t walk_layout(void *scratch, void *zero, int64_t capacity, int per_w
     return off;
 }
 
-size_t walk_scratch_bytes(int64_t capacity, int per_wave) {
-    return walk_layout(nullptr, nullptr, capacity, per_wave, nullptr);
+size_t walk_scratch_bytes(int64_t capacity, int widest) {
+    return walk_layout(nullptr, nullptr, capacity, widest, nullptr);
 }
 
 // Segments per wave: the blocks that fit the SMs, so every block of a wave is
@@ -1096,11 +1116,11 @@ cudaError_t walk_init() {
 // lane instead of the speculative windows.
 cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
                         const uint32_t *n_ptr, int64_t capacity, uint32_t s0, void *scratch,
-                        void *zero, int per_wave, bool parallel, double window_sigmas,
+                        void *zero, int widest, int per_wave, bool parallel, double window_sigmas,
                         const uint8_t *chunk_two, const ChunkStat *chunk_stat, ExtraWord *extra,
                         const uint32_t *err, cudaStream_t stream, int priority) {
     WalkBuffers B;
-    walk_layout(scratch, zero, capacity, per_wave, &B);
+    walk_layout(scratch, zero, capacity, widest, &B);
     B.entries = entries;
     B.second = second;
     B.chunk_two = chunk_two;
@@ -1109,8 +1129,7 @@ cudaError_t launch_walk(const AmbEntry *entries, const SecondInterval *second,
     const uint32_t serial_below = parallel ? kSerialBelow : 0xFFFFFFFFu;
     int64_t places = 1;
     if (parallel) {
-        const uint32_t cap = (uint32_t)std::min<int64_t>(capacity, 0xFFFFFF00ll);
-        const WalkPlan plan = walk_plan(cap, (uint32_t)per_wave);
+        const WalkPlan plan = walk_plan(walk_channels(capacity), (uint32_t)per_wave);
         const uint32_t blocks = std::min((uint32_t)per_wave, plan.chunks);
         const uint32_t launches = wave_launches(plan);
         // half a wave's chunks (a shorter chain may have longer waves than the

@@ -986,7 +986,7 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
     e = launch_gate(b.cancel, err, stream);
     if (e != cudaSuccess) return e;
     e = launch_walk(b.entries, b.second, n_amb, b.capacity, s0, b.walk_scratch, b.walk_zero,
-                    b.per_wave, b.parallel_walk, b.window_sigmas, b.chunk_two, b.chunk_stat,
+                    b.widest_wave, b.per_wave, b.parallel_walk, b.window_sigmas, b.chunk_two, b.chunk_stat,
                     b.extra, err, stream, pr);
     if (e != cudaSuccess) return e;
     marks.mark(6, stream);

@@ -211,6 +211,11 @@ FX_API int fx_set_parallel_walk(fx_context *ctx, int enable);
  * candidate windows (less total work, for throughput when several frames
  * are in flight) and more waves (longer latency for one frame). */
 FX_API int fx_set_walk_wave(fx_context *ctx, int32_t segments);
+/* Host only: the segment records a walk over a list of `channels` uses with
+ * that wave setting, and the records its scratch holds (no reference
+ * counterpart). */
+FX_API int fx_walk_segments(int64_t channels, int32_t segments, int64_t *used,
+                            int64_t *reserved);
 /* 1 (default): the latency-bound kernels of a pass (the producer's scan, the
  * writer's prefix and interval kernels, the walk) are launched at the
  * device's greatest execution priority, so that with several frames in

@@ -46,3 +46,25 @@ def test_every_layout_draws_as_the_oracle(h, w, spec, wave, sigmas):
     assert np.array_equal(result.output_rgb16, expected.output_rgb16)
     assert result.replay.public_rng_advances == expected.public_rng_advances
     assert result.replay.final_rng_state == expected.final_rng_state
+
+
+# lists of 605,000 channels: waves just below the widest take more segment records than
+# the widest; windows of 16 sigma keep more survivors than the pool of kept lists holds,
+# and windows of 0 sigma end wave after wave early
+@pytest.mark.parametrize("wave, sigmas", [(588, 4.5), (591, 4.5), (591, 16.0), (0, 16.0),
+                                          (300, 0.0), (591, 0.0)])
+def test_waves_near_the_widest_draw_as_the_oracle(wave, sigmas):
+    job, expected = _case(1094, 1100, "native")
+    ctx, lib = engine.context(), _lib.load()
+    assert lib.fx_set_list_capacity(ctx.handle, 605000) == 0
+    assert lib.fx_set_walk_wave(ctx.handle, wave) == 0
+    assert lib.fx_set_walk_window(ctx.handle, sigmas) == 0
+    try:
+        result = process_b200(job)
+    finally:
+        assert lib.fx_set_list_capacity(ctx.handle, 0) == 0
+        assert lib.fx_set_walk_wave(ctx.handle, 0) == 0
+        assert lib.fx_set_walk_window(ctx.handle, 4.5) == 0
+    assert np.array_equal(result.output_rgb16, expected.output_rgb16)
+    assert result.replay.public_rng_advances == expected.public_rng_advances
+    assert result.replay.final_rng_state == expected.final_rng_state
