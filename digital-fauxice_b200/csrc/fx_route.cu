@@ -26,6 +26,8 @@
 //   k_pairs        (label, label) pairs of two label planes, emitted only
 //                  where a pixel starts a new pair locally (the host removes
 //                  the remaining duplicates).
+#include <utility>
+
 #include "fx_internal.cuh"
 
 namespace fx {
@@ -360,7 +362,8 @@ constexpr int32_t kDistInf = 0x3FFFFFFF;
 // with k below the best so far can lower it; the row distances come from the
 // 64 bits to either side of the pixel.  A block covers 16 rows x 256 columns
 // with 64 pixels of halo in shared memory (7 KB); a tile without a set
-// pixel only writes zeros.  Pixels outside the frame are no background.  A
+// pixel only writes zeros.  Tiles are numbered along x: a tall mask has more
+// rows of them than the 65,535 blocks of the other axes.  Pixels outside the frame are no background.  A
 // deeper pixel gets kDistInf, from which the relaxation finishes it.
 // (Relaxing every tile from scratch took four launches of 500 us on a native
 // frame; this takes one of 140 us after 35 us of packing, 39 instead of 80 us on
@@ -374,7 +377,8 @@ __global__ void __launch_bounds__(kRouteThreads)
     constexpr int kRows = kNearRows + 2 * 64, kCols = kNearWords + 4;
     __shared__ uint32_t t[kRows][kCols + 1];
     const int wpr = words_per_row(w);
-    const int y0 = blockIdx.y * kNearRows, w0 = blockIdx.x * kNearWords;
+    const unsigned across = (wpr + kNearWords - 1) / kNearWords;
+    const int y0 = blockIdx.x / across * kNearRows, w0 = blockIdx.x % across * kNearWords;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool any = false;
     for (int k = threadIdx.x; k < kRows * kCols; k += kRouteThreads) {
@@ -430,7 +434,9 @@ __global__ void __launch_bounds__(kRouteThreads)
     k_dist_relax(const int32_t *__restrict__ in, int32_t *__restrict__ out, int h, int w,
                  uint32_t *changed) {
     __shared__ int32_t t[2][kDistSide][kDistSide];
-    const int y0 = blockIdx.y * kDistTile - kDistHalo, x0 = blockIdx.x * kDistTile - kDistHalo;
+    const unsigned across = (unsigned)(((int64_t)w + kDistTile - 1) / kDistTile);
+    const int y0 = blockIdx.x / across * kDistTile - kDistHalo;
+    const int x0 = blockIdx.x % across * kDistTile - kDistHalo;
     for (int k = threadIdx.x; k < kDistSide * kDistSide; k += blockDim.x) {
         const int r = k / kDistSide, c = k % kDistSide;
         const int y = y0 + r, x = x0 + c;
@@ -677,6 +683,30 @@ static unsigned grid_for(int64_t n) {
 
 using namespace fx;
 
+// Launch kRouteThreads (or `threads`) a block; false when the launch is refused.
+template <typename... KArgs, typename... Args>
+static bool launch(void (*kernel)(KArgs...), dim3 grid, cudaStream_t stream, int threads,
+                   Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    if (cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...) == cudaSuccess) return true;
+    cudaGetLastError();  // reported by the caller's status
+    return false;
+}
+
+// Tiles of rows x cols pixels that cover h x w, as a one-dimensional grid.
+static unsigned tiles_of(int64_t h, int64_t w, int rows, int cols) {
+    return (unsigned)((h + rows - 1) / rows * ((w + cols - 1) / cols));
+}
+
+// Copies a word back and waits for the stream.
+static bool fetch(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream) == cudaSuccess &&
+           cudaStreamSynchronize(stream) == cudaSuccess;
+}
+
 // Blocks of a grid-stride kernel with one warp per four 32-pixel words.
 static unsigned grid_for_words(int64_t words) {
     const int64_t b = (words + kRouteThreads / 8 - 1) / (kRouteThreads / 8);
@@ -698,19 +728,20 @@ FX_API int fx_label8(const uint8_t *d_mask, int32_t h, int32_t w, int32_t *d_lab
     const int64_t nblocks = (words + kRouteThreads - 1) / kRouteThreads;
     uint32_t *bits = reinterpret_cast<uint32_t *>(d_labels);
     if (cudaMemsetAsync(d_err, 0, sizeof(uint32_t), st) != cudaSuccess) return FX_ERR_CUDA;
-    k_pack<<<grid_for_words(words), kRouteThreads, 0, st>>>(d_mask, h, w, bits, d_forest);
-    k_ccl_union<<<grid_for(words), kRouteThreads, 0, st>>>(bits, h, w, d_forest, d_err);
-    k_ccl_flatten<<<(unsigned)nblocks, kRouteThreads, 0, st>>>(bits, h, w, d_forest,
-                                                              d_block_scratch, d_err);
-    k_ccl_scan<<<1, 1024, 0, st>>>(d_block_scratch, nblocks);
-    k_ccl_number<<<(unsigned)nblocks, kRouteThreads, 0, st>>>(bits, h, w, d_forest,
-                                                             d_block_scratch);
-    k_ccl_labels<<<grid_for_words(words), kRouteThreads, 0, st>>>(d_mask, d_forest, h, w,
-                                                                  d_labels);
+    const unsigned nb = (unsigned)nblocks;
     uint32_t total = 0, err = 0;
-    cudaMemcpyAsync(&total, d_block_scratch + nblocks, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&err, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return FX_ERR_CUDA;
+    if (!launch(k_pack, grid_for_words(words), st, kRouteThreads, d_mask, h, w, bits, d_forest) ||
+        !launch(k_ccl_union, grid_for(words), st, kRouteThreads, bits, h, w, d_forest, d_err) ||
+        !launch(k_ccl_flatten, nb, st, kRouteThreads, bits, h, w, d_forest, d_block_scratch,
+                d_err) ||
+        !launch(k_ccl_scan, 1, st, 1024, d_block_scratch, nblocks) ||
+        !launch(k_ccl_number, nb, st, kRouteThreads, bits, h, w, d_forest, d_block_scratch) ||
+        !launch(k_ccl_labels, grid_for_words(words), st, kRouteThreads, d_mask, d_forest, h, w,
+                d_labels) ||
+        cudaMemcpyAsync(&total, d_block_scratch + nblocks, sizeof(uint32_t),
+                        cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        !fetch(&err, d_err, sizeof(uint32_t), st))
+        return FX_ERR_CUDA;
     if (err) return FX_ERR_INTERNAL;
     *count = total;
     return FX_OK;
@@ -726,13 +757,14 @@ FX_API int fx_chessboard_distance(const uint8_t *d_mask, int32_t h, int32_t w, i
     const int wpr = words_per_row(w);
     uint32_t changed = 0;
     if (cudaMemsetAsync(d_flag, 0, sizeof(uint32_t), st) != cudaSuccess) return FX_ERR_CUDA;
-    k_pack<<<grid_for_words((int64_t)h * wpr), kRouteThreads, 0, st>>>(d_mask, h, w, bits, nullptr);
-    k_dist_near<<<dim3((wpr + kNearWords - 1) / kNearWords, (h + kNearRows - 1) / kNearRows),
-                  kRouteThreads, 0, st>>>(bits, h, w, d_dist, d_flag);
-    cudaMemcpyAsync(&changed, d_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return FX_ERR_CUDA;
+    if (!launch(k_pack, grid_for_words((int64_t)h * wpr), st, kRouteThreads, d_mask, h, w, bits,
+                static_cast<int32_t *>(nullptr)) ||
+        !launch(k_dist_near, tiles_of(h, wpr, kNearRows, kNearWords), st, kRouteThreads, bits, h,
+                w, d_dist, d_flag) ||
+        !fetch(&changed, d_flag, sizeof(uint32_t), st))
+        return FX_ERR_CUDA;
     if (!changed) return FX_OK;
-    const dim3 grid((w + kDistTile - 1) / kDistTile, (h + kDistTile - 1) / kDistTile);
+    const unsigned grid = tiles_of(h, w, kDistTile, kDistTile);
     int32_t *a = d_dist, *b = d_work;
     // every launch moves each front by up to kDistHalo pixels; the distance
     // of any pixel is below max(h, w), which bounds the launches
@@ -740,9 +772,9 @@ FX_API int fx_chessboard_distance(const uint8_t *d_mask, int32_t h, int32_t w, i
     for (int64_t it = 0; it < limit && changed; ++it) {
         changed = 0;
         if (cudaMemsetAsync(d_flag, 0, sizeof(uint32_t), st) != cudaSuccess) return FX_ERR_CUDA;
-        k_dist_relax<<<grid, kRouteThreads, 0, st>>>(a, b, h, w, d_flag);
-        cudaMemcpyAsync(&changed, d_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) return FX_ERR_CUDA;
+        if (!launch(k_dist_relax, grid, st, kRouteThreads, a, b, h, w, d_flag) ||
+            !fetch(&changed, d_flag, sizeof(uint32_t), st))
+            return FX_ERR_CUDA;
         int32_t *t = a;
         a = b;
         b = t;
@@ -761,9 +793,11 @@ FX_API int fx_label_stats(const int32_t *d_labels, const int32_t *d_plane, int32
     if (!d_labels || !d_area || !d_box || h < 1 || w < 1 || k < 0) return FX_ERR_INVALID_ARGUMENT;
     if (k == 0) return FX_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    k_stats_init<<<grid_for(k), kRouteThreads, 0, st>>>(k, d_area, d_box, d_plane ? d_vmax : nullptr);
-    k_stats<<<grid_for_words((int64_t)h * words_per_row(w)), kRouteThreads, 0, st>>>(
-        d_labels, d_plane, h, w, k, d_area, d_box, d_plane ? d_vmax : nullptr);
+    int32_t *vmax = d_plane ? d_vmax : nullptr;
+    if (!launch(k_stats_init, grid_for(k), st, kRouteThreads, k, d_area, d_box, vmax) ||
+        !launch(k_stats, grid_for_words((int64_t)h * words_per_row(w)), st, kRouteThreads,
+                d_labels, d_plane, h, w, k, d_area, d_box, vmax))
+        return FX_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess ? FX_OK : FX_ERR_CUDA;
 }
 
@@ -776,12 +810,14 @@ FX_API int fx_dilate_square(const uint8_t *d_in, int32_t h, int32_t w, int32_t r
         const dim3 grid((words_per_row(w) + kDilateWords - 1) / kDilateWords,
                         (h + kDilateRows - 1) / kDilateRows);
         if (grid.y <= 65535u) {
-            k_dilate_tile<<<grid, kRouteThreads, 0, st>>>(d_in, h, w, rv, rh, d_out);
+            if (!launch(k_dilate_tile, grid, st, kRouteThreads, d_in, h, w, rv, rh, d_out))
+                return FX_ERR_CUDA;
             return cudaStreamSynchronize(st) == cudaSuccess ? FX_OK : FX_ERR_CUDA;
         }
     }
-    k_dilate_cols<<<(w + 127) / 128, 128, 0, st>>>(d_in, h, w, rv, d_work);
-    k_dilate_rows<<<(h + 127) / 128, 128, 0, st>>>(d_work, h, w, rh, d_out);
+    if (!launch(k_dilate_cols, tiles_of(1, w, 1, 128), st, 128, d_in, h, w, rv, d_work) ||
+        !launch(k_dilate_rows, tiles_of(1, h, 1, 128), st, 128, d_work, h, w, rh, d_out))
+        return FX_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess ? FX_OK : FX_ERR_CUDA;
 }
 
@@ -793,11 +829,11 @@ FX_API int fx_label_pairs(const int32_t *d_a, const int32_t *d_b, int32_t h, int
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), st) != cudaSuccess)
         return FX_ERR_CUDA;
-    k_pairs<<<grid_for((int64_t)h * w), kRouteThreads, 0, st>>>(
-        d_a, d_b, h, w, capacity, reinterpret_cast<int2 *>(d_pairs), d_count);
     unsigned long long c = 0;
-    cudaMemcpyAsync(&c, d_count, sizeof(c), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return FX_ERR_CUDA;
+    if (!launch(k_pairs, grid_for((int64_t)h * w), st, kRouteThreads, d_a, d_b, h, w, capacity,
+                reinterpret_cast<int2 *>(d_pairs), d_count) ||
+        !fetch(&c, d_count, sizeof(c), st))
+        return FX_ERR_CUDA;
     *count = (int64_t)c;
     return (int64_t)c > capacity ? FX_ERR_OUT_OF_MEMORY : FX_OK;
 }
@@ -896,8 +932,9 @@ FX_API int fx_map_labels(const int32_t *d_labels, int64_t n, const int32_t *d_ma
     if (!d_labels || !d_map || (!d_out_i32 && !d_out_u8) || n < 1 || k < 0)
         return FX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    k_map_labels<<<grid_for(n), kRouteThreads, 0, st>>>(d_labels, n, d_map, k, d_out_i32,
-                                                       d_out_u8);
+    if (!launch(k_map_labels, grid_for(n), st, kRouteThreads, d_labels, n, d_map, k, d_out_i32,
+                d_out_u8))
+        return FX_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess ? FX_OK : FX_ERR_CUDA;
 }
 
@@ -908,10 +945,11 @@ FX_API int fx_clear_label(uint8_t *d_mask, const int32_t *d_labels, int64_t n, i
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(d_scratch, 0, sizeof(unsigned long long), st) != cudaSuccess)
         return FX_ERR_CUDA;
-    k_clear_label<<<grid_for(n), kRouteThreads, 0, st>>>(d_mask, d_labels, n, id, d_scratch);
     unsigned long long c = 0;
-    cudaMemcpyAsync(&c, d_scratch, sizeof(c), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return FX_ERR_CUDA;
+    if (!launch(k_clear_label, grid_for(n), st, kRouteThreads, d_mask, d_labels, n, id,
+                d_scratch) ||
+        !fetch(&c, d_scratch, sizeof(c), st))
+        return FX_ERR_CUDA;
     *cleared = (int64_t)c;
     return FX_OK;
 }
@@ -925,7 +963,9 @@ FX_API int fx_count_where(const int32_t *d_key, const int32_t *d_cond, int64_t n
     if (cudaMemsetAsync(d_counts, 0, (size_t)(k + 1) * sizeof(unsigned long long), st) !=
         cudaSuccess)
         return FX_ERR_CUDA;
-    k_count_where<<<grid_for_words((n + 31) / 32), kRouteThreads, 0, st>>>(d_key, d_cond, n, k, d_counts);
+    if (!launch(k_count_where, grid_for_words((n + 31) / 32), st, kRouteThreads, d_key, d_cond, n,
+                k, d_counts))
+        return FX_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess ? FX_OK : FX_ERR_CUDA;
 }
 
@@ -936,8 +976,9 @@ FX_API int fx_tile_extract(const int32_t *d_labels, int32_t h, int32_t w, int32_
         x0 + tw > w)
         return FX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    k_tile_extract<<<grid_for((int64_t)th * tw), kRouteThreads, 0, st>>>(d_labels, w, y0, x0, th,
-                                                                        tw, id, d_tile);
+    if (!launch(k_tile_extract, grid_for((int64_t)th * tw), st, kRouteThreads, d_labels, w, y0, x0,
+                th, tw, id, d_tile))
+        return FX_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess ? FX_OK : FX_ERR_CUDA;
 }
 
@@ -949,7 +990,8 @@ FX_API int fx_tile_scatter(const int32_t *d_tile_labels, int32_t h, int32_t w, i
         x0 + tw > w)
         return FX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    k_tile_scatter<<<grid_for((int64_t)th * tw), kRouteThreads, 0, st>>>(d_tile_labels, w, y0, x0,
-                                                                        th, tw, base, d_plane);
+    if (!launch(k_tile_scatter, grid_for((int64_t)th * tw), st, kRouteThreads, d_tile_labels, w, y0,
+                x0, th, tw, base, d_plane))
+        return FX_ERR_CUDA;
     return cudaStreamSynchronize(st) == cudaSuccess ? FX_OK : FX_ERR_CUDA;
 }

@@ -212,3 +212,29 @@ def test_dilation_tiles_match_oracle(shape, radius):
     mask[shape[0] // 2, shape[1] // 2] = True
     out = _dev().dilate(torch.from_numpy(mask.view(np.uint8)).cuda(), *shape, radius)
     assert np.array_equal(out.cpu().numpy().view(np.bool_), ro.dilate_square(mask, radius))
+
+
+# rows of 16-row tiles on both sides of 65,535, the blocks of a grid's second axis, and of
+# the 32-row tiles of the relaxation, which the gap of 300 rows reaches
+@pytest.mark.parametrize("h, w", [(1048560, 1), (1048577, 1), (1048577, 40), (2097153, 1)])
+def test_chessboard_distance_of_tall_masks(h, w):
+    import torch
+
+    rows = np.arange(h)
+    background = np.concatenate([rows[:h - 400:50], rows[h - 101:]])  # whole rows
+    mask = np.ones((h, w), np.uint8)
+    mask[background] = 0
+    after = np.searchsorted(background, rows)
+    expected = np.minimum(np.abs(rows - background[np.minimum(after, len(background) - 1)]),
+                          np.abs(rows - background[np.maximum(after - 1, 0)]))
+    assert expected.max() >= 150
+    dist = _dev().distance(torch.from_numpy(mask).cuda(), h, w).cpu().numpy()
+    assert np.array_equal(dist, np.broadcast_to(expected[:, None], (h, w)))
+
+
+def test_census_of_a_tall_mask_measures_its_regions():
+    mask = np.zeros((1048577, 1), bool)
+    mask[1000:1040] = mask[700000:700003] = mask[-90:-20] = True
+    result = routing.route_at_floor_mask(mask)
+    assert [(r.area, r.max_chessboard_radius) for r in result.provisional_regions] == [
+        (40, 20), (3, 2), (70, 35)]
