@@ -610,8 +610,8 @@ __global__ void __launch_bounds__(kRouteThreads)
     }
 }
 
-// Larger radii: each thread sweeps one column or one row twice (nearest set
-// pixel before and after), so any radius costs the same.
+// Larger radii, and a dilation in place: each thread sweeps one column or one
+// row twice (nearest set pixel before and after), so any radius costs the same.
 __global__ void k_dilate_cols(const uint8_t *__restrict__ in, int h, int w, int r,
                               uint8_t *__restrict__ out) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -806,7 +806,12 @@ FX_API int fx_dilate_square(const uint8_t *d_in, int32_t h, int32_t w, int32_t r
     if (!d_in || !d_work || !d_out || h < 1 || w < 1 || radius < 0) return FX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int rv = radius < h - 1 ? radius : h - 1, rh = radius < w - 1 ? radius : w - 1;
-    if (rv <= kDilateBits && rh <= kDilateBits) {
+    // a block of the tile kernel reads its halo from d_in while others write
+    // d_out; planes that overlap take the two sweeps through d_work
+    const uintptr_t in = reinterpret_cast<uintptr_t>(d_in), out = reinterpret_cast<uintptr_t>(d_out);
+    const uintptr_t n = (uintptr_t)h * (uintptr_t)w;
+    const bool apart = in + n <= out || out + n <= in;
+    if (apart && rv <= kDilateBits && rh <= kDilateBits) {
         const dim3 grid((words_per_row(w) + kDilateWords - 1) / kDilateWords,
                         (h + kDilateRows - 1) / kDilateRows);
         if (grid.y <= 65535u) {

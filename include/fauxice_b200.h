@@ -359,7 +359,7 @@ FX_API int fx_label_stats(const int32_t *d_labels, const int32_t *d_plane, int32
                           void *stream);
 /* Square (Chebyshev) dilation by `radius`, zero outside the frame, the
  * radius clipped per axis to the frame (routing.py:304-336).  d_work is
- * uint8[h*w] scratch. */
+ * uint8[h*w] scratch, apart from the other two; d_out may be d_in. */
 FX_API int fx_dilate_square(const uint8_t *d_in, int32_t h, int32_t w, int32_t radius,
                             uint8_t *d_work, uint8_t *d_out, void *stream);
 /* Distinct (a, b) pairs of two label planes over pixels where both are

@@ -238,3 +238,22 @@ def test_census_of_a_tall_mask_measures_its_regions():
     result = routing.route_at_floor_mask(mask)
     assert [(r.area, r.max_chessboard_radius) for r in result.provisional_regions] == [
         (40, 20), (3, 2), (70, 35)]
+
+
+@pytest.mark.parametrize("offset", [0, 1, 1500])  # the output's start in the input plane
+@pytest.mark.parametrize("radius", [1, 12, 31])
+def test_dilation_in_place_matches_oracle(radius, offset):
+    import torch
+
+    h, w = 700, 1100
+    mask = np.random.default_rng(radius).random((h, w)) < 0.001
+    plane = torch.zeros(h * w + offset, dtype=torch.uint8, device="cuda")
+    plane[:h * w] = torch.from_numpy(mask.view(np.uint8).ravel()).cuda()
+    work = torch.empty(h * w, dtype=torch.uint8, device="cuda")
+    at = plane.data_ptr()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert _lib.load().fx_dilate_square(ctypes.c_void_p(at), h, w, radius,
+                                        ctypes.c_void_p(work.data_ptr()),
+                                        ctypes.c_void_p(at + offset), stream) == 0
+    out = plane[offset:].cpu().numpy().reshape(h, w)
+    assert np.array_equal(out.view(np.bool_), ro.dilate_square(mask, radius))
