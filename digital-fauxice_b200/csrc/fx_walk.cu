@@ -891,7 +891,10 @@ __global__ void __launch_bounds__(kWinThreads, kWinBlocksPerSM)
 // one dependent chain of 23 cycles, so a piece takes 512 of them, and the
 // pieces of a native frame are about one warp per scheduler.  Walking each
 // 4096-channel segment on one lane took 124 us whatever the frame's size;
-// this takes 42 us on a native frame (6.6 M channels) and 19 us on 256x256.
+// this takes 78 us on a native frame (8.9 M channels) and 19 us on 256x256.
+// A serial walk (a short chain, or all of one) is one lane: only its row is
+// staged, and the idle lanes don't hold it off the unrolled steps (113.9 ->
+// 45.2 ms for the 2.2 M channels of a 2892x1973 frame).
 constexpr int kRewalkChunk = 32;  // channels per staged chunk
 constexpr int kRewalkRing = 3;
 
@@ -959,10 +962,12 @@ __global__ void __launch_bounds__(32)
     const uint32_t mine = (b - from + kRewalkChunk - 1) / kRewalkChunk;
     const uint32_t chunks = __reduce_max_sync(0xFFFFFFFFu, mine);
     if (chunks == 0) return;
+    // lanes up to the last with channels (one alone on a serial walk)
+    const int rows = 32 - __clz(__ballot_sync(0xFFFFFFFFu, mine > 0u));
     auto issue = [&](uint32_t k) {
         if (k < chunks) {
 #pragma unroll 8
-            for (int q = 0; q < 32; ++q) {
+            for (int q = 0; q < rows; ++q) {
                 const uint32_t f = __shfl_sync(0xFFFFFFFFu, from, q) + k * kRewalkChunk + lane;
                 if (f < __shfl_sync(0xFFFFFFFFu, b, q)) {
                     const uint32_t sa =
@@ -985,7 +990,9 @@ __global__ void __launch_bounds__(32)
         const uint4 *row = S.e[k % kRewalkRing][lane];
         const bool two = cnt && B.chunk_two[i / kWalkChunk] != 0;
         uint32_t bits = 0;
-        if (__all_sync(0xFFFFFFFFu, cnt == (uint32_t)kRewalkChunk && !two)) {
+        // a lane past its end steps through whatever its row holds; its state
+        // and count are not used again
+        if (__all_sync(0xFFFFFFFFu, cnt == 0u || (cnt == (uint32_t)kRewalkChunk && !two))) {
 #pragma unroll
             for (int r = 0; r < kRewalkChunk; ++r) {
                 const uint4 e = row[r];

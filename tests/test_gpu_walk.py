@@ -68,3 +68,20 @@ def test_waves_near_the_widest_draw_as_the_oracle(wave, sigmas):
     assert np.array_equal(result.output_rgb16, expected.output_rgb16)
     assert result.replay.public_rng_advances == expected.public_rng_advances
     assert result.replay.final_rng_state == expected.final_rng_state
+
+
+@pytest.mark.parametrize("h, w, spec", [(61, 64, "native"), (200, 333, "heavy"),
+                                        (517, 611, "heavy"), (300, 411, "native")])
+def test_serial_walk_draws_as_the_oracle(h, w, spec):
+    """One lane walks the whole chain (rows of 32 channels and a remainder)."""
+
+    job, expected = _case(h, w, spec)
+    ctx, lib = engine.context(), _lib.load()
+    assert lib.fx_set_parallel_walk(ctx.handle, 0) == 0
+    try:
+        result = process_b200(job)
+    finally:
+        assert lib.fx_set_parallel_walk(ctx.handle, 1) == 0
+    assert np.array_equal(result.output_rgb16, expected.output_rgb16)
+    assert result.replay.public_rng_advances == expected.public_rng_advances
+    assert result.replay.final_rng_state == expected.final_rng_state
