@@ -257,3 +257,17 @@ def test_dilation_in_place_matches_oracle(radius, offset):
                                         ctypes.c_void_p(at + offset), stream) == 0
     out = plane[offset:].cpu().numpy().reshape(h, w)
     assert np.array_equal(out.view(np.bool_), ro.dilate_square(mask, radius))
+
+
+@pytest.mark.parametrize("shape", [(300, 300), (701, 933), (97, 63)])
+@pytest.mark.parametrize("kind", ["stripes", "checker", "noise"])
+def test_many_links_a_word_match_oracle(shape, kind):
+    import torch
+
+    y, x = np.ogrid[:shape[0], :shape[1]]
+    mask = {"stripes": (x % 2 == 0) & (y >= 0), "checker": (x + y) % 2 == 0,
+            "noise": np.random.default_rng(shape[0]).random(shape) < 0.5}[kind]
+    labels, count = _dev().label8(torch.from_numpy(mask.view(np.uint8)).cuda(), *shape)
+    expected, expected_count = ro.label8(mask)
+    assert count == expected_count
+    assert np.array_equal(labels.cpu().numpy(), expected)
