@@ -608,6 +608,15 @@ FX_API int fx_stage_table(int32_t h, const float *p1, const float *p2, const flo
     return host_stage_table(h, p1, p2, mv, mi, factor_b, stages);
 }
 
+FX_API int fx_write_site(const fx_params *params, int32_t floor_enabled, const double *candidates,
+                         const float *originals, uint32_t meta, uint32_t redraw, uint32_t *state,
+                         float *values, int32_t *draws) {
+    if (!params || !candidates || !originals || !state || !values || !draws)
+        return FX_ERR_INVALID_ARGUMENT;
+    return host_write_site(*params, floor_enabled != 0, candidates, originals, meta, redraw, state,
+                           values, draws);
+}
+
 FX_API int fx_producer_rows(fx_context *ctx, const uint16_t *main_rgbi, int32_t h, int32_t w,
                             float *p1, float *p2, float *mv, float *mi) {
     if (!ctx || !main_rgbi || h < 1 || w < 8 || !p1 || !p2 || !mv || !mi)

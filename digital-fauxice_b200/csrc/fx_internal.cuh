@@ -139,25 +139,24 @@ __host__ __device__ __forceinline__ DitherConst dither_const(const fx_params &p)
 }
 
 // Raw delta for a first-draw state s1 (before the accept test).
-__device__ __forceinline__ double dither_raw_delta(double cand, double envelope, float span,
-                                                   uint32_t s1) {
+__host__ __device__ __forceinline__ double dither_raw_delta(double cand, double envelope,
+                                                            float span, uint32_t s1) {
     const double unit = (double)(s1 + 1u) * kNormalization - 0.5;
     const double random_value = 0.0 + unit * (double)span;
     return envelope * random_value;
 }
 
-// conditional_dither_delta split in two: the state-free part of one
-// channel (whether it draws, the float32-rounded candidate, the binary64
-// envelope and the float32 span), computed once for both draws a channel
-// may take, and one draw with the state advanced in place.
+// The state-free part of conditional_dither_delta for one channel: whether it
+// draws, the float32-rounded candidate, the binary64 envelope and the float32
+// span, computed once for both draws a channel may take.
 struct DitherChannel {
     double cand, envelope;
     float span;
     bool draws;
 };
 
-__device__ __forceinline__ DitherChannel dither_channel(double value, float scale32,
-                                                        const DitherConst &dc) {
+__host__ __device__ __forceinline__ DitherChannel dither_channel(double value, float scale32,
+                                                                 const DitherConst &dc) {
     DitherChannel ch;
     const float cand32 = (float)value;
     ch.cand = (double)cand32;
@@ -167,17 +166,59 @@ __device__ __forceinline__ DitherChannel dither_channel(double value, float scal
     return ch;
 }
 
-// One draw: the accepted delta (or 0).  `drew` reports whether the LCG
-// advanced.
-__device__ __forceinline__ double dither_draw(const DitherChannel &ch, const DitherConst &dc,
-                                              uint32_t &state, int &drew) {
-    drew = 0;
-    if (!ch.draws) return 0.0;
-    state = (125u * state + 1u) & kLcgMask;
-    drew = 1;
-    const double d = dither_raw_delta(ch.cand, ch.envelope, ch.span, state);
-    const double changed = ch.cand + d;
-    return (dc.low < changed && changed < dc.high) ? d : 0.0;
+// One attempted site from the state before its first draw, as the reference's
+// writer runs it: every draw is made and every test evaluated, whatever the
+// classification (meta) and the walk (redraw: a bit per RNG-dependent channel,
+// 1 for two draws) say; `agrees` is whether they say the same draws.
+struct WrittenSite {
+    float value[3];
+    bool kept[3];    // the channel keeps its original
+    uint32_t draws;
+    bool agrees;
+};
+
+__host__ __device__ __forceinline__ WrittenSite write_site(const double cand[3],
+                                                           const float orig[3],
+                                                           bool floor_enabled,
+                                                           const float scales[3],
+                                                           const DitherConst &dc, uint8_t meta,
+                                                           uint32_t redraw, uint32_t &state) {
+    WrittenSite out;
+    out.draws = 0;
+    out.agrees = true;
+    bool valid = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) valid &= isfinite(cand[c]) && cand[c] > 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        uint32_t told = (uint32_t)meta_code(meta, c);
+        if (told == 3u) {  // one draw and a copy, or two
+            told = 1u + (redraw & 1u);
+            redraw >>= 1;
+        }
+        uint32_t made = 0;
+        out.value[c] = orig[c];
+        out.kept[c] = true;
+        if (valid) {
+            const DitherChannel ch = dither_channel(cand[c], scales[c], dc);
+            auto draw = [&] {
+                state = (125u * state + 1u) & kLcgMask;
+                ++made;
+                const double d = dither_raw_delta(ch.cand, ch.envelope, ch.span, state);
+                const double moved = ch.cand + d;
+                return (dc.low < moved && moved < dc.high) ? d : 0.0;
+            };
+            double d = ch.draws ? draw() : 0.0;
+            out.kept[c] = floor_enabled && cand[c] + d <= (double)orig[c];
+            if (!out.kept[c]) {
+                if (floor_enabled && ch.draws) d = draw();
+                out.value[c] = (float)(cand[c] + d);
+            }
+        }
+        out.draws += made;
+        out.agrees &= made == told;
+    }
+    return out;
 }
 
 // ---------------------------------------------------------------------------
@@ -334,6 +375,9 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
                           uint8_t *changed_out, uint32_t *err, cudaStream_t stream,
                           const Marks &marks);
 size_t dev_counters_bytes();
+int host_write_site(const fx_params &p, bool floor_enabled, const double cand[3],
+                    const float orig[3], uint32_t meta, uint32_t redraw, uint32_t *state,
+                    float values[3], int32_t *draws);
 cudaError_t walk_init();
 size_t walk_scratch_bytes(int64_t capacity, int widest);
 int64_t walk_segments(int64_t capacity, int per_wave);

@@ -357,9 +357,10 @@ constexpr int kUnitSites = 256;  // most sites of a unit
 static_assert(kSegment == 1024 && kUnitSites == 32 * 8, "32 and 8 meta bytes per lane");
 
 // Sites of a unit of k_coef and k_apply (template instances).  256 keep a
-// warp's lists dense; where 64 still give every resident warp at most one
-// unit, the frame is bound by one unit's latency and 64 are faster: a 256x256
-// frame's chain 29 -> 19 us and apply 24 -> 20.
+// warp's lists dense; where 64 still give every resident warp of k_coef at most
+// one unit, the frame is bound by one unit's latency and 64 are faster: a
+// 256x256 frame's chain 29 -> 19 us and apply 24 -> 20, of 580x600 34 -> 23 and
+// 25 -> 25.
 static int unit_sites(int64_t segments, int resident_warps) {
     return segments * (kSegment / 64) <= resident_warps ? 64 : kUnitSites;
 }
@@ -595,9 +596,21 @@ cudaError_t writer_identity_table(const float *lut, const uint32_t *hi, const ui
     return cudaGetLastError();
 }
 
-constexpr int kApplyBlocksPerSM = 5;  // k_apply's resident blocks per SM
+constexpr int kApplyBlocksPerSM = 4;  // k_apply's resident blocks per SM
 static int g_apply_blocks = kApplyBlocksPerSM * 148;
 static int g_coef_blocks = kCoefBlocksPerSM * 148;
+
+int host_write_site(const fx_params &p, bool floor_enabled, const double cand[3],
+                    const float orig[3], uint32_t meta, uint32_t redraw, uint32_t *state,
+                    float values[3], int32_t *draws) {
+    uint32_t s = *state & kLcgMask;
+    const WrittenSite out = write_site(cand, orig, floor_enabled, p.dither_scales, dither_const(p),
+                                       (uint8_t)meta, redraw, s);
+    for (int c = 0; c < 3; ++c) values[c] = out.value[c];
+    *draws = (int32_t)out.draws;
+    *state = s;
+    return out.agrees ? FX_OK : FX_ERR_INTERNAL;
+}
 
 cudaError_t writer_init() {
     int device = 0, sms = 0;
@@ -641,16 +654,17 @@ cudaError_t writer_init() {
 //     (their output is the identity emit);
 //   * the list is processed densely, one attempted site per lane, from its
 //     own start state: the segment's, advanced by the draws inside it.
-// A channel's classification and the walk's bit say which of its draws
-// decides its value, so at most one is evaluated, and none where the original
-// is copied.  The first six units are the startup rows' counts; the last block
-// to finish chains the rows and writes the final state.
-// Measured on a native frame with half its pixels attempted: 505 us as blocks
-// of 256 threads with a block scan, four pixels per thread, both draws of
-// every channel and a six-digit jump per site (564 warp instructions per 32
-// pixels, 357 now); 332 us so.  The gathers' L1 decides the rest: with the
-// samples staged in shared memory five blocks took 505 us and six 866, with a
-// 128 KB emit table instead of the two factor tables 420.
+// Every draw is evaluated again and compared with the classification and the
+// walk's bits (write_site).  The first six units are the startup rows' counts;
+// the last block to finish chains the rows and writes the final state.
+// Bound: instruction issue and the gathers' L1.  Measured on a native frame
+// with half its pixels attempted, every draw evaluated: 505 us as blocks of 256
+// threads with a block scan, four pixels per thread and a six-digit jump per
+// site; 396 us so.  Four blocks per SM: five at 48 registers 403; with the next
+// 32 sites' loads in flight, four blocks took 424, five 457 and three 453.
+// Without the comparison, at most one draw a channel, it took 330.  The gathers' L1 decides
+// the rest: with the samples staged in shared memory five blocks took 505 us
+// and six 866, with a 128 KB emit table instead of the two factor tables 420.
 constexpr int kApplyWarps = 8;
 
 __device__ void apply_final(const uint32_t *seg_base, const uint32_t *seg_amb, int64_t segments,
@@ -825,90 +839,52 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kApplyBlocksPerSM)
             seg_t = f.a * seg_t + f.c;
         }
         __syncwarp();  // the list is complete
-        // ---- attempted sites, densely: one round's loads are in flight while
-        // the round before is computed ------------------------------------------
-        struct Site {
-            uint2 entry, raw, words;  // list entry, samples, extra draws
-            double cand[3];
-        };
-        auto fetch = [&](uint32_t k) {
-            Site q;
-            if (k < total) {
-                q.entry = list[k];
-                const int64_t site = seg * kSegment + (q.entry.x & 0xFFFFu);
-                q.raw = reinterpret_cast<const uint2 *>(rgbi)[site - su];
-                const uint32_t a =
-                    (uint32_t)min((int64_t)(seg_a + (q.entry.y >> 16)), capacity);
-                q.words = __ldg(reinterpret_cast<const uint2 *>(extra) + (a >> 5));
-#pragma unroll
-                for (int c = 0; c < 3; ++c) q.cand[c] = cand[3 * site + c];
-            }
-            return q;
-        };
-        Site cur = fetch(lane);
+        // ---- attempted sites, densely ------------------------------------------
         for (uint32_t k = lane; k < total; k += 32) {
-            const Site q = cur;
-            cur = fetch(k + 32);
-            const uint8_t mi = (uint8_t)(q.entry.x >> 16);
-            // H*W < 2^31
-            const uint32_t pixel = (uint32_t)(seg * kSegment + (q.entry.x & 0xFFFFu) - su);
-            const uint32_t lanes[3] = {q.raw.x & 0xFFFFu, q.raw.x >> 16, q.raw.y & 0xFFFFu};
+            const uint2 entry = list[k];
+            const int64_t site = seg * kSegment + (entry.x & 0xFFFFu);
+            const uint32_t pixel = (uint32_t)(site - su);  // H*W < 2^31
+            const uint2 raw = reinterpret_cast<const uint2 *>(rgbi)[pixel];
+            const uint32_t lanes[3] = {raw.x & 0xFFFFu, raw.x >> 16, raw.y & 0xFFFFu};
             uint16_t e0[3];
+            float orig[3];
+            double c3[3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) e0[c] = __ldg(ident + lanes[c]);
+            for (int c = 0; c < 3; ++c) {
+                c3[c] = cand[3 * site + c];
+                e0[c] = __ldg(ident + lanes[c]);
+                orig[c] = __ldg(lut + lanes[c]);
+            }
             // the walk's bits of this site's RNG-dependent channels, and the
             // extra draws before them
-            const uint32_t a = (uint32_t)min((int64_t)(seg_a + (q.entry.y >> 16)), capacity);
+            const uint8_t mi = (uint8_t)(entry.x >> 16);
+            const uint32_t a = (uint32_t)min((int64_t)(seg_a + (entry.y >> 16)), capacity);
             const uint32_t sh = a & 31u;
-            uint32_t redraw = q.words.y >> sh;
+            const uint2 words = __ldg(reinterpret_cast<const uint2 *>(extra) + (a >> 5));
+            uint32_t redraw = words.y >> sh;
             if (sh + (uint32_t)meta_amb(mi) > 32u)
                 redraw |= __ldg(&extra[(a >> 5) + 1].bits) << (32u - sh);
-            const uint32_t n = (q.entry.y & 0xFFFFu) + q.words.x +
-                               (uint32_t)__popc(q.words.y & ((1u << sh) - 1u)) - seg_e;
+            const uint32_t n = (entry.y & 0xFFFFu) + words.x +
+                               (uint32_t)__popc(words.y & ((1u << sh) - 1u)) - seg_e;
             const Affine f0 = s_jump[0][n & 127u], f1 = s_jump[1][(n >> 7) & 127u];
             uint32_t state = (f1.a * (f0.a * seg_t + f0.c) + f1.c) >> 8;
             const bool floor_enabled =
                 p.driver_gate_primary || stages[pixel / (uint32_t)w + 6].gate_secondary;
-            bool valid = true;
-            if ((mi & 0x3Fu) == 0u)  // no draws: all channels outside the bounds, or invalid
-#pragma unroll
-                for (int c = 0; c < 3; ++c) valid &= isfinite(q.cand[c]) && q.cand[c] > 0.0;
+            const WrittenSite out =
+                write_site(c3, orig, floor_enabled, p.dither_scales, dc, mi, redraw, state);
+            // (a list past its capacity is run again with a longer one)
+            if (!out.agrees && (int64_t)(seg_a + (entry.y >> 16)) + meta_amb(mi) <= capacity)
+                raise_error(err, FX_ERR_INTERNAL);
+            draws_total += out.draws;
             bool wrote = false, differs = false;
             uint16_t *o = rgb_out + 3 * (int64_t)pixel;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                int code = meta_code(mi, c);
-                if (code == 3) {  // one draw and a copy, or two
-                    code = (redraw & 1u) ? 2 : 1;
-                    redraw >>= 1;
-                }
-                // the draw that decides the value (the first draw copies the
-                // original where the floor gate is on)
-                if (code >= 1) state = (125u * state + 1u) & kLcgMask;
-                if (code == 2) state = (125u * state + 1u) & kLcgMask;
-                draws_total += (uint32_t)code;
                 uint16_t e = e0[c];
-                if (valid && !(code == 1 && floor_enabled)) {
-                    const double c3 = q.cand[c];
-                    float v;
-                    bool copied = false;
-                    if (code == 0) {
-                        const float orig = __ldg(lut + lanes[c]);
-                        copied = floor_enabled && c3 <= (double)orig;
-                        v = (float)c3;
-                    } else {
-                        const DitherChannel ch = dither_channel(c3, p.dither_scales[c], dc);
-                        const double d = dither_raw_delta(ch.cand, ch.envelope, ch.span, state);
-                        const double moved = ch.cand + d;
-                        v = (float)(c3 + ((dc.low < moved && moved < dc.high) ? d : 0.0));
-                    }
-                    if (!copied) {
-                        if (!isfinite(v)) ok = false;
-                        else e = emit_index(emit_index_of(v), hi, lo);
-                        // an output that differs was written; one that does not
-                        // may still come from another value
-                        wrote |= e != e0[c] || !(v == __ldg(lut + lanes[c]));
-                    }
+                if (!out.kept[c]) {
+                    if (!isfinite(out.value[c])) ok = false;
+                    else e = emit_index(emit_index_of(out.value[c]), hi, lo);
+                    wrote |= !(out.value[c] == orig[c]);
                 }
                 differs |= e != e0[c];
                 o[c] = e;
@@ -973,8 +949,7 @@ cudaError_t launch_writer(const Geometry &g, const uint8_t *meta, const double *
                     g.sites, segs, b.seg_raw, b.seg_base, b.seg_amb, ctr, err);
     if (e != cudaSuccess) return e;
     const uint32_t *n_amb = b.seg_amb + segs;
-    const int us = unit_sites(segs, std::min(g_coef_blocks * kCoefWarps,
-                                             g_apply_blocks * kApplyWarps));
+    const int us = unit_sites(segs, g_coef_blocks * kCoefWarps);
     const int64_t unit_blocks = (segs * (kSegment / us) + kCoefWarps - 1) / kCoefWarps;
     e = launch_chained(us == 64 ? k_coef<64> : k_coef<kUnitSites>,
                     dim3((unsigned)std::min<int64_t>(unit_blocks, g_coef_blocks)),

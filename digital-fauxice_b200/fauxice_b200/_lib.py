@@ -142,6 +142,8 @@ SIGNATURES = {
     "fx_sync_counters": ([_P, ctypes.POINTER(FxCounters)], ctypes.c_int),
     "fx_set_slots": ([_P, ctypes.c_int32], ctypes.c_int),
     "fx_set_parallel_walk": ([_P, ctypes.c_int], ctypes.c_int),
+    "fx_write_site": ([_P, ctypes.c_int32, _P, _P, ctypes.c_uint32, ctypes.c_uint32, _P, _P, _P],
+                      ctypes.c_int),
     "fx_set_walk_wave": ([_P, ctypes.c_int32], ctypes.c_int),
     "fx_walk_segments": ([ctypes.c_int64, ctypes.c_int32, _P, _P], ctypes.c_int),
     "fx_set_launch_priority": ([_P, ctypes.c_int], ctypes.c_int),

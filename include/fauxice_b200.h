@@ -182,6 +182,15 @@ FX_API int fx_stage_table(int32_t height, const float *scaled_input, const float
                           const float *mean_visible, const float *mean_infrared,
                           float auxiliary_factor_b, fx_stage *stages);
 
+/* write_reconstructed_pixel (reconstruction.py:916-982) of one attempted site
+ * from the RNG state before it; host computation, the same code that the emit
+ * kernel runs.  `meta` holds a draw code per channel in bits 2c, 2c + 1 (0, 1
+ * or 2 draws, 3: one or two) and `redraw` a bit per code-3 channel in order (1:
+ * two draws); FX_ERR_INTERNAL when the draws made are others. */
+FX_API int fx_write_site(const fx_params *params, int32_t floor_enabled,
+                         const double *candidates, const float *originals, uint32_t meta,
+                         uint32_t redraw, uint32_t *state, float *values, int32_t *draws);
+
 /* The whole main-scan pass for one frame, synchronous, host buffers:
  * streaming.py:365-552 (run_streaming_replay) / cuda_backend/engine.py:183
  * (run_streaming_replay_cuda), including the hidden startup replay, the
