@@ -644,7 +644,8 @@ def run_b200(args, world, rank, local, frames=None, heavy=None, pool=None):
         }
         if frames is not None:
             line["batched"] = run_batched(ctx, frames, args, golden)
-            line["e2e_batched"] = run_e2e_batched(frames, line["batched"])
+            line["e2e_batched"] = run_e2e_batched(frames, line["batched"],
+                                                  args.batch_steps)
         if heavy is not None:
             line["heavy_batched"] = run_heavy(ctx, heavy, args, golden, line.get("batched"))
         if pool is not None:
@@ -858,7 +859,7 @@ def run_heavy(ctx, frames, args, golden, batched):
     }
 
 
-def run_e2e_batched(frames, batched):
+def run_e2e_batched(frames, batched, steps):
     """The batched mix through the public host-buffer API: 16 jobs of host
     numpy frames into process_batch (validation, prepass, staged uploads,
     passes, downloads and output SHA-256 digests all inside the timed
@@ -872,13 +873,17 @@ def run_e2e_batched(frames, batched):
     jobs = [make_job(f, synthetic.make_prepass(f)) for f in frames]
     slots = inspect.signature(batch.process_batch).parameters["slots"].default
     batch.process_batch(jobs)  # warm: pinned staging of every slot
-    t0 = time.perf_counter()
-    results = batch.process_batch(jobs)
-    elapsed = time.perf_counter() - t0
+    times = []
+    for _ in range(steps):
+        t0 = time.perf_counter()
+        results = batch.process_batch(jobs)
+        times.append(time.perf_counter() - t0)
+    elapsed = statistics.median(times)
     mp = sum(f.shape[0] * f.shape[1] for f in frames) / 1e6
     exact = all(r.replay.output_sha256 == d for r, d in zip(results, digests))
     return {"value": round(mp / elapsed, 1), "unit": "MP/s", "ms_per_step": round(1e3 * elapsed, 1),
-            "frames": len(frames), "slots": slots,
+            "frames": len(frames), "slots": slots, "steps": steps,
+            "ms_each": [round(1e3 * t, 1) for t in times],
             "h2d_bytes_per_step": int(sum(f.nbytes for f in frames)),
             "d2h_bytes_per_step": int(sum(f.shape[0] * f.shape[1] * 6 for f in frames)),
             "bit_exact_vs_device_batch": bool(exact),
