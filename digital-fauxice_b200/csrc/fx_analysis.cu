@@ -59,7 +59,7 @@ __device__ __forceinline__ float nonfinite(float x, float seen) { return fmaf(x,
 // padded too, but edge-replicated (the decision bars clamp their indices,
 // streaming.py:166-198): padded (y, x) holds the aux of (clamp(y), clamp(x)).
 //
-// Bound: wavefronts in L1 (the four LUT gathers per pixel; 61% of its peak)
+// Bound: wavefronts in L1 (the four LUT gathers per pixel; 57% of its peak)
 // and the planes' bytes (32 per position, 4 TB/s).  Native frame 159 us;
 // one column per thread, each with its own binary64 division and a fifth
 // gather, took 217.  Stores that stay in L2 (no .cs) 165; a column per lane

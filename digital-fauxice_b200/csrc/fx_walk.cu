@@ -891,10 +891,11 @@ __global__ void __launch_bounds__(kWinThreads, kWinBlocksPerSM)
 // one dependent chain of 23 cycles, so a piece takes 512 of them, and the
 // pieces of a native frame are about one warp per scheduler.  Walking each
 // 4096-channel segment on one lane took 124 us whatever the frame's size;
-// this takes 78 us on a native frame (8.9 M channels) and 19 us on 256x256.
+// this takes 60 us on a native frame (8.9 M channels) and 15 us on 256x256.
 // A serial walk (a short chain, or all of one) is one lane: only its row is
 // staged, and the idle lanes don't hold it off the unrolled steps (113.9 ->
-// 45.2 ms for the 2.2 M channels of a 2892x1973 frame).
+// 45.2 ms for the 2.2 M channels of a 2892x1973 frame; a warp of pieces that
+// end apart gains as well, 78 -> 60 us).
 constexpr int kRewalkChunk = 32;  // channels per staged chunk
 constexpr int kRewalkRing = 3;
 

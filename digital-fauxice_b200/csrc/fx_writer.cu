@@ -19,9 +19,10 @@
 //   4. the walk (fx_walk.cu) visits only the RNG-dependent channels: a
 //      multiply-add, a test and a conditional LCG step per channel,
 //      parallelised over segments by speculation.  Output: the running count of extra draws.
-//   5. k_apply: every public site computes its values from its own start
-//      state g^(fixed + extra before it)(s0), in parallel, and emits public
-//      RGB16 with the counters.
+//   5. k_apply: every public site makes its draws and computes its values from
+//      its own start state g^(fixed + extra before it)(s0), in parallel, and
+//      emits public RGB16 with the counters.  Draws that differ from what steps
+//      1 and 4 say fail the pass.
 #include <algorithm>
 
 #include "fx_internal.cuh"
